@@ -681,11 +681,17 @@ __global__ void __launch_bounds__(256) k_reinit_lin(const R *s, const R *phi0, c
     R star[3], sel[3];
     int which[3];
     for (int d = 0; d < 3; d++) {
-      R v[6];  // scaled D1(c-2 .. c+3)
+      R v[6], gp, gm;  // D1(c-2 .. c+3)
 #pragma unroll
-      for (int f = -2; f <= 3; f++) v[f + 2] = (s[c + f * st[d]] - s[c + (f - 1) * st[d]]) * inv[d];
-      const R gp = fused::weno<R, EXACT>(v[5], v[4], v[3], v[2], v[1]);
-      const R gm = fused::weno<R, EXACT>(v[0], v[1], v[2], v[3], v[4]);
+      for (int f = -2; f <= 3; f++) v[f + 2] = s[c + f * st[d]] - s[c + (f - 1) * st[d]];
+      if constexpr (EXACT) {
+        weno5_pm64(v, wide64(inv[d]), Consts<R>::tiny, gp, gm);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 6; q++) v[q] *= inv[d];
+        gp = (R)fused::weno5_fast(v[5], v[4], v[3], v[2], v[1]);
+        gm = (R)fused::weno5_fast(v[0], v[1], v[2], v[3], v[4]);
+      }
       R u, w, du, dw;
       if (pc > R(0)) {
         u = rmax(-gp, R(0)); du = (-gp > R(0)) ? R(-1) : R(0);

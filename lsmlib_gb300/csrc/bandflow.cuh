@@ -60,35 +60,19 @@ __device__ __forceinline__ void raise_key(unsigned long long *key, unsigned long
   if (k > __ldcg(key)) atomicMax(key, k);
 }
 
-// WENO5 with the local routines' epsilon floor (spatial_derivatives2d_local.f.in:892)
+// Both WENO5 sides of one axis at a cell, with the local routines' epsilon
+// floor (spatial_derivatives2d_local.f.in:892), on its six undivided
+// differences
 template <class R, bool EXACT>
-__device__ __forceinline__ R weno_local(R v1, R v2, R v3, R v4, R v5) {
+__device__ __forceinline__ void weno_local_pm(const R D[6], R inv, R &gp, R &gm) {
   if constexpr (EXACT) {
-    const R c13 = 1.0 / 3.0, c76 = 7.0 / 6.0, c116 = 11.0 / 6.0, c16 = 1.0 / 6.0, c56 = 5.0 / 6.0;
-    const R c1312 = 13.0 / 12.0, c14 = 0.25;
-    R m = v1 * v1;
-    m = rmax(m, v2 * v2);
-    m = rmax(m, v3 * v3);
-    m = rmax(m, v4 * v4);
-    m = rmax(m, v5 * v5);
-    const R eps = R(1e-6) * m + R(1.e-35);
-    const R p1 = c13 * v1 - c76 * v2 + c116 * v3;
-    const R p2 = -(c16 * v2) + c56 * v3 + c13 * v4;
-    const R p3 = c13 * v3 + c56 * v4 - c16 * v5;
-    R t = v1 - R(2.0) * v2 + v3, u = v1 - R(4.0) * v2 + R(3.0) * v3;
-    const R S1 = c1312 * (t * t) + c14 * (u * u);
-    t = v2 - R(2.0) * v3 + v4; u = v2 - v4;
-    const R S2 = c1312 * (t * t) + c14 * (u * u);
-    t = v3 - R(2.0) * v4 + v5; u = R(3.0) * v3 - R(4.0) * v4 + v5;
-    const R S3 = c1312 * (t * t) + c14 * (u * u);
-    R a1 = R(0.1) / ((S1 + eps) * (S1 + eps));
-    R a2 = R(0.6) / ((S2 + eps) * (S2 + eps));
-    R a3 = R(0.3) / ((S3 + eps) * (S3 + eps));
-    const R is = R(1.0) / (a1 + a2 + a3);
-    a1 = a1 * is; a2 = a2 * is; a3 = a3 * is;
-    return a1 * p1 + a2 * p2 + a3 * p3;
+    weno5_pm64(D, wide64(inv), 1.e-35, gp, gm);
   } else {
-    return (R)fused::weno5_fast((float)v1, (float)v2, (float)v3, (float)v4, (float)v5);
+    float v[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) v[q] = (float)(D[q] * inv);
+    gp = (R)fused::weno5_fast(v[5], v[4], v[3], v[2], v[1]);
+    gm = (R)fused::weno5_fast(v[0], v[1], v[2], v[3], v[4]);
   }
 }
 
@@ -144,13 +128,12 @@ __device__ __forceinline__ R cell_rhs(const BandArgs<R> &a, int i, int j, int k,
   // HJ WENO5 plus/minus from the band values of src
   const R inv = a.inv_dx;
   R gp[3], gm[3];
-#pragma unroll
+#pragma unroll 1
   for (int d = 0; d < 3; d++) {
-    R v[6];
+    R D[6];
 #pragma unroll
-    for (int q = -2; q <= 3; q++) v[q + 2] = (c[q * s[d]] - c[(q - 1) * s[d]]) * inv;
-    gp[d] = weno_local<R, EXACT>(v[5], v[4], v[3], v[2], v[1]);
-    gm[d] = weno_local<R, EXACT>(v[0], v[1], v[2], v[3], v[4]);
+    for (int q = -2; q <= 3; q++) D[q + 2] = c[q * s[d]] - c[(q - 1) * s[d]];
+    weno_local_pm<R, EXACT>(D, inv, gp[d], gm[d]);
   }
   return godunov_rhs<R>(a, vn, gp, gm, h_over_dx);
 }

@@ -11,6 +11,7 @@
 // This translation unit is compiled with -fmad=false (FP64 parity form).
 #include "lsmgpu_common.cuh"
 #include "stencil_math.cuh"
+#include "weno64.cuh"
 #include "../../include/lsmgpu_toolbox3d.h"
 
 namespace lsmgpu {
@@ -36,14 +37,12 @@ __device__ __forceinline__ void side_values(const Diffs<R> &d, R inv, R &plus, R
   if (S == ENO1) { plus = eno1_plus(d, inv); minus = eno1_minus(d, inv); }
   if (S == ENO2) { plus = eno2_plus(d, inv); minus = eno2_minus(d, inv); }
   if (S == ENO3) { plus = eno3_plus(d, inv); minus = eno3_minus(d, inv); }
-  if (S == WENO5) { plus = weno5_plus(d, inv); minus = weno5_minus(d, inv); }
 }
 template <int S>
 __device__ __forceinline__ R side_value(const Diffs<R> &d, R inv, bool use_minus) {
   if (S == ENO1) return use_minus ? eno1_minus(d, inv) : eno1_plus(d, inv);
   if (S == ENO2) return use_minus ? eno2_minus(d, inv) : eno2_plus(d, inv);
-  if (S == ENO3) return use_minus ? eno3_minus(d, inv) : eno3_plus(d, inv);
-  return use_minus ? weno5_minus(d, inv) : weno5_plus(d, inv);
+  return use_minus ? eno3_minus(d, inv) : eno3_plus(d, inv);
 }
 
 // load phi(c-3..c+3) along stride s (only the reach the scheme needs)
@@ -56,7 +55,67 @@ __device__ __forceinline__ void load_line(R a[7], const R *c, long long s) {
   }
 }
 
-struct Out3 { View<R> x, y, z; };
+struct Out3 {
+  View<R> x, y, z;
+  __device__ __forceinline__ R &at(int d, int i, int j, int k) const {
+    return (d == 0 ? x : (d == 1 ? y : z))(i, j, k);
+  }
+};
+
+// The undivided differences D1(c-2) .. D1(c+3) along stride s.
+__device__ __forceinline__ void line_diffs(R d[6], const R *c, long long s) {
+  R a[7];
+  load_line<3>(a, c, s);
+#pragma unroll
+  for (int q = 0; q < 6; q++) d[q] = a[q + 1] - a[q];
+}
+
+// HJ WENO5 (spatial_derivatives3d.f.in:1161-1611).  Bound by the arithmetic
+// (weno64.cuh), not by memory.  The axes run in a loop that is not unrolled:
+// one axis' two reconstructions are some 1,900 instructions, and three copies
+// would not stay in the instruction cache.  An axis with stride 0 (one that a
+// 2D or 1D call does not have) has differences of exactly 0 and derivatives
+// of exactly 0.
+__global__ void __launch_bounds__(256) k_hj_pm_weno5(Out3 plus, Out3 minus, View<const R> phi, Box fb, R ix, R iy,
+                                                     R iz) {
+  LSMGPU_CELL_INDEX(fb, i, j, k);
+  const R *c = phi.p + phi.off(i, j, k);
+#pragma unroll 1
+  for (int d = 0; d < 3; d++) {
+    const long long s = phi.stride(d);
+    R gp = R(0), gm = R(0);
+    if (s != 0) {
+      R D[6];
+      line_diffs(D, c, s);
+      weno5_pm64(D, wide64(d == 0 ? ix : (d == 1 ? iy : iz)), Consts<R>::tiny, gp, gm);
+    }
+    plus.at(d, i, j, k) = gp;
+    minus.at(d, i, j, k) = gm;
+  }
+}
+
+// Upwind HJ WENO5 (spatial_derivatives3d.f.in:2628-2996): the side is chosen
+// on the differences, so lanes of both signs share one reconstruction.
+__global__ void __launch_bounds__(256) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx, View<const R> vy,
+                                                         View<const R> vz, Box fb, R ix, R iy, R iz) {
+  LSMGPU_CELL_INDEX(fb, i, j, k);
+  const R *c = phi.p + phi.off(i, j, k);
+#pragma unroll 1
+  for (int d = 0; d < 3; d++) {
+    const R u = (d == 0 ? vx : (d == 1 ? vy : vz))(i, j, k);
+    const long long s = phi.stride(d);
+    R out = R(0);
+    if (!(fabs(u) < Consts<R>::zero_tol) && s != 0) {
+      // phi(c-3) is read by the minus side only, phi(c+3) by the plus side only
+      R D[6], v[5];
+      line_diffs(D, c, s);
+#pragma unroll
+      for (int q = 0; q < 5; q++) v[q] = u > R(0) ? D[q] : D[5 - q];
+      out = weno5_side64(v, wide64(d == 0 ? ix : (d == 1 ? iy : iz)), Consts<R>::tiny);
+    }
+    g.at(d, i, j, k) = out;
+  }
+}
 
 template <int S>
 __global__ void k_hj_pm(Out3 plus, Out3 minus, View<const R> phi, Box fb, R ix, R iy, R iz) {
@@ -120,7 +179,10 @@ void hj_pm(const char *name, R *pxp, R *pyp, R *pzp, const Box &pb, R *pxm, R *p
   View<const R> ph = view((const R *)call.in(phi, phb.size()), phb);
   if (!call.ok()) return;
   Grid3 g = cover(fb);
-  LSMGPU_LAUNCH(k_hj_pm<S>, g.grid, g.block, 0, P, M, ph, fb, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
+  if constexpr (S == WENO5)
+    LSMGPU_LAUNCH(k_hj_pm_weno5, g.grid, g.block, 0, P, M, ph, fb, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
+  else
+    LSMGPU_LAUNCH(k_hj_pm<S>, g.grid, g.block, 0, P, M, ph, fb, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
   call.finish();
 }
 
@@ -141,8 +203,12 @@ void hj_upwind(const char *name, R *px, R *py, R *pz, const Box &gb, const R *ph
   View<const R> VZ = view((const R *)call.in(vz, nv), vb);
   if (!call.ok()) return;
   Grid3 g = cover(fb);
-  LSMGPU_LAUNCH(k_hj_upwind<S>, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, R(1.0) / dx, R(1.0) / dy,
-                R(1.0) / dz);
+  if constexpr (S == WENO5)
+    LSMGPU_LAUNCH(k_hj_upwind_weno5, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, R(1.0) / dx, R(1.0) / dy,
+                  R(1.0) / dz);
+  else
+    LSMGPU_LAUNCH(k_hj_upwind<S>, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, R(1.0) / dx, R(1.0) / dy,
+                  R(1.0) / dz);
   call.finish();
 }
 

@@ -23,6 +23,7 @@
 #include "lsmgpu_common.cuh"
 #include "stencil_math.cuh"
 #include "tma.cuh"
+#include "weno64.cuh"
 
 namespace lsmgpu {
 namespace fused {
@@ -171,12 +172,6 @@ __device__ __forceinline__ float weno5_fast(float v1, float v2, float v3, float 
   return __fdividef(fmaf(n1, p1, fmaf(n2, p2, n3 * p3)), n1 + n2 + n3);
 }
 
-template <class R, bool EXACT>
-__device__ __forceinline__ R weno(R v1, R v2, R v3, R v4, R v5) {
-  if constexpr (EXACT) return weno5_exact<R>(v1, v2, v3, v4, v5);
-  else return (R)weno5_fast((float)v1, (float)v2, (float)v3, (float)v4, (float)v5);
-}
-
 // reinitialization RHS; the FP32 form keeps the FP64 zero tolerance so it
 // approximates the FP64 computation, and uses reciprocal square roots
 template <class R, bool EXACT>
@@ -237,51 +232,50 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
   if (i >= L.nx || j >= L.ny) return;
   const int sx = tx + 4, sy = ty + 3;
   const int kmax = min(TZ, L.nz - z0);
+  const Wide64 wide[3] = {wide64(a.inv[0]), wide64(a.inv[1]), wide64(a.inv[2])};
+  const int st[3] = {1, SX, SX * SY};
 
   for (int tz = 0; tz < kmax; tz++) {
     const int k = z0 + tz;
     const int sz = tz + 3;
     const R *c = tile + (sz * SY + sy) * SX + sx;
-    const int st[3] = {1, SX, SX * SY};
     R rhs;
     if (MODE == REINIT) {
-      R gp[3], gm[3];
-#pragma unroll
+      const R pc = a.use0 ? a.phi0[L.idx(i, j, k)] : c[0];
+      R n2 = R(0);
+#pragma unroll 1
       for (int d = 0; d < 3; d++) {
-        R v[6];  // scaled D1(c-2 .. c+3)
+        const int s = st[d];
+        R D[6], gp, gm;  // D1(c-2 .. c+3)
 #pragma unroll
-        for (int f = -2; f <= 3; f++) v[f + 2] = (c[f * st[d]] - c[(f - 1) * st[d]]) * a.inv[d];
-        gp[d] = weno<R, EXACT>(v[5], v[4], v[3], v[2], v[1]);
-        gm[d] = weno<R, EXACT>(v[0], v[1], v[2], v[3], v[4]);
+        for (int f = -2; f <= 3; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
+        weno5_pm64(D, wide[d], Consts<R>::tiny, gp, gm);
+        const R t = reinit_axis(pc, gp, gm);
+        n2 = d == 0 ? t * t : n2 + t * t;
       }
-      const long long cell = L.idx(i, j, k);
-      const R pc = a.use0 ? a.phi0[cell] : c[0];
-      rhs = reinit_term<R, EXACT>(pc, gp, gm, a.dx_sq, a.use0 != 0);
+      rhs = reinit_from_sq<R>(pc, n2, a.dx_sq, a.use0 != 0);
     } else {
-      R g[3], vel[3];
-      const long long cell = L.idx(i, j, k);
-#pragma unroll
-      for (int d = 0; d < 3; d++) vel[d] = (MODE == ADV_CONST) ? a.vconst[d] : a.vel[d][cell];
-#pragma unroll
+      R dot = R(0);
+#pragma unroll 1
       for (int d = 0; d < 3; d++) {
-        // spatial_derivatives3d.f.in:2756-2812
-        if (fabs(vel[d]) < Consts<double>::zero_tol) {
-          g[d] = R(0);
-        } else if (vel[d] > R(0)) {
-          R v[5];
+        // spatial_derivatives3d.f.in:2756-2812: |v| < zero_tol gives 0, v > 0
+        // takes the backward stencil, otherwise the forward one
+        const R u = (MODE == ADV_CONST) ? a.vconst[d] : a.vel[d][L.idx(i, j, k)];
+        const int s = st[d];
+        R g = R(0);
+        if (!(fabs(u) < Consts<double>::zero_tol)) {
+          R D[6], v[5];
 #pragma unroll
-          for (int f = -2; f <= 2; f++) v[f + 2] = (c[f * st[d]] - c[(f - 1) * st[d]]) * a.inv[d];
-          g[d] = weno<R, EXACT>(v[0], v[1], v[2], v[3], v[4]);
-        } else {
-          R v[5];
+          for (int f = -2; f <= 3; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
 #pragma unroll
-          for (int f = -1; f <= 3; f++) v[f + 1] = (c[f * st[d]] - c[(f - 1) * st[d]]) * a.inv[d];
-          g[d] = weno<R, EXACT>(v[4], v[3], v[2], v[1], v[0]);
+          for (int q = 0; q < 5; q++) v[q] = u > R(0) ? D[q] : D[5 - q];
+          g = weno5_side64(v, wide[d], Consts<R>::tiny);
         }
+        dot = d == 0 ? u * g : dot + u * g;
       }
       // lsm3dZeroOutLevelSetEqnRHS then lsm3dAddAdvectionTermToLSERHS
       // (level_set_evolution3d.f.in:38, :113-116)
-      rhs = R(0) - (vel[0] * g[0] + vel[1] * g[1] + vel[2] * g[2]);
+      rhs = R(0) - dot;
     }
 
     const long long cell = L.idx(i, j, k);

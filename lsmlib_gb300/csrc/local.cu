@@ -13,6 +13,7 @@
 // This translation unit is compiled with -fmad=false (FP64 parity form).
 #include "lsmgpu_common.cuh"
 #include "stencil_math.cuh"
+#include "weno64.cuh"
 #include "../../include/lsmgpu_toolbox3d.h"
 
 namespace lsmgpu {
@@ -123,34 +124,6 @@ void dn_local(View<R> dn, const Box &db, View<const R> dm, const Box &mb, int n,
 struct PM3 { View<R> x, y, z; __device__ View<R> operator[](int d) const { return d == 0 ? x : (d == 1 ? y : z); } };
 
 __device__ __forceinline__ long long dstride(const View<R> &v, int d) { return d == 0 ? 1 : (d == 1 ? v.s1 : v.s2); }
-
-// WENO5 with the local routines' epsilon floor 1e-35
-// (spatial_derivatives2d_local.f.in:892)
-__device__ __forceinline__ R weno5_local(R v1, R v2, R v3, R v4, R v5) {
-  const R c13 = 1.0 / 3.0, c76 = 7.0 / 6.0, c116 = 11.0 / 6.0, c16 = 1.0 / 6.0, c56 = 5.0 / 6.0;
-  const R c1312 = 13.0 / 12.0, c14 = 0.25;
-  R m = v1 * v1;
-  m = rmax(m, v2 * v2);
-  m = rmax(m, v3 * v3);
-  m = rmax(m, v4 * v4);
-  m = rmax(m, v5 * v5);
-  const R eps = R(1e-6) * m + R(1.e-35);
-  const R p1 = c13 * v1 - c76 * v2 + c116 * v3;
-  const R p2 = -(c16 * v2) + c56 * v3 + c13 * v4;
-  const R p3 = c13 * v3 + c56 * v4 - c16 * v5;
-  R t = v1 - R(2.0) * v2 + v3, u = v1 - R(4.0) * v2 + R(3.0) * v3;
-  const R S1 = c1312 * (t * t) + c14 * (u * u);
-  t = v2 - R(2.0) * v3 + v4; u = v2 - v4;
-  const R S2 = c1312 * (t * t) + c14 * (u * u);
-  t = v3 - R(2.0) * v4 + v5; u = R(3.0) * v3 - R(4.0) * v4 + v5;
-  const R S3 = c1312 * (t * t) + c14 * (u * u);
-  R a1 = R(0.1) / ((S1 + eps) * (S1 + eps));
-  R a2 = R(0.6) / ((S2 + eps) * (S2 + eps));
-  R a3 = R(0.3) / ((S3 + eps) * (S3 + eps));
-  const R is = R(1.0) / (a1 + a2 + a3);
-  a1 = a1 * is; a2 = a2 * is; a3 = a3 * is;
-  return a1 * p1 + a2 * p2 + a3 * p3;
-}
 
 // ---- max / sum reductions over lists ----------------------------------------
 __device__ __forceinline__ unsigned long long okey(R v) {
@@ -463,8 +436,12 @@ void lsm3dhjweno5local_(PMARGS, R *d1, BOXARG(d1), DXP, IDX3, const int *nlo0, c
       if (!gd(i, j, k)) return;
       const long long c = D1.off(i, j, k), s = dstride(D1, d);
       const R *q = D1.p;
-      P[d](i, j, k) = weno5_local(q[c + 3 * s] * w, q[c + 2 * s] * w, q[c + s] * w, q[c] * w, q[c - s] * w);
-      M[d](i, j, k) = weno5_local(q[c - 2 * s] * w, q[c - s] * w, q[c] * w, q[c + s] * w, q[c + 2 * s] * w);
+      // epsilon floor 1e-35 (spatial_derivatives2d_local.f.in:892)
+      const R D[6] = {q[c - 2 * s], q[c - s], q[c], q[c + s], q[c + 2 * s], q[c + 3 * s]};
+      R gp, gm;
+      weno5_pm64(D, wide64(w), 1.e-35, gp, gm);
+      P[d](i, j, k) = gp;
+      M[d](i, j, k) = gm;
     });
   }
   lc.c.finish();

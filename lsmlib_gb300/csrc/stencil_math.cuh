@@ -110,52 +110,6 @@ __device__ __forceinline__ R eno3_minus(const Diffs<R> &d, R inv) {
   return x * inv;
 }
 
-// WENO5-JS on five scaled first differences, in the exact form of
-// spatial_derivatives3d.f.in:1296-1323 (parity form).
-template <class R>
-__device__ __forceinline__ R weno5_exact(R v1, R v2, R v3, R v4, R v5) {
-  const R c13 = R(1.0 / 3.0), c76 = R(7.0 / 6.0), c116 = R(11.0 / 6.0);
-  const R c16 = R(1.0 / 6.0), c56 = R(5.0 / 6.0), c1312 = R(13.0 / 12.0);
-  const R c14 = R(0.25);
-  R m = v1 * v1;
-  m = rmax(m, v2 * v2);
-  m = rmax(m, v3 * v3);
-  m = rmax(m, v4 * v4);
-  m = rmax(m, v5 * v5);
-  const R eps = R(1e-6) * m + Consts<R>::tiny;
-  const R p1 = c13 * v1 - c76 * v2 + c116 * v3;
-  const R p2 = -(c16 * v2) + c56 * v3 + c13 * v4;
-  const R p3 = c13 * v3 + c56 * v4 - c16 * v5;
-  R t = v1 - R(2.0) * v2 + v3;
-  R u = v1 - R(4.0) * v2 + R(3.0) * v3;
-  const R S1 = c1312 * (t * t) + c14 * (u * u);
-  t = v2 - R(2.0) * v3 + v4;
-  u = v2 - v4;
-  const R S2 = c1312 * (t * t) + c14 * (u * u);
-  t = v3 - R(2.0) * v4 + v5;
-  u = R(3.0) * v3 - R(4.0) * v4 + v5;
-  const R S3 = c1312 * (t * t) + c14 * (u * u);
-  R a1 = R(0.1) / ((S1 + eps) * (S1 + eps));
-  R a2 = R(0.6) / ((S2 + eps) * (S2 + eps));
-  R a3 = R(0.3) / ((S3 + eps) * (S3 + eps));
-  const R inv_sum = R(1.0) / (a1 + a2 + a3);
-  a1 = a1 * inv_sum;
-  a2 = a2 * inv_sum;
-  a3 = a3 * inv_sum;
-  return a1 * p1 + a2 * p2 + a3 * p3;
-}
-
-// plus side: v = D1(c+3..c-1); minus side: v = D1(c-2..c+2)
-// (spatial_derivatives3d.f.in:1286-1367)
-template <class R>
-__device__ __forceinline__ R weno5_plus(const Diffs<R> &d, R inv) {
-  return weno5_exact<R>(d.D1(3) * inv, d.D1(2) * inv, d.D1(1) * inv, d.D1(0) * inv, d.D1(-1) * inv);
-}
-template <class R>
-__device__ __forceinline__ R weno5_minus(const Diffs<R> &d, R inv) {
-  return weno5_exact<R>(d.D1(-2) * inv, d.D1(-1) * inv, d.D1(0) * inv, d.D1(1) * inv, d.D1(2) * inv);
-}
-
 // Godunov |grad phi|^2 of level_set_evolution3d.f.in:210-223 for normal
 // speed sign `pos` (vn > 0).
 template <class R>
@@ -179,26 +133,32 @@ __device__ __forceinline__ R godunov_normal_sq(bool pos, const R p[3], const R m
 
 // Reinitialization right-hand side of reinitialization3d.f.in:159-199 (Peng
 // form, use0 = false) and :217-256 (phi0 form, use0 = true).  `pc` is phi
-// (or phi0) at the cell.
+// (or phi0) at the cell.  One axis' Godunov value, the RHS from the sum of
+// their squares (taken in axis order), and both together.
+template <class R>
+__device__ __forceinline__ R reinit_axis(R pc, R gp, R gm) {
+  R u, w;
+  if (pc > R(0)) {
+    u = rmax(-gp, R(0));
+    w = rmax(gm, R(0));
+  } else {
+    u = rmax(gp, R(0));
+    w = rmax(-gm, R(0));
+  }
+  return rmax(u, w);
+}
+template <class R>
+__device__ __forceinline__ R reinit_from_sq(R pc, R n2, R dx_sq, bool use0) {
+  if (!(fabs(pc) >= Consts<R>::zero_tol)) return R(0);
+  const R sgn = use0 ? pc / sqrt(pc * pc + dx_sq) : pc / sqrt(pc * pc + n2 * dx_sq);
+  return sgn * (R(1.0) - sqrt(n2));
+}
 template <class R>
 __device__ __forceinline__ R reinit_rhs(R pc, const R gp[3], const R gm[3], R dx_sq, bool use0) {
   R st[3];
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    R u, w;
-    if (pc > R(0)) {
-      u = rmax(-gp[d], R(0));
-      w = rmax(gm[d], R(0));
-    } else {
-      u = rmax(gp[d], R(0));
-      w = rmax(-gm[d], R(0));
-    }
-    st[d] = rmax(u, w);
-  }
-  if (!(fabs(pc) >= Consts<R>::zero_tol)) return R(0);
-  const R n2 = st[0] * st[0] + st[1] * st[1] + st[2] * st[2];
-  const R sgn = use0 ? pc / sqrt(pc * pc + dx_sq) : pc / sqrt(pc * pc + n2 * dx_sq);
-  return sgn * (R(1.0) - sqrt(n2));
+  for (int d = 0; d < 3; d++) st[d] = reinit_axis(pc, gp[d], gm[d]);
+  return reinit_from_sq(pc, st[0] * st[0] + st[1] * st[1] + st[2] * st[2], dx_sq, use0);
 }
 
 // Curvature numerator in the term order of curvature3d.f.in:109-117.

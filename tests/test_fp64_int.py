@@ -1,0 +1,59 @@
+"""FP64 arithmetic on the integer pipes (csrc/fp64_int.cuh) and the WENO5
+reconstruction on it (csrc/weno64.cuh): the same bits as FP64 hardware.
+
+On the host the routines are compiled with the system compiler and compared
+with the host's FP64 operations; on the GPU the drop-in WENO5 routines are
+compared with the oracle on fields that take both of their paths."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import lsmlib_gb300 as L
+from tests import harness as H
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_host_arithmetic_equals_hardware(seed, tmp_path):
+    exe = str(tmp_path / "fp64_int")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", os.path.join(ROOT, "lsmlib_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "fp64_int_driver.cpp"), "-o", exe], check=True)
+    out = subprocess.run([exe, "300000", str(seed)], check=True, capture_output=True, text=True).stdout.split()
+    assert out == ["0", "0"]
+
+
+def field(kind, gb):
+    """Fields on which the integer path, the FP64-unit path or a mix of both
+    runs, cell by cell."""
+    rng = np.random.default_rng(17)
+    f = H.rough_field(rng, gb)
+    if kind == "flat":
+        f[...] = 0.75
+    elif kind == "dyadic":
+        f = np.round(f * 4) / 4
+    elif kind == "tiny":
+        f *= 1e-170
+    elif kind == "mixed":
+        f *= 10.0 ** rng.integers(-200, 120, size=f.shape)
+    elif kind == "nonfinite":
+        f[rng.random(f.shape) < 0.01] = np.inf
+        f[rng.random(f.shape) < 0.01] = np.nan
+    return np.asfortranarray(f)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["rough", "flat", "dyadic", "tiny", "mixed", "nonfinite"])
+@pytest.mark.parametrize("sym", ["lsm3dhjweno5_", "lsm3dupwindhjweno5_"])
+def test_dropin_weno5_on_all_scales(sym, kind, gpu_lib):
+    vals = H.dense_case(sym, seed=3)
+    vals["phi"] = field(kind, H.GB)
+    with np.errstate(all="ignore"):
+        want, _ = H.run(H.oracle(), sym, vals)
+        got, _ = H.run(gpu_lib, sym, vals)
+    L.check()
+    for name in H.written_names(sym):
+        if name in got and not name.startswith("d"):
+            assert H.same(want[name], got[name]), name
