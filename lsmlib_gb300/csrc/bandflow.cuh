@@ -82,24 +82,10 @@ __device__ __forceinline__ void weno_local_pm(const R D[6], R inv, R &gp, R &gm)
 template <class R>
 __device__ __forceinline__ R cell_vn(const BandArgs<R> &a, const R *c, const long long s[3]) {
   const R f = a.f_half;
-  const R g0 = (c[s[0]] - c[-s[0]]) * f, g1 = (c[s[1]] - c[-s[1]]) * f, g2 = (c[s[2]] - c[-s[2]]) * f;
-  const R tol = Consts<double>::zero_tol;
-  R x2 = g0 * g0, y2 = g1 * g1, z2 = g2 * g2;
-  if (x2 < tol) x2 = R(0);
-  if (y2 < tol) y2 = R(0);
-  if (z2 < tol) z2 = R(0);
-  const R t = sqrt(x2 + y2 + z2);
-  const R mag = (t < tol) ? R(0) : t;
-  const R fxx = a.f_xx, fxy = a.f_xy;
-  const R xx = (c[s[0]] - R(2.0) * c[0] + c[-s[0]]) * fxx;
-  const R yy = (c[s[1]] - R(2.0) * c[0] + c[-s[1]]) * fxx;
-  const R zz = (c[s[2]] - R(2.0) * c[0] + c[-s[2]]) * fxx;
-  const R xy = (c[s[0] + s[1]] - c[s[0] - s[1]] - c[-s[0] + s[1]] + c[-s[0] - s[1]]) * fxy;
-  const R xz = (c[s[0] + s[2]] - c[s[0] - s[2]] - c[-s[0] + s[2]] + c[-s[0] - s[2]]) * fxy;
-  const R yz = (c[s[1] + s[2]] - c[s[1] - s[2]] - c[-s[1] + s[2]] + c[-s[1] - s[2]]) * fxy;
-  const R den = mag * mag * mag;
-  const R kappa = (den < tol) ? R(0) : curv_numerator(xx, yy, zz, xy, xz, yz, g0, g1, g2) / den;
-  return a.a_n - a.b_n * kappa;
+  const R g0 = mul_(c[s[0]] - c[-s[0]], f), g1 = mul_(c[s[1]] - c[-s[1]], f), g2 = mul_(c[s[2]] - c[-s[2]], f);
+  const R mag = grad_magnitude(g0, g1, g2, R(Consts<double>::zero_tol));
+  const R kappa = mean_curvature2(c, s[0], s[1], s[2], g0, g1, g2, mag, a.f_xx, a.f_xx, a.f_xx, a.f_xy, a.f_xy, a.f_xy);
+  return a.a_n - mul_(a.b_n, kappa);
 }
 
 // Godunov normal-velocity term (level_set_evolution3d_local.f.in:236-273) from
@@ -108,14 +94,15 @@ __device__ __forceinline__ R cell_vn(const BandArgs<R> &a, const R *c, const lon
 template <class R>
 __device__ __forceinline__ R godunov_rhs(const BandArgs<R> &a, R vn, const R gp[3], const R gm[3], R &h_over_dx) {
   const R tol = Consts<double>::zero_tol;
-  const R sq = godunov_normal_sq<R>(vn > R(0), gp, gm);
+  const R sq = godunov_normal_sq<R>(is_pos_(vn), gp, gm);
   R rhs = R(0);
-  if (fabs(vn) >= tol) rhs = rhs - vn * sqrt(sq);
+  if (at_least_(vn, tol)) rhs = rhs - mul_(vn, sqrt_(sq));
   const R dx = a.dx, inv = a.inv_dx;
   const R mx2 = dx * dx;
-  const R cx = rmax(fabs(gp[0]), fabs(gm[0])), cy = rmax(fabs(gp[1]), fabs(gm[1])), cz = rmax(fabs(gp[2]), fabs(gm[2]));
-  const R ng = sqrt(cx * cx + cy * cy + cz * cz + mx2);
-  h_over_dx = (ng > tol) ? fabs(vn) / ng * (cx * inv + cy * inv + cz * inv) : R(-1.0);
+  const R cx = max_nonneg_(abs_(gp[0]), abs_(gm[0])), cy = max_nonneg_(abs_(gp[1]), abs_(gm[1]));
+  const R cz = max_nonneg_(abs_(gp[2]), abs_(gm[2]));
+  const R ng = sqrt_(sqr_(cx) + sqr_(cy) + sqr_(cz) + mx2);
+  h_over_dx = (ng > tol) ? mul_(div_(abs_(vn), ng), mul_(cx, inv) + mul_(cy, inv) + mul_(cz, inv)) : R(-1.0);
   return rhs;
 }
 

@@ -22,38 +22,21 @@ struct CurvArgs {
   R fxx, fyy, fzz, fxy, fxz, fyz;
 };
 
+// The FP64 form is bound by its arithmetic: 28 additions on the FP64 pipe and
+// 35 products, a division and a root on the integer pipes (about 89 FP64
+// instructions as written).
 template <class R>
-__global__ void k_mean_curvature(CurvArgs<R> a) {
+__global__ void __launch_bounds__(256) k_mean_curvature(CurvArgs<R> a) {
   LSMGPU_CELL_INDEX(a.fb, i, j, k);
   const R *c = a.phi.p + a.phi.off(i, j, k);
   const long long sx = 1, sy = a.phi.s1, sz = a.phi.s2;
-  // central gradient
-  const R px = (c[sx] - c[-sx]) * a.gx;
-  const R py = (c[sy] - c[-sy]) * a.gy;
-  const R pz = (c[sz] - c[-sz]) * a.gz;
-  // gradient magnitude with the reference's 1e-8 clamps
-  const R tol = R(1.e-8);
-  R x2 = px * px, y2 = py * py, z2 = pz * pz;
-  if (x2 < tol) x2 = R(0);
-  if (y2 < tol) y2 = R(0);
-  if (z2 < tol) z2 = R(0);
-  const R t = sqrt(x2 + y2 + z2);
-  const R g = (t < tol) ? R(0) : t;
+  // central gradient, its magnitude with the reference's 1e-8 clamps, curvature
+  const R px = mul_(c[sx] - c[-sx], a.gx);
+  const R py = mul_(c[sy] - c[-sy], a.gy);
+  const R pz = mul_(c[sz] - c[-sz], a.gz);
+  const R g = grad_magnitude(px, py, pz, R(1.e-8));
   if (a.mag.p) a.mag(i, j, k) = g;
-  // second derivatives and curvature
-  const R xx = (c[sx] - R(2.0) * c[0] + c[-sx]) * a.fxx;
-  const R yy = (c[sy] - R(2.0) * c[0] + c[-sy]) * a.fyy;
-  const R zz = (c[sz] - R(2.0) * c[0] + c[-sz]) * a.fzz;
-  const R xy = (c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy]) * a.fxy;
-  const R xz = (c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz]) * a.fxz;
-  const R yz = (c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz]) * a.fyz;
-  const R den = g * g * g;
-  R out;
-  if (den < R(Consts<double>::zero_tol))
-    out = R(0);
-  else
-    out = curv_numerator(xx, yy, zz, xy, xz, yz, px, py, pz) / den;
-  a.kappa(i, j, k) = out;
+  a.kappa(i, j, k) = mean_curvature2(c, sx, sy, sz, px, py, pz, g, a.fxx, a.fyy, a.fzz, a.fxy, a.fxz, a.fyz);
 }
 
 inline bool pinned_host(const void *p) {

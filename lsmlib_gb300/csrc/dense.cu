@@ -30,7 +30,7 @@ template <int S> struct SchemeInfo;
 template <> struct SchemeInfo<ENO1> { static constexpr int reach = 1, order = 1; };
 template <> struct SchemeInfo<ENO2> { static constexpr int reach = 2, order = 2; };
 template <> struct SchemeInfo<ENO3> { static constexpr int reach = 3, order = 3; };
-template <> struct SchemeInfo<WENO5> { static constexpr int reach = 3, order = 1; };
+template <> struct SchemeInfo<WENO5> { static constexpr int reach = 3; };
 
 template <int S>
 __device__ __forceinline__ void side_values(const Diffs<R> &d, R inv, R &plus, R &minus) {
@@ -71,50 +71,59 @@ __device__ __forceinline__ void line_diffs(R d[6], const R *c, long long s) {
 }
 
 // HJ WENO5 (spatial_derivatives3d.f.in:1161-1611).  Bound by the arithmetic
-// (weno64.cuh), not by memory.  The axes run in a loop that is not unrolled:
-// one axis' two reconstructions are some 1,900 instructions, and three copies
-// would not stay in the instruction cache.  An axis with stride 0 (one that a
-// 2D or 1D call does not have) has differences of exactly 0 and derivatives
-// of exactly 0.
-__global__ void __launch_bounds__(256) k_hj_pm_weno5(Out3 plus, Out3 minus, View<const R> phi, Box fb, R ix, R iy,
-                                                     R iz) {
-  LSMGPU_CELL_INDEX(fb, i, j, k);
-  const R *c = phi.p + phi.off(i, j, k);
-#pragma unroll 1
-  for (int d = 0; d < 3; d++) {
-    const long long s = phi.stride(d);
-    R gp = R(0), gm = R(0);
-    if (s != 0) {
-      R D[6];
-      line_diffs(D, c, s);
-      weno5_pm64(D, wide64(d == 0 ? ix : (d == 1 ? iy : iz)), Consts<R>::tiny, gp, gm);
-    }
-    plus.at(d, i, j, k) = gp;
-    minus.at(d, i, j, k) = gm;
-  }
+// (weno64.cuh), not by memory, so each thread takes one axis of one cell
+// (blockIdx.x counts the axes within a block of cells): three times the
+// threads of one third the length fill the last wave better, the axes of a
+// cell block run next to each other and share its lines in the L2, and a 2D
+// or 1D call launches only the axes it has.
+struct AxisCell {
+  int d, i, j, k;
+  bool in;
+};
+__device__ __forceinline__ AxisCell axis_cell(const Box &fb, unsigned axes) {
+  AxisCell a;
+  a.d = (int)(blockIdx.x % axes);
+  a.i = fb.lo[0] + (blockIdx.x / axes) * blockDim.x + threadIdx.x;
+  a.j = fb.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
+  a.k = fb.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
+  a.in = a.i <= fb.hi[0] && a.j <= fb.hi[1] && a.k <= fb.hi[2];
+  return a;
 }
 
-// Upwind HJ WENO5 (spatial_derivatives3d.f.in:2628-2996): the side is chosen
-// on the differences, so lanes of both signs share one reconstruction.
-__global__ void __launch_bounds__(256) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx, View<const R> vy,
-                                                         View<const R> vz, Box fb, R ix, R iy, R iz) {
-  LSMGPU_CELL_INDEX(fb, i, j, k);
-  const R *c = phi.p + phi.off(i, j, k);
-#pragma unroll 1
-  for (int d = 0; d < 3; d++) {
-    const R u = (d == 0 ? vx : (d == 1 ? vy : vz))(i, j, k);
-    const long long s = phi.stride(d);
-    R out = R(0);
-    if (!(fabs(u) < Consts<R>::zero_tol) && s != 0) {
-      // phi(c-3) is read by the minus side only, phi(c+3) by the plus side only
-      R D[6], v[5];
-      line_diffs(D, c, s);
+__global__ void __launch_bounds__(256, 5) k_hj_pm_weno5(Out3 plus, Out3 minus, View<const R> phi, Box fb, unsigned axes,
+                                                        R ix, R iy, R iz) {
+  const AxisCell a = axis_cell(fb, axes);
+  if (!a.in) return;
+  R D[6], gp, gm;
+  line_diffs(D, phi.p + phi.off(a.i, a.j, a.k), phi.stride(a.d));
+  weno5_pm64(D, wide64(a.d == 0 ? ix : (a.d == 1 ? iy : iz)), Consts<R>::tiny, gp, gm);
+  plus.at(a.d, a.i, a.j, a.k) = gp;
+  minus.at(a.d, a.i, a.j, a.k) = gm;
+}
+
+// Upwind HJ WENO5 (spatial_derivatives3d.f.in:2628-2996).  The plus side is
+// the minus side of the mirrored line, negated (every rounding is symmetric),
+// so a lane walks its line with the stride's sign and lanes of both sides run
+// the same reconstruction.
+__global__ void __launch_bounds__(256, 5) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx,
+                                                            View<const R> vy, View<const R> vz, Box fb, unsigned axes,
+                                                            R ix, R iy, R iz) {
+  const AxisCell a = axis_cell(fb, axes);
+  if (!a.in) return;
+  const R u = (a.d == 0 ? vx : (a.d == 1 ? vy : vz))(a.i, a.j, a.k);
+  R out = R(0);
+  if (!below_(u, R(Consts<R>::zero_tol))) {
+    const bool pos = is_pos_(u);
+    const R *c = phi.p + phi.off(a.i, a.j, a.k);
+    const long long s = pos ? phi.stride(a.d) : -phi.stride(a.d);
+    R x[6], D[5];
 #pragma unroll
-      for (int q = 0; q < 5; q++) v[q] = u > R(0) ? D[q] : D[5 - q];
-      out = weno5_side64(v, wide64(d == 0 ? ix : (d == 1 ? iy : iz)), Consts<R>::tiny);
-    }
-    g.at(d, i, j, k) = out;
+    for (int q = 0; q < 6; q++) x[q] = __ldg(c + (q - 3) * s);
+#pragma unroll
+    for (int q = 0; q < 5; q++) D[q] = x[q + 1] - x[q];
+    out = flip_if_(weno5_side64(D, wide64(a.d == 0 ? ix : (a.d == 1 ? iy : iz)), Consts<R>::tiny), !pos);
   }
+  g.at(a.d, a.i, a.j, a.k) = out;
 }
 
 template <int S>
@@ -179,9 +188,10 @@ void hj_pm(const char *name, R *pxp, R *pyp, R *pzp, const Box &pb, R *pxm, R *p
   View<const R> ph = view((const R *)call.in(phi, phb.size()), phb);
   if (!call.ok()) return;
   Grid3 g = cover(fb);
-  if constexpr (S == WENO5)
-    LSMGPU_LAUNCH(k_hj_pm_weno5, g.grid, g.block, 0, P, M, ph, fb, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
-  else
+  if constexpr (S == WENO5) {
+    g.grid.x *= g_lift_dims;
+    LSMGPU_LAUNCH(k_hj_pm_weno5, g.grid, g.block, 0, P, M, ph, fb, g_lift_dims, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
+  } else
     LSMGPU_LAUNCH(k_hj_pm<S>, g.grid, g.block, 0, P, M, ph, fb, R(1.0) / dx, R(1.0) / dy, R(1.0) / dz);
   call.finish();
 }
@@ -203,10 +213,11 @@ void hj_upwind(const char *name, R *px, R *py, R *pz, const Box &gb, const R *ph
   View<const R> VZ = view((const R *)call.in(vz, nv), vb);
   if (!call.ok()) return;
   Grid3 g = cover(fb);
-  if constexpr (S == WENO5)
-    LSMGPU_LAUNCH(k_hj_upwind_weno5, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, R(1.0) / dx, R(1.0) / dy,
+  if constexpr (S == WENO5) {
+    g.grid.x *= g_lift_dims;
+    LSMGPU_LAUNCH(k_hj_upwind_weno5, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, g_lift_dims, R(1.0) / dx, R(1.0) / dy,
                   R(1.0) / dz);
-  else
+  } else
     LSMGPU_LAUNCH(k_hj_upwind<S>, g.grid, g.block, 0, G, ph, VX, VY, VZ, fb, R(1.0) / dx, R(1.0) / dy,
                   R(1.0) / dz);
   call.finish();
@@ -244,14 +255,7 @@ __global__ void k_laplacian2(View<R> lap, View<const R> phi, Box fb, R ix, R iy,
 
 __global__ void k_gradmag(View<const R> px, View<const R> py, View<const R> pz, View<R> mag, Box fb) {
   LSMGPU_CELL_INDEX(fb, i, j, k);
-  const R tol = R(1.e-8);
-  R x = px(i, j, k), y = py(i, j, k), z = pz(i, j, k);
-  R x2 = x * x, y2 = y * y, z2 = z * z;
-  if (x2 < tol) x2 = R(0);
-  if (y2 < tol) y2 = R(0);
-  if (z2 < tol) z2 = R(0);
-  const R t = sqrt(x2 + y2 + z2);
-  mag(i, j, k) = (t < tol) ? R(0) : t;
+  mag(i, j, k) = grad_magnitude(px(i, j, k), py(i, j, k), pz(i, j, k), R(1.e-8));
 }
 
 // ---- RK stages ---------------------------------------------------------------
@@ -264,10 +268,11 @@ __global__ void k_rk(View<R> out, View<const R> a, View<const R> u, View<const R
   LSMGPU_CELL_INDEX(fb, i, j, k);
   const R L = rhs(i, j, k);
   R v;
-  if (KIND == 0) v = u(i, j, k) + dt * L;
-  if (KIND == 1) v = R(0.5) * (u(i, j, k) + a(i, j, k) + dt * L);
-  if (KIND == 2) v = R(0.75) * u(i, j, k) + R(0.25) * (a(i, j, k) + dt * L);
-  if (KIND == 3) v = R(1.0 / 3.0) * u(i, j, k) + R(2.0 / 3.0) * (a(i, j, k) + dt * L);
+  const R w = mul_(dt, L);
+  if (KIND == 0) v = u(i, j, k) + w;
+  if (KIND == 1) v = R(0.5) * (u(i, j, k) + a(i, j, k) + w);
+  if (KIND == 2) v = fma(R(0.25), a(i, j, k) + w, mul_(R(0.75), u(i, j, k)));  // the product by 1/4 is exact
+  if (KIND == 3) v = mul_(R(1.0 / 3.0), u(i, j, k)) + mul_(R(2.0 / 3.0), a(i, j, k) + w);
   out(i, j, k) = v;
 }
 
@@ -298,8 +303,8 @@ __global__ void k_fill(View<R> a, Box b, R v) {
 __global__ void k_add_advection(View<R> rhs, View<const R> px, View<const R> py, View<const R> pz,
                                 View<const R> vx, View<const R> vy, View<const R> vz, Box fb) {
   LSMGPU_CELL_INDEX(fb, i, j, k);
-  rhs(i, j, k) = rhs(i, j, k) - (vx(i, j, k) * px(i, j, k) + vy(i, j, k) * py(i, j, k) +
-                                 vz(i, j, k) * pz(i, j, k));
+  rhs(i, j, k) = rhs(i, j, k) - (mul_(vx(i, j, k), px(i, j, k)) + mul_(vy(i, j, k), py(i, j, k)) +
+                                 mul_(vz(i, j, k), pz(i, j, k)));
 }
 
 // vn field (const_vn == false) or constant (const_vn == true)
@@ -308,10 +313,10 @@ __global__ void k_add_normal(View<R> rhs, View<const R> pxp, View<const R> pyp, 
                              View<const R> vn, bool const_vn, R vn_const, Box fb) {
   LSMGPU_CELL_INDEX(fb, i, j, k);
   const R w = const_vn ? vn_const : vn(i, j, k);
-  if (!(fabs(w) >= Consts<R>::zero_tol)) return;
+  if (!at_least_(w, R(Consts<R>::zero_tol))) return;
   const R p[3] = {pxp(i, j, k), pyp(i, j, k), pzp(i, j, k)};
   const R m[3] = {pxm(i, j, k), pym(i, j, k), pzm(i, j, k)};
-  rhs(i, j, k) = rhs(i, j, k) - w * sqrt(godunov_normal_sq(w > R(0), p, m));
+  rhs(i, j, k) = rhs(i, j, k) - mul_(w, sqrt_(godunov_normal_sq(is_pos_(w), p, m)));
 }
 
 __global__ void k_add_const_curv(View<R> rhs, View<const R> px, View<const R> py, View<const R> pz,
@@ -319,16 +324,16 @@ __global__ void k_add_const_curv(View<R> rhs, View<const R> px, View<const R> py
                                  View<const R> pyy, View<const R> pyz, View<const R> pzz, R b, Box fb) {
   LSMGPU_CELL_INDEX(fb, i, j, k);
   const R x = px(i, j, k), y = py(i, j, k), z = pz(i, j, k);
-  const R m2 = x * x + y * y + z * z;
+  const R m2 = sqr_(x) + sqr_(y) + sqr_(z);
   R curv;
-  if (m2 < Consts<R>::zero_tol) {
+  if (below_(m2, R(Consts<R>::zero_tol))) {
     curv = R(0);
   } else {
     curv = curv_numerator(pxx(i, j, k), pyy(i, j, k), pzz(i, j, k), pxy(i, j, k), pxz(i, j, k),
                           pyz(i, j, k), x, y, z);
-    curv = curv / m2;
+    curv = div_(curv, m2);
   }
-  rhs(i, j, k) = rhs(i, j, k) + b * curv;
+  rhs(i, j, k) = rhs(i, j, k) + mul_(b, curv);
 }
 
 // ---- reinitialization --------------------------------------------------------
@@ -349,20 +354,8 @@ __global__ void k_mean_curv2(View<R> kappa, View<const R> phi, View<const R> px,
   LSMGPU_CELL_INDEX(fb, i, j, k);
   const R *c = phi.p + phi.off(i, j, k);
   const long long sx = 1, sy = phi.s1, sz = phi.s2;
-  const R xx = (c[sx] - R(2.0) * c[0] + c[-sx]) * fxx;
-  const R yy = (c[sy] - R(2.0) * c[0] + c[-sy]) * fyy;
-  const R zz = (c[sz] - R(2.0) * c[0] + c[-sz]) * fzz;
-  const R xy = (c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy]) * fxy;
-  const R xz = (c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz]) * fxz;
-  const R yz = (c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz]) * fyz;
-  const R g = mag(i, j, k);
-  const R den = g * g * g;
-  R out;
-  if (den < Consts<R>::zero_tol)
-    out = R(0);
-  else
-    out = curv_numerator(xx, yy, zz, xy, xz, yz, px(i, j, k), py(i, j, k), pz(i, j, k)) / den;
-  kappa(i, j, k) = out;
+  kappa(i, j, k) = mean_curvature2(c, sx, sy, sz, px(i, j, k), py(i, j, k), pz(i, j, k), mag(i, j, k), fxx, fyy, fzz,
+                                   fxy, fxz, fyz);
 }
 
 // Gaussian curvature (order 2, 4) and mean curvature (order 4): the order-2
@@ -390,17 +383,20 @@ __device__ __forceinline__ R okey_inv(unsigned long long k) {
   return __longlong_as_double((long long)u);
 }
 
-__device__ __forceinline__ void block_max_commit(R v, unsigned long long *key) {
-  for (int o = 16; o > 0; o >>= 1) v = rmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __shared__ R part[32];
+// Maximum of the keys of a block of whole warps into *key.  On keys the
+// shuffles and comparisons are integer work (an FP64 comparison holds the
+// FP64 pipe for some 64 cycles).  The running key only grows, so a block that
+// cannot raise the value it reads skips the atomic.
+__device__ __forceinline__ void block_max_commit(unsigned long long v, unsigned long long *key) {
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __shared__ unsigned long long part[32];
   const int t = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int nt = blockDim.x * blockDim.y * blockDim.z;
   if ((t & 31) == 0) part[t >> 5] = v;
   __syncthreads();
-  if (t < 32) {
-    R w = (t < (nt + 31) / 32) ? part[t] : R(-1.0e308);
-    for (int o = 16; o > 0; o >>= 1) w = rmax(w, __shfl_xor_sync(0xffffffffu, w, o));
-    if (t == 0) atomicMax(key, okey(w));
+  if (t == 0) {
+    for (int q = 1; q < nt / 32; q++) v = max(v, part[q]);
+    if (v > __ldcg(key)) atomicMax(key, v);
   }
 }
 
@@ -420,32 +416,39 @@ struct RedArgs {
   R vn_const, ix, iy, iz, max_dx_sq;
 };
 
+constexpr int kRedZ = 8;  // planes a thread walks: fewer blocks to fold, more loads in flight
+
 template <int MODE>
-__global__ void k_reduce_max(RedArgs A, Box ib, unsigned long long *key) {
-  const int i = ib.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = ib.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = ib.lo[2] + blockIdx.z * blockDim.z + threadIdx.z;
-  R v = R(-1.0e308);
-  bool take = i <= ib.hi[0] && j <= ib.hi[1] && k <= ib.hi[2];
-  if (take && A.cv_sgn != 0 && !(MODE == 3 && i == ib.lo[0] && j == ib.lo[1] && k == ib.lo[2])) {
-    const R c = A.cv(i, j, k);
-    take = A.cv_sgn > 0 ? c > R(0) : c < R(0);
-  }
-  if (take) {
-    if (MODE == 0) {
-      v = fabs(A.a(i, j, k)) * A.ix + fabs(A.b(i, j, k)) * A.iy + fabs(A.c(i, j, k)) * A.iz;
-    } else if (MODE == 3) {
-      v = fabs(A.a(i, j, k) - A.b(i, j, k));
-    } else {
-      const R avn = (MODE == 2) ? fabs(A.vn_const) : fabs(A.vn(i, j, k));
-      const R cx = rmax(fabs(A.pxp(i, j, k)), fabs(A.pxm(i, j, k)));
-      const R cy = rmax(fabs(A.pyp(i, j, k)), fabs(A.pym(i, j, k)));
-      const R cz = rmax(fabs(A.pzp(i, j, k)), fabs(A.pzm(i, j, k)));
-      const R ng = sqrt(cx * cx + cy * cy + cz * cz + A.max_dx_sq);
-      v = avn / ng * (cx * A.ix + cy * A.iy + cz * A.iz);
+__global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned long long *key) {
+  const int i = ib.lo[0] + blockIdx.x * 32 + threadIdx.x;
+  const int j = ib.lo[1] + blockIdx.y * 8 + threadIdx.y;
+  const int k0 = ib.lo[2] + blockIdx.z * kRedZ;
+  unsigned long long best = okey(R(-1.0e308));
+  if (i <= ib.hi[0] && j <= ib.hi[1]) {
+#pragma unroll 4
+    for (int k = k0; k < k0 + kRedZ && k <= ib.hi[2]; k++) {
+      if (A.cv_sgn != 0 && !(MODE == 3 && i == ib.lo[0] && j == ib.lo[1] && k == ib.lo[2])) {
+        const R c = A.cv(i, j, k);
+        if (!is_pos_(flip_if_(c, A.cv_sgn < 0))) continue;
+      }
+      R v;
+      if (MODE == 0) {
+        v = mul_(abs_(A.a(i, j, k)), A.ix) + mul_(abs_(A.b(i, j, k)), A.iy) + mul_(abs_(A.c(i, j, k)), A.iz);
+      } else if (MODE == 3) {
+        v = abs_(A.a(i, j, k) - A.b(i, j, k));
+      } else {
+        const R avn = abs_((MODE == 2) ? A.vn_const : A.vn(i, j, k));
+        const R cx = max_nonneg_(abs_(A.pxp(i, j, k)), abs_(A.pxm(i, j, k)));
+        const R cy = max_nonneg_(abs_(A.pyp(i, j, k)), abs_(A.pym(i, j, k)));
+        const R cz = max_nonneg_(abs_(A.pzp(i, j, k)), abs_(A.pzm(i, j, k)));
+        const R ng = sqrt_(sqr_(cx) + sqr_(cy) + sqr_(cz) + A.max_dx_sq);
+        v = mul_(div_(avn, ng), mul_(cx, A.ix) + mul_(cy, A.iy) + mul_(cz, A.iz));
+      }
+      // a NaN exceeds nothing (the reference's comparison is false)
+      if (fpi::mag(v) <= fpi::kInfBits) best = max(best, okey(v));
     }
   }
-  block_max_commit(v, key);
+  block_max_commit(best, key);
 }
 
 // final scalar: mode 0-2 give dt = cfl/(max + tiny) with the running max
@@ -468,8 +471,9 @@ void reduce_max(Call &call, RedArgs &A, const Box &ib, R *out, R cfl, R init) {
   if (!call.ok()) return;
   LSMGPU_LAUNCH(k_set_key, 1, 1, 0, key, init);
   if (!ib.empty()) {
-    Grid3 g = cover(ib);
-    LSMGPU_LAUNCH(k_reduce_max<MODE>, g.grid, g.block, 0, A, ib, key);
+    const dim3 grd((unsigned)((ib.n(0) + 31) / 32), (unsigned)((ib.n(1) + 7) / 8),
+                   (unsigned)((ib.n(2) + kRedZ - 1) / kRedZ));
+    LSMGPU_LAUNCH(k_reduce_max<MODE>, grd, dim3(32, 8), 0, A, ib, key);
   }
   LSMGPU_LAUNCH(k_finish_scalar, 1, 1, 0, key, dout, MODE, cfl, init);
   call.finish();

@@ -203,14 +203,9 @@ constexpr bool uses_reinit_x2() {
   return !EXACT && sizeof(R) == 4 && MODE == REINIT;
 }
 
-// Tile depth of the FP32 k_stage_f32 launches of a grid: 8, or 4 where the
-// 4-plane tiles fill whole waves of resident CTAs at least 10% better (a
-// partly filled last wave costs a whole one; five CTAs per SM at either
-// depth; a grid of less than one wave gets twice the CTAs).  At 128^3, 1024
-// 8-plane tiles are 1.35 waves on 152 SMs, 2048 4-plane tiles 2.7; at 192^3
-// and 256^3 both depths fill their waves equally and 8 is kept.
-inline int stage_tz_f32(const Layout &L) {
-  static int sms_of[64] = {};  // SM count per device, read once
+// SM count of the current device
+inline int sm_count() {
+  static int sms_of[64] = {};  // per device, read once
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
     if (sms_of[dev] == 0) {
@@ -221,7 +216,16 @@ inline int stage_tz_f32(const Layout &L) {
   } else {
     cudaGetLastError();
   }
-  const long long slots = 5LL * sms;
+  return sms;
+}
+// Tile depth of the FP32 k_stage_f32 launches of a grid: 8, or 4 where the
+// 4-plane tiles fill whole waves of resident CTAs at least 10% better (a
+// partly filled last wave costs a whole one; five CTAs per SM at either
+// depth; a grid of less than one wave gets twice the CTAs).  At 128^3, 1024
+// 8-plane tiles are 1.35 waves on 152 SMs, 2048 4-plane tiles 2.7; at 192^3
+// and 256^3 both depths fill their waves equally and 8 is kept.
+inline int stage_tz_f32(const Layout &L) {
+  const long long slots = 5LL * sm_count();
   const long long cols = (long long)((L.nx + TX - 1) / TX) * ((L.ny + TY - 1) / TY);
   auto eff = [&](int tz) {
     const long long tiles = cols * ((L.nz + tz - 1) / tz);
@@ -229,6 +233,20 @@ inline int stage_tz_f32(const Layout &L) {
     return (double)L.nz / ((double)waves * slots * tz / (double)cols);  // used fraction of the wave slots
   };
   return eff(4) > 1.1 * eff(8) ? 4 : 8;
+}
+
+// Tile depth of the FP64 k_stage launches: the arithmetic of one plane takes
+// far longer than its share of the tile load, so shallow tiles cost nothing
+// and only the tail of the launch matters: 4 planes where the grid still has
+// 16 tiles per resident CTA slot (four per SM), else 2, else 1.  (8 where 4
+// would exceed the grid's z extent limit.)
+inline int stage_tz_f64(const Layout &L) {
+  const long long slots = 4LL * sm_count();
+  const long long cols = (long long)((L.nx + TX - 1) / TX) * ((L.ny + TY - 1) / TY);
+  if (L.nz > 4 * 65535) return 8;
+  for (int tz = 4; tz > 1; tz /= 2)
+    if (cols * ((L.nz + tz - 1) / tz) >= 16 * slots) return tz;
+  return 1;
 }
 
 // Tensor map of a padded work buffer with the staged box of the stage kernel
@@ -240,7 +258,7 @@ bool encode_stage_tmap(CUtensorMap *m, const R *p, const Layout &L) {
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, RSX, RSY, RZ + 6);
   if constexpr (!EXACT && sizeof(R) == 4)
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f32(L) + 6);
-  return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, SZ);
+  return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f64(L) + 6);
 }
 
 // Launches one stage kernel; with prepare_only it only sets the kernel's
@@ -286,8 +304,9 @@ static void launch_stage(const CUtensorMap &tm, const StageArgs<R> &a, bool prep
     if (tz == 4) k_stage_f32<MODE, 4><<<grd, blk, smem, stream()>>>(tm, a);
     else k_stage_f32<MODE, 8><<<grd, blk, smem, stream()>>>(tm, a);
   } else {
-    dim3 grd((unsigned)((L.nx + TX - 1) / TX), (unsigned)((L.ny + TY - 1) / TY), (unsigned)((L.nz + TZ - 1) / TZ));
-    k_stage<R, MODE, EXACT><<<grd, blk, (size_t)SX * SY * SZ * sizeof(R), stream()>>>(tm, a);
+    const int tz = stage_tz_f64(L);
+    dim3 grd((unsigned)((L.nx + TX - 1) / TX), (unsigned)((L.ny + TY - 1) / TY), (unsigned)((L.nz + tz - 1) / tz));
+    k_stage<R, MODE, EXACT><<<grd, blk, (size_t)SX * SY * (tz + 6) * sizeof(R), stream()>>>(tm, a, tz);
   }
   note_launch();
 }

@@ -8,7 +8,7 @@
 // layers in y and z; rows padded to a multiple of 32 elements so each row
 // starts on a 128-byte boundary.  A CTA of 32 x 8 threads owns a 32 x 8 x 8
 // tile and stages the tile plus its 3-cell halo (40 x 14 x 14 elements) into
-// shared memory with one 3D TMA load; the x origin of the box is the tile's
+// shared memory with one 3D TMA load (the FP64 stage: 1 to 4 planes per tile); the x origin of the box is the tile's
 // 32-aligned row offset, which satisfies TMA's 16-byte rule for both element
 // sizes.  Each thread then walks the 8 cells of its z column.
 //
@@ -197,14 +197,19 @@ __device__ __forceinline__ R reinit_term(R pc, const R gp[3], const R gm[3], R d
 // ---------------------------------------------------------------------------
 // the stage kernel
 // ---------------------------------------------------------------------------
+// The FP64 stage.  Bound by its arithmetic (weno64.cuh: the FP64 pipe with the
+// integer pipes close behind), so the tile only has to be there in time: tiles
+// of `tz` planes (1 to 4, chosen by the launcher so that the last wave of
+// tiles is a small part of the run), four CTAs per SM at 64 registers.
 template <class R, int MODE, bool EXACT>
-__global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUtensorMap tm, StageArgs<R> a) {
+__global__ void __launch_bounds__(TX * TY, MODE == REINIT ? 4 : 5) k_stage(const __grid_constant__ CUtensorMap tm, StageArgs<R> a, int tzn) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R *tile = reinterpret_cast<R *>(smem_raw);
   __shared__ __align__(8) uint64_t bar;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + TX * ty;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
+  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * tzn;
+  const int szn = tzn + 6;
 
   if (tid == 0) {
     prefetch_tmap(&tm);
@@ -213,7 +218,7 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
   }
   __syncthreads();
   if (tid == 0) {
-    mbar_arrive_expect_tx(&bar, (uint32_t)(SX * SY * SZ * sizeof(R)));
+    mbar_arrive_expect_tx(&bar, (uint32_t)(SX * SY * szn * sizeof(R)));
     // padded coordinates of interior cell (x0 - 4, y0 - 3, z0 - 3)
     tma_load_3d(tile, &tm, x0 + GX - 4, y0 + GY - 3, z0 + GZ - 3, &bar);
   }
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
     return;
   }
   if (a.ghost) {
-    fill_face_ghosts<R>(tile, SX, SY, SZ, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
+    fill_face_ghosts<R>(tile, SX, SY, szn, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
     __syncthreads();
   }
 
@@ -231,9 +236,7 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
   const int i = x0 + tx, j = y0 + ty;
   if (i >= L.nx || j >= L.ny) return;
   const int sx = tx + 4, sy = ty + 3;
-  const int kmax = min(TZ, L.nz - z0);
-  const Wide64 wide[3] = {wide64(a.inv[0]), wide64(a.inv[1]), wide64(a.inv[2])};
-  const int st[3] = {1, SX, SX * SY};
+  const int kmax = min(tzn, L.nz - z0);
 
   for (int tz = 0; tz < kmax; tz++) {
     const int k = z0 + tz;
@@ -245,13 +248,13 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
       R n2 = R(0);
 #pragma unroll 1
       for (int d = 0; d < 3; d++) {
-        const int s = st[d];
+        const int s = d == 0 ? 1 : (d == 1 ? SX : SX * SY);
         R D[6], gp, gm;  // D1(c-2 .. c+3)
 #pragma unroll
         for (int f = -2; f <= 3; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
-        weno5_pm64(D, wide[d], Consts<R>::tiny, gp, gm);
+        weno5_pm64(D, wide64(a.inv[d]), Consts<R>::tiny, gp, gm);
         const R t = reinit_axis(pc, gp, gm);
-        n2 = d == 0 ? t * t : n2 + t * t;
+        n2 = d == 0 ? sqr_(t) : n2 + sqr_(t);
       }
       rhs = reinit_from_sq<R>(pc, n2, a.dx_sq, a.use0 != 0);
     } else {
@@ -259,19 +262,19 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
 #pragma unroll 1
       for (int d = 0; d < 3; d++) {
         // spatial_derivatives3d.f.in:2756-2812: |v| < zero_tol gives 0, v > 0
-        // takes the backward stencil, otherwise the forward one
+        // takes the backward stencil, otherwise the forward one, which is
+        // the backward one of the mirrored line, negated: v g = |v| g'
         const R u = (MODE == ADV_CONST) ? a.vconst[d] : a.vel[d][L.idx(i, j, k)];
-        const int s = st[d];
         R g = R(0);
-        if (!(fabs(u) < Consts<double>::zero_tol)) {
-          R D[6], v[5];
+        if (!below_(u, R(Consts<double>::zero_tol))) {
+          const int s0 = d == 0 ? 1 : (d == 1 ? SX : SX * SY), s = is_pos_(u) ? s0 : -s0;
+          R D[5];
 #pragma unroll
-          for (int f = -2; f <= 3; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
-#pragma unroll
-          for (int q = 0; q < 5; q++) v[q] = u > R(0) ? D[q] : D[5 - q];
-          g = weno5_side64(v, wide[d], Consts<R>::tiny);
+          for (int f = -2; f <= 2; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
+          g = weno5_side64(D, wide64(a.inv[d]), Consts<R>::tiny);
         }
-        dot = d == 0 ? u * g : dot + u * g;
+        const R t = mul_(abs_(u), g);
+        dot = d == 0 ? t : dot + t;
       }
       // lsm3dZeroOutLevelSetEqnRHS then lsm3dAddAdvectionTermToLSERHS
       // (level_set_evolution3d.f.in:38, :113-116)
@@ -279,14 +282,9 @@ __global__ void __launch_bounds__(TX * TY) k_stage(const __grid_constant__ CUten
     }
 
     const long long cell = L.idx(i, j, k);
-    R u;
-    if (a.stage == 1) {
-      u = c[0] + a.dt * rhs;  // tvd_runge_kutta3d.f:78
-    } else if (a.stage == 2) {
-      u = R(0.75) * a.phi_n[cell] + R(0.25) * (c[0] + a.dt * rhs);  // :403-404
-    } else {
-      u = R(1.0 / 3.0) * a.phi_n[cell] + R(2.0 / 3.0) * (c[0] + a.dt * rhs);  // :490-492
-    }
+    R u = c[0] + mul_(a.dt, rhs);  // tvd_runge_kutta3d.f:78
+    if (a.stage == 2) u = fma(R(0.25), u, mul_(R(0.75), a.phi_n[cell]));  // :403-404 (u / 4 is exact)
+    if (a.stage == 3) u = mul_(R(1.0 / 3.0), a.phi_n[cell]) + mul_(R(2.0 / 3.0), u);  // :490-492
     a.out[cell] = u;
 
     if (a.periodic) {

@@ -597,13 +597,7 @@ void lsm3dgradientmagnitudelocal_(const R *phi_x, const R *phi_y, const R *phi_z
   if (!lc.c.ok()) return;
   for_list(L, *nlo, *nhi, [=] __device__(int i, int j, int k) {
     if (!g(i, j, k)) return;
-    const R tol = Consts<R>::zero_tol;
-    R x2 = X(i, j, k) * X(i, j, k), y2 = Y(i, j, k) * Y(i, j, k), z2 = Z(i, j, k) * Z(i, j, k);
-    if (x2 < tol) x2 = R(0);
-    if (y2 < tol) y2 = R(0);
-    if (z2 < tol) z2 = R(0);
-    const R t = sqrt(x2 + y2 + z2);
-    O(i, j, k) = (t < tol) ? R(0) : t;
+    O(i, j, k) = grad_magnitude(X(i, j, k), Y(i, j, k), Z(i, j, k), R(Consts<R>::zero_tol));
   });
   lc.c.finish();
 }
@@ -736,11 +730,11 @@ void lsm3daddconstcurvtermtolserhslocal_(R *lse_rhs, BOXARG(r), const R *phi_x, 
   for_list(L, *nlo, *nhi, [=] __device__(int i, int j, int k) {
     if (!g(i, j, k)) return;
     const R x = X(i, j, k), y = Y(i, j, k), z = Z(i, j, k);
-    const R m2 = x * x + y * y + z * z;
+    const R m2 = sqr_(x) + sqr_(y) + sqr_(z);
     R curv = R(0);
-    if (!(m2 < Consts<R>::zero_tol))
-      curv = curv_numerator(XX(i, j, k), YY(i, j, k), ZZ(i, j, k), XY(i, j, k), XZ(i, j, k), YZ(i, j, k), x, y, z) / m2;
-    O(i, j, k) = O(i, j, k) + bb * curv;
+    if (!below_(m2, R(Consts<R>::zero_tol)))
+      curv = div_(curv_numerator(XX(i, j, k), YY(i, j, k), ZZ(i, j, k), XY(i, j, k), XZ(i, j, k), YZ(i, j, k), x, y, z), m2);
+    O(i, j, k) = O(i, j, k) + mul_(bb, curv);
   });
   lc.c.finish();
 }
@@ -789,17 +783,7 @@ void lsm3dcomputemeancurvatureorder2local_(R *kappa, BOXARG(k), const R *phi, BO
     if (!g(i, j, k)) return;
     const R *c = F.p + F.off(i, j, k);
     const long long sx = 1, sy = F.s1, sz = F.s2;
-    const R xx = (c[sx] - R(2.0) * c[0] + c[-sx]) * fxx;
-    const R yy = (c[sy] - R(2.0) * c[0] + c[-sy]) * fyy;
-    const R zz = (c[sz] - R(2.0) * c[0] + c[-sz]) * fzz;
-    const R xy = (c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy]) * fxy;
-    const R xz = (c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz]) * fxz;
-    const R yz = (c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz]) * fyz;
-    const R gg = G(i, j, k);
-    const R den = gg * gg * gg;
-    K(i, j, k) = (den < Consts<R>::zero_tol)
-                     ? R(0)
-                     : curv_numerator(xx, yy, zz, xy, xz, yz, X(i, j, k), Y(i, j, k), Z(i, j, k)) / den;
+    K(i, j, k) = mean_curvature2(c, sx, sy, sz, X(i, j, k), Y(i, j, k), Z(i, j, k), G(i, j, k), fxx, fyy, fzz, fxy, fxz, fyz);
   });
   lc.c.finish();
 }

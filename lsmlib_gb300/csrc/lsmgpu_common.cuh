@@ -150,6 +150,10 @@ struct Grid3 {
 };
 inline Grid3 cover(const Box &fb, int bx = 32, int by = 4, int bz = 2) {
   Grid3 g;
+  // one plane (a 2D call) or one row (1D): the block's threads go to the
+  // axes that are there
+  if (fb.n(2) == 1) { by *= bz; bz = 1; }
+  if (fb.n(2) == 1 && fb.n(1) == 1) { bx *= by; by = 1; }
   g.block = dim3(bx, by, bz);
   g.grid = dim3((unsigned)((fb.n(0) + bx - 1) / bx), (unsigned)((fb.n(1) + by - 1) / by),
                 (unsigned)((fb.n(2) + bz - 1) / bz));

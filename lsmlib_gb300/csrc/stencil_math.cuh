@@ -13,6 +13,10 @@
 // D1(c+f) = a[f+3] - a[f+2].
 #pragma once
 
+#include <type_traits>
+
+#include "fp64_int.cuh"
+
 namespace lsmgpu {
 
 template <class R>
@@ -110,22 +114,90 @@ __device__ __forceinline__ R eno3_minus(const Diffs<R> &d, R inv) {
   return x * inv;
 }
 
+// The FP64 forms below keep their products, quotients, square roots and
+// comparisons off the FP64 pipe (fp64_int.cuh); same bits.
+template <class R>
+__device__ __forceinline__ R mul_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::mul_any(a, b);
+  else return a * b;
+}
+template <class R>
+__device__ __forceinline__ R sqr_(R a) {
+  if constexpr (std::is_same<R, double>::value) return fpi::sqr_any(a);
+  else return a * a;
+}
+template <class R>
+__device__ __forceinline__ R div_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::div_any(a, b);
+  else return a / b;
+}
+template <class R>
+__device__ __forceinline__ R sqrt_(R a) {
+  if constexpr (std::is_same<R, double>::value) return fpi::sqrt_any(a);
+  else return sqrt(a);
+}
+// |a|; a or -a; a > 0; a > 0 ? a : 0; a > b ? a : b of values not negative; a < b, |a| < b
+// and |a| >= b for a constant b > 0
+template <class R>
+__device__ __forceinline__ bool is_pos_(R a) {
+  if constexpr (std::is_same<R, double>::value) return fpi::is_positive(a);
+  else return a > R(0);
+}
+template <class R>
+__device__ __forceinline__ R abs_(R a) {
+  if constexpr (std::is_same<R, double>::value) return fpi::abs_bits(a);
+  else return fabs(a);
+}
+template <class R>
+__device__ __forceinline__ R flip_if_(R a, bool flip) {
+  if constexpr (std::is_same<R, double>::value) return fpi::flip_if(a, flip);
+  else return flip ? -a : a;
+}
+template <class R>
+__device__ __forceinline__ R pos_part_(R a) { return is_pos_(a) ? a : R(0); }
+template <class R>
+__device__ __forceinline__ R max_nonneg_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::max_nonneg(a, b);
+  else return rmax(a, b);
+}
+template <class R>
+__device__ __forceinline__ bool less_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::less_than(a, b);
+  else return a < b;
+}
+template <class R>
+__device__ __forceinline__ bool below_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::below(a, b);
+  else return fabs(a) < b;
+}
+template <class R>
+__device__ __forceinline__ bool at_least_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::at_least(a, b);
+  else return fabs(a) >= b;
+}
+
 // Godunov |grad phi|^2 of level_set_evolution3d.f.in:210-223 for normal
-// speed sign `pos` (vn > 0).
+// speed sign `pos` (vn > 0).  The FP64 form takes the larger of the two
+// one-sided magnitudes before squaring (rounding is monotone: same bits).
 template <class R>
 __device__ __forceinline__ R godunov_normal_sq(bool pos, const R p[3], const R m[3]) {
   R s = R(0);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    R a, b;
-    if (pos) {
-      a = rmax(m[d], R(0));
-      b = rmin(p[d], R(0));
+    R t;
+    if constexpr (std::is_same<R, double>::value) {
+      t = sqr_(max_nonneg_(pos_part_(flip_if_(m[d], !pos)), pos_part_(flip_if_(p[d], pos))));
     } else {
-      a = rmin(m[d], R(0));
-      b = rmax(p[d], R(0));
+      R a, b;
+      if (pos) {
+        a = rmax(m[d], R(0));
+        b = rmin(p[d], R(0));
+      } else {
+        a = rmin(m[d], R(0));
+        b = rmax(p[d], R(0));
+      }
+      t = rmax(a * a, b * b);
     }
-    const R t = rmax(a * a, b * b);
     s = (d == 0) ? t : s + t;
   }
   return s;
@@ -137,35 +209,92 @@ __device__ __forceinline__ R godunov_normal_sq(bool pos, const R p[3], const R m
 // their squares (taken in axis order), and both together.
 template <class R>
 __device__ __forceinline__ R reinit_axis(R pc, R gp, R gm) {
-  R u, w;
-  if (pc > R(0)) {
-    u = rmax(-gp, R(0));
-    w = rmax(gm, R(0));
-  } else {
-    u = rmax(gp, R(0));
-    w = rmax(-gm, R(0));
-  }
-  return rmax(u, w);
+  const bool pos = is_pos_(pc);
+  return max_nonneg_(pos_part_(flip_if_(gp, pos)), pos_part_(flip_if_(gm, !pos)));
 }
 template <class R>
 __device__ __forceinline__ R reinit_from_sq(R pc, R n2, R dx_sq, bool use0) {
-  if (!(fabs(pc) >= Consts<R>::zero_tol)) return R(0);
-  const R sgn = use0 ? pc / sqrt(pc * pc + dx_sq) : pc / sqrt(pc * pc + n2 * dx_sq);
-  return sgn * (R(1.0) - sqrt(n2));
+  if (!at_least_(pc, R(Consts<R>::zero_tol))) return R(0);
+  const R q = sqr_(pc) + (use0 ? dx_sq : mul_(n2, dx_sq));
+  return mul_(div_(pc, sqrt_(q)), R(1.0) - sqrt_(n2));
 }
 template <class R>
 __device__ __forceinline__ R reinit_rhs(R pc, const R gp[3], const R gm[3], R dx_sq, bool use0) {
   R st[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) st[d] = reinit_axis(pc, gp[d], gm[d]);
-  return reinit_from_sq(pc, st[0] * st[0] + st[1] * st[1] + st[2] * st[2], dx_sq, use0);
+  return reinit_from_sq(pc, sqr_(st[0]) + sqr_(st[1]) + sqr_(st[2]), dx_sq, use0);
 }
 
 // Curvature numerator in the term order of curvature3d.f.in:109-117.
 template <class R>
-__device__ __forceinline__ R curv_numerator(R xx, R yy, R zz, R xy, R xz, R yz, R x, R y, R z) {
+__device__ __forceinline__ R curv_numerator_unit(R xx, R yy, R zz, R xy, R xz, R yz, R x, R y, R z) {
   return xx * y * y + yy * x * x - R(2) * xy * x * y + xx * z * z + zz * x * x - R(2) * xz * x * z +
          yy * z * z + zz * y * y - R(2) * yz * y * z;
+}
+#ifdef __CUDACC__
+static __device__ __noinline__ double curv_numerator_cold(double xx, double yy, double zz, double xy, double xz,
+                                                          double yz, double x, double y, double z) {
+  return curv_numerator_unit(xx, yy, zz, xy, xz, yz, x, y, z);
+}
+#endif
+// The FP64 form checks once that its nine values are zero or within
+// 2^-150 .. 2^150 (every product is then normal or zero) and takes the 21
+// products on the integer pipes; the doubled ones ride in the fma of their
+// sum, 2 ((xy x) y) being the same number as ((2 xy) x) y.
+template <class R>
+__device__ __forceinline__ R curv_numerator(R xx, R yy, R zz, R xy, R xz, R yz, R x, R y, R z) {
+#ifdef __CUDACC__
+  if constexpr (std::is_same<R, double>::value) {
+    const double v[9] = {xx, yy, zz, xy, xz, yz, x, y, z};
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 9; q++) ok = ok && fpi::plain<150>(fpi::words(v[q]));
+    if (!ok) return curv_numerator_cold(xx, yy, zz, xy, xz, yz, x, y, z);
+    const fpi::Op X = fpi::unpack(x, 1), Y = fpi::unpack(y, 1), Z = fpi::unpack(z, 1);
+    const fpi::Op XX = fpi::unpack(xx, 1), YY = fpi::unpack(yy, 1), ZZ = fpi::unpack(zz, 1);
+    auto term = [](const fpi::Op &a, const fpi::Op &b, const fpi::Op &c) {
+      return fpi::mul(fpi::unpack(fpi::mul(a, b), 1), c);
+    };
+    double s = term(XX, Y, Y) + term(YY, X, X);
+    s = fma(-2.0, term(fpi::unpack(xy, 1), X, Y), s);
+    s = s + term(XX, Z, Z) + term(ZZ, X, X);
+    s = fma(-2.0, term(fpi::unpack(xz, 1), X, Z), s);
+    s = s + term(YY, Z, Z) + term(ZZ, Y, Y);
+    return fma(-2.0, term(fpi::unpack(yz, 1), Y, Z), s);
+  }
+#endif
+  return curv_numerator_unit(xx, yy, zz, xy, xz, yz, x, y, z);
+}
+
+// |grad phi| from its components with the squares below `tol` dropped and a
+// root below it taken as 0 (spatial_derivatives3d.f.in:3630-3652)
+template <class R>
+__device__ __forceinline__ R grad_magnitude(R x, R y, R z, R tol) {
+  R x2 = sqr_(x), y2 = sqr_(y), z2 = sqr_(z);
+  if (below_(x2, tol)) x2 = R(0);
+  if (below_(y2, tol)) y2 = R(0);
+  if (below_(z2, tol)) z2 = R(0);
+  const R t = sqrt_(x2 + y2 + z2);
+  return below_(t, tol) ? R(0) : t;
+}
+
+// Second-order mean curvature (curvature3d.f.in:89-121) at phi's cell c with
+// strides sx, sy, sz, from the first derivatives, |grad phi| and the factors
+// 1/dx^2 .. and 1/(4 dx dy) ..
+template <class R, class I>
+__device__ __forceinline__ R mean_curvature2(const R *c, I sx, I sy, I sz, R px, R py, R pz, R g, R fxx, R fyy, R fzz,
+                                             R fxy, R fxz, R fyz) {
+  const R den = mul_(mul_(g, g), g);
+  if (less_(den, R(Consts<double>::zero_tol))) return R(0);
+  // c+ - 2 c0 is one fma: 2 c0 is exact
+  const R xx = mul_(fma(R(-2.0), c[0], c[sx]) + c[-sx], fxx);
+  const R yy = mul_(fma(R(-2.0), c[0], c[sy]) + c[-sy], fyy);
+  const R zz = mul_(fma(R(-2.0), c[0], c[sz]) + c[-sz], fzz);
+  const R xy = mul_(c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy], fxy);
+  const R xz = mul_(c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz], fxz);
+  const R yz = mul_(c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz], fyz);
+  return div_(curv_numerator(xx, yy, zz, xy, xz, yz, px, py, pz), den);
 }
 
 // one axis of the combined external + normal velocity Godunov selection

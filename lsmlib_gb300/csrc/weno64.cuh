@@ -73,7 +73,7 @@ constexpr uint32_t kDiffFloor = 500, kValueFloor = 300, kSquareFloor = 600;
 __device__ __forceinline__ Wide64 wide64(double inv) {
   Wide64 w;
   w.inv = inv;
-  w.op = fpi::unpack(inv, 1);
+  w.op = fpi::unpack_normal(inv);
   const uint32_t hi = fpi::words(inv).hi, e = hi >> 20;  // a negative or non-finite one is out of range
   w.lim = (e >= 823 && e <= 1223) ? (2145u - e) << 20 : 0u;
   return w;
@@ -103,28 +103,27 @@ __device__ __forceinline__ Diff64 divided(double d, const Wide64 &w) {
   r.o = fpi::unpack(r.v, kValueFloor);
   return r;
 }
-__device__ __forceinline__ double times(const Diff64 &d, double c) { return fpi::mul(d.o, fpi::unpack(c, 1)); }
+__device__ __forceinline__ double times(const Diff64 &d, double c) { return fpi::mul(d.o, fpi::unpack_normal(c)); }
 __device__ __forceinline__ double square64(double v) { return fpi::sqr(fpi::unpack(v, kSquareFloor)); }
 // 13/12 t^2 + u^2 / 4
 __device__ __forceinline__ double indicator64(double t, double u) {
-  return fma(0.25, square64(u), fpi::mul(fpi::unpack(square64(t), 1), fpi::unpack(13.0 / 12.0, 1)));
+  return fma(0.25, square64(u), fpi::mul(fpi::unpack(square64(t), 1), fpi::unpack_normal(13.0 / 12.0)));
 }
 // epsilon from the bits of the largest |v|
 __device__ __forceinline__ double epsilon64(unsigned long long m, double tiny) {
   const double mm = square64(__longlong_as_double((long long)m));
-  return fpi::mul(fpi::unpack(mm, 1), fpi::unpack(1e-6, 1)) + tiny;
+  return fpi::mul(fpi::unpack(mm, 1), fpi::unpack_normal(1e-6)) + tiny;
 }
 // the weighted sum of the three candidates
 __device__ __forceinline__ double combine64(double S1, double S2, double S3, double eps, double p1, double p2,
                                             double p3) {
-  const double a1 = fpi::div_pos(0.1, fpi::sqr(fpi::unpack(S1 + eps, 1)));
-  const double a2 = fpi::div_pos(0.6, fpi::sqr(fpi::unpack(S2 + eps, 1)));
-  const double a3 = fpi::div_pos(0.3, fpi::sqr(fpi::unpack(S3 + eps, 1)));
-  const fpi::Op is = fpi::unpack(fpi::div_pos(1.0, a1 + a2 + a3), 1);
-  const double w1 = fpi::mul(fpi::unpack(a1, 1), is), w2 = fpi::mul(fpi::unpack(a2, 1), is);
-  const double w3 = fpi::mul(fpi::unpack(a3, 1), is);
-  return fpi::mul(fpi::unpack(w1, 1), fpi::unpack(p1, 1)) + fpi::mul(fpi::unpack(w2, 1), fpi::unpack(p2, 1)) +
-         fpi::mul(fpi::unpack(w3, 1), fpi::unpack(p3, 1));
+  auto part = [&](double d, double S) { return fpi::div_pos(d, fpi::sqr(fpi::unpack_normal(S + eps))); };
+  const double a1 = part(0.1, S1), a2 = part(0.6, S2), a3 = part(0.3, S3);
+  const fpi::Op is = fpi::unpack_normal(fpi::div_pos(1.0, a1 + a2 + a3));
+  auto term = [&](double a, double p) {
+    return fpi::mul(fpi::unpack_normal(fpi::mul(fpi::unpack_normal(a), is)), fpi::unpack(p, 1));
+  };
+  return term(a1, p1) + term(a2, p2) + term(a3, p3);
 }
 
 // One side on the undivided differences d[0..4] (v1 .. v5 once divided).

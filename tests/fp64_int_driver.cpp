@@ -57,11 +57,32 @@ static long scalar_routines(long n) {
   for (long i = 0; i < n; i++) {
     const double a = operand(512, 1534), b = operand(512, 1534), d = fabs(operand(600, 1446));
     bad += fpi::mul(fpi::unpack(a, 1), fpi::unpack(b, 1)) != a * b;
-    bad += fpi::mul(fpi::unpack(0.0, 1), fpi::unpack(b, 1)) != 0.0;
+    bad += fpi::mul(fpi::unpack(i & 1 ? 0.0 : -0.0, 1), fpi::unpack(b, 1)) != 0.0;
     bad += fpi::sqr(fpi::unpack(a, 1)) != a * a;
     bad += fpi::div_pos(c[i & 3], d) != c[i & 3] / d;
     const double num = fabs(operand(600, 1446));
     bad += fpi::div_pos(num, d) != num / d;
+    const double r = fabs(operand(1, 2046)), sq = r > 1e-150 && r < 1e150 ? r * r : r;
+    bad += fpi::sqrt_pos(r) != std::sqrt(r);
+    bad += fpi::sqrt_pos(sq) != std::sqrt(sq);
+  }
+  return bad;
+}
+
+// the forms that take any operand, over the whole range and the special values
+static long any_operands(long n) {
+  long bad = 0;
+  const double special[10] = {0.0, -0.0, INFINITY, -INFINITY, NAN, 5e-324, 2.2250738585072014e-308,
+                              1.7976931348623157e308, 1e-200, 1e200};
+  for (long i = 0; i < n; i++) {
+    const double a = g() % 8 ? operand(0, 2046) : special[g() % 10], b = g() % 8 ? operand(0, 2046) : special[g() % 10];
+    bad += !same(fpi::mul_any(a, b), a * b) || !same(fpi::sqr_any(a), a * a);
+    bad += !same(fpi::div_any(a, b), a / b) || !same(fpi::sqrt_any(a), std::sqrt(a));
+    bad += !same(fpi::abs_bits(a), fabs(a)) || !same(fpi::flip_if(a, i & 1), (i & 1) ? -a : a);
+    bad += fpi::is_positive(a) != (a > 0) || !same(fpi::positive_part(a), a > 0 ? a : 0.0);
+    const double x = fabs(a), y = fabs(b), t = 1e-11;
+    bad += !same(fpi::max_nonneg(x, y), x > y ? x : y);
+    bad += fpi::less_than(a, t) != (a < t) || fpi::below(a, t) != (fabs(a) < t) || fpi::at_least(a, t) != (fabs(a) >= t);
   }
   return bad;
 }
@@ -110,6 +131,6 @@ static long reconstructions(long n) {
 int main(int argc, char **argv) {
   const long n = argc > 1 ? atol(argv[1]) : 1000000;
   g.seed(argc > 2 ? (uint64_t)atol(argv[2]) : 1);
-  printf("%ld %ld\n", scalar_routines(n), reconstructions(n));
+  printf("%ld %ld %ld\n", scalar_routines(n), any_operands(n), reconstructions(n));
   return 0;
 }
