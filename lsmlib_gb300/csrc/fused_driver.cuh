@@ -196,7 +196,7 @@ void launch_bc(R *buf, const Layout &L, int bc) {
 }
 
 // The FP32 reinitialization stage runs the window-sharing kernel of
-// reinit_x2.cuh (64 x 8 x RZ tiles); every other form runs k_stage /
+// reinit_x2.cuh (64 x 8 cell tiles); every other form runs k_stage /
 // k_stage_f32 (32 x 8 x TZ tiles).
 template <class R, int MODE, bool EXACT>
 constexpr bool uses_reinit_x2() {
@@ -249,13 +249,29 @@ inline int stage_tz_f64(const Layout &L) {
   return 1;
 }
 
+// Tile depth of the FP32 reinitialization stage (k_reinit_x2).  A grid of
+// fewer 8-plane tiles than SMs is a matter of one tile's latency, about 4 us
+// and 0.95 us per plane: 4 planes, or 2 where 4-plane tiles are fewer than SMs
+// too (37 x 33 x 41: 13.2 -> 7.6 us per stage; 64^3: 13.3 -> 8.8).  Larger
+// grids take 8 or 10 planes, whichever makes the busiest SM's tiles shorter
+// in all, a tile costing one plane beside its own (128^3: 29.5 us with 8, 27.4
+// with 10; 160 x 150 x 140: 44.7 and 48.0; 256^3: 157.6 and 155.6).
+inline int reinit_tz(const Layout &L) {
+  const long long cols = (long long)((L.nx + RX - 1) / RX) * ((L.ny + RY - 1) / RY);
+  const int sms = sm_count();
+  auto tiles = [&](int tz) { return cols * ((L.nz + tz - 1) / tz); };
+  if (tiles(8) < sms) return tiles(4) < sms ? 2 : 4;
+  auto planes = [&](int tz) { return (tiles(tz) + sms - 1) / sms * (tz + 1); };
+  return planes(10) < planes(8) ? 10 : 8;
+}
+
 // Tensor map of a padded work buffer with the staged box of the stage kernel
 // launch_stage<R, MODE, EXACT> runs.
 template <class R, int MODE, bool EXACT>
 bool encode_stage_tmap(CUtensorMap *m, const R *p, const Layout &L) {
   const long long ex = (long long)L.nx + GX + 3, ey = (long long)L.ny + 2 * GY, ez = (long long)L.nz + 2 * GZ;
   if constexpr (uses_reinit_x2<R, MODE, EXACT>())
-    return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, RSX, RSY, RZ + 6);
+    return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, RSX, RSY, reinit_tz(L) + 6);
   if constexpr (!EXACT && sizeof(R) == 4)
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f32(L) + 6);
   return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f64(L) + 6);
@@ -273,12 +289,13 @@ static void launch_stage(const CUtensorMap &tm, const StageArgs<R> &a, bool prep
   static bool attr_set = false;
   if constexpr (uses_reinit_x2<R, MODE, EXACT>()) {
     if (!attr_set) {
-      cudaFuncSetAttribute(k_reinit_x2<RZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)reinit_x2_smem(RZ));
+      cudaFuncSetAttribute(k_reinit_x2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)reinit_x2_smem(RZ_MAX));
       attr_set = true;
     }
     if (prepare_only) return;
-    dim3 grd((unsigned)((L.nx + RX - 1) / RX), (unsigned)((L.ny + RY - 1) / RY), (unsigned)((L.nz + RZ - 1) / RZ));
-    k_reinit_x2<RZ><<<grd, dim3(32, RY), reinit_x2_smem(RZ), stream()>>>(tm, a);
+    const int tz = reinit_tz(L);
+    dim3 grd((unsigned)((L.nx + RX - 1) / RX), (unsigned)((L.ny + RY - 1) / RY), (unsigned)((L.nz + tz - 1) / tz));
+    k_reinit_x2<<<grd, dim3(32, RY), reinit_x2_smem(tz), stream()>>>(tm, a, tz);
     note_launch();
     return;
   }

@@ -120,16 +120,16 @@ __device__ __noinline__ void fill_face_ghosts(R *tile, int sdx, int sdy, int sdz
     const int loA = PA == 0 ? lo0 : lo1, hiA = PA == 0 ? hi0 : hi1;
     const int loB = PB == 1 ? lo1 : lo2, hiB = PB == 1 ? hi1 : hi2;
     const int loG = AX == 0 ? lo0 : (AX == 1 ? lo1 : lo2), hiG = AX == 0 ? hi0 : (AX == 1 ? hi1 : hi2);
-    for (int pa = loA + (int)threadIdx.x; pa <= hiA; pa += blockDim.x)
-      for (int pb = loB + (int)threadIdx.y; pb <= hiB; pb += blockDim.y)
-        for (int g = loG; g <= hiG; g++) {
-          const int c0 = AX == 0 ? g : pa;
-          const int c1 = AX == 1 ? g : (PA == 1 ? pa : pb);
-          const int c2 = AX == 2 ? g : pb;
-          const int at = (c0 - ox) + (c1 - oy) * sdx + (c2 - oz) * sxy;
-          const int d = up ? g - e_at : -g;
-          tile[at] = extrap(tile[at + (e_at - g) * st], tile[at + (n_at - g) * st], d, kind);
-        }
+    // both values of a line are read once, before its ghost cells are written
+    for (int pb = loB + (int)threadIdx.y; pb <= hiB; pb += blockDim.y)
+      for (int pa = loA + (int)threadIdx.x; pa <= hiA; pa += blockDim.x) {
+        const int c0 = AX == 0 ? e_at : pa;
+        const int c1 = AX == 1 ? e_at : (PA == 1 ? pa : pb);
+        const int c2 = AX == 2 ? e_at : pb;
+        R *edge = tile + (c0 - ox) + (c1 - oy) * sdx + (c2 - oz) * sxy;
+        const R e = *edge, n = edge[(n_at - e_at) * st];
+        for (int g = loG; g <= hiG; g++) edge[(g - e_at) * st] = extrap(e, n, up ? g - e_at : -g, kind);
+      }
   };
   // only the faces the tile crosses
   if (ox < 0) face(std::integral_constant<int, 0>{}, 0);

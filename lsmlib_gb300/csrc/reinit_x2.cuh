@@ -29,8 +29,9 @@
 // Differences are not divided by dx: WENO5 is homogeneous of degree one in
 // them, so the reconstructed derivatives are scaled once at the end.
 //
-// Tile: 64 x 8 x RZ cells per CTA of 32 x 8 threads; the tile plus its halo
-// (72 x 14 x (RZ + 6)) is staged by one TMA load.  With extrapolation
+// Tile: 64 x 8 x tz cells per CTA of 32 x 8 threads (tz even, 2 to 10, chosen
+// per grid by the launcher); the tile plus its halo (72 x 14 x (tz + 6)) is
+// staged by one TMA load.  With extrapolation
 // boundary conditions the ghost cells the stencils read are computed in
 // shared memory from the tile's interior cells (fill_face_ghosts in
 // fused_stage.cuh), so the stage needs no separate ghost-fill launch.
@@ -43,14 +44,9 @@ namespace fused {
 
 constexpr int RX = 64, RY = 8;    // cells of a tile in x and y
 constexpr int RSX = RX + 8, RSY = RY + 6;  // staged tile in x and y
-constexpr int RZ = 8;             // planes of a tile (the depth the steppers launch)
-// staged tile of a TILE_Z-plane tile: 72 x 14 x (TILE_Z + 6) floats
-constexpr size_t reinit_x2_smem(int tile_z) { return (size_t)RSX * RSY * (tile_z + 6) * sizeof(float); }
-// CTAs per SM the kernel is built for: three 8-plane tiles fit the SM's
-// shared memory (67 KB each with the static arrays) and registers (80 per
-// thread); a 16-plane tile needs 100 KB, so two.
-constexpr int reinit_x2_ctas(int tile_z) { return tile_z <= 8 ? 3 : 2; }
-
+constexpr int RZ_MAX = 10;        // planes of the deepest tile
+// staged tile of a tz-plane tile: 72 x 14 x (tz + 6) floats
+constexpr size_t reinit_x2_smem(int tz) { return (size_t)RSX * RSY * (tz + 6) * sizeof(float); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, sp(-1.f), a); }
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
@@ -169,26 +165,22 @@ static __device__ __noinline__ void write_periodic_images(float *out, const Layo
   if (oi && oj && ok) out[c + sx + sy + sz] = val;
 }
 
-// (a template so that each translation unit including this header has its
-// own instance, as with the other stage kernels)
-template <int TILE_Z = RZ>
-__global__ void __launch_bounds__(256, reinit_x2_ctas(TILE_Z))
-    k_reinit_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a) {
-  static_assert(TILE_Z % 2 == 0 && TILE_Z % RY == 0, "the prologues pack plane pairs and cover the planes by rows");
-  constexpr int RZ = TILE_Z, RSZ = TILE_Z + 6;
-  constexpr size_t kReinitX2Smem = reinit_x2_smem(TILE_Z);
+// (static: each translation unit including this header has its own instance,
+// as with the other stage kernels; 80 registers for three CTAs per SM)
+static __global__ void __launch_bounds__(256, 3)
+    k_reinit_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a, int tzn) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *tile = reinterpret_cast<float *>(smem_raw);
   __shared__ __align__(8) uint64_t bar;
   // tile-edge values of the neighbouring lanes / rows that do not exist:
   // x: per (plane, row) minus(x0) and the forms of triples x0-1, x0;
   // y: per (plane, x pair) minus(y0)
-  __shared__ float xedge[6][RZ][RY];
-  __shared__ float2 yedge[RZ][32];
+  __shared__ float xedge[6][RZ_MAX][RY];
+  __shared__ float2 yedge[RZ_MAX][32];
   __shared__ float2 yx[2][RY][32];  // minus(j+1) handed to the next row, by plane parity
   const int lane = threadIdx.x, w = threadIdx.y;
   const int tid = lane + 32 * w;
-  const int x0 = blockIdx.x * RX, y0 = blockIdx.y * RY, z0 = blockIdx.z * RZ;
+  const int x0 = blockIdx.x * RX, y0 = blockIdx.y * RY, z0 = blockIdx.z * tzn;
   const Layout &L = a.L;
 
   if (tid == 0) {
@@ -198,7 +190,7 @@ __global__ void __launch_bounds__(256, reinit_x2_ctas(TILE_Z))
   }
   __syncthreads();
   if (tid == 0) {
-    mbar_arrive_expect_tx(&bar, (uint32_t)kReinitX2Smem);
+    mbar_arrive_expect_tx(&bar, (uint32_t)reinit_x2_smem(tzn));
     tma_load_3d(tile, &tm, x0 + GX - 4, y0 + GY - 3, z0 + GZ - 3, &bar);
   }
   if (!mbar_wait(&bar, 0, kMaxPolls)) {
@@ -207,13 +199,13 @@ __global__ void __launch_bounds__(256, reinit_x2_ctas(TILE_Z))
     return;
   }
   if (a.ghost) {
-    fill_face_ghosts<float>(tile, RSX, RSY, RSZ, x0 - 4, y0 - 3, z0 - 3, L, a.ghost);
+    fill_face_ghosts<float>(tile, RSX, RSY, tzn + 6, x0 - 4, y0 - 3, z0 - 3, L, a.ghost);
     __syncthreads();
   }
 
   const int st_y = RSX, st_z = RSX * RSY;
   // ---- prologue: the tile-edge values, two planes per thread as a pair ------
-  if (tid < RY * RZ / 2) {
+  if (tid < RY * tzn / 2) {
     const int pw = tid % RY, pz = 2 * (tid / RY);
     const float *r0 = tile + ((pz + 3) * RSY + pw + 3) * RSX, *r1 = r0 + st_z;
     float2 p[6];  // phi(x0-3 .. x0+2)
@@ -234,7 +226,7 @@ __global__ void __launch_bounds__(256, reinit_x2_ctas(TILE_Z))
   {
     // minus(y0) of each x pair, planes w and w + RY
 #pragma unroll 1
-    for (int tz = w; tz < RZ; tz += RY) {
+    for (int tz = w; tz < tzn; tz += RY) {
       const float *c = tile + (tz + 3) * st_z + 2 * lane + 4;
       float2 p[6];  // phi(y0-3 .. y0+2)
 #pragma unroll
@@ -255,7 +247,7 @@ __global__ void __launch_bounds__(256, reinit_x2_ctas(TILE_Z))
   const bool two = i + 1 < L.nx;
   const bool live = row_live && i < L.nx;
   const int sx = 2 * lane + 4, sy = w + 3;
-  const int kmax = min(RZ, L.nz - z0);
+  const int kmax = min(tzn, L.nz - z0);
   const float *col = tile + sy * st_y + sx;  // (i, j) column, plane index sz
   auto ld2 = [&](int sz, int dx, int dy) {
     return *reinterpret_cast<const float2 *>(col + sz * st_z + dy * st_y + dx);

@@ -177,3 +177,25 @@ def test_identical_calls_replay_the_cached_graph(precision, gpu_lib):
     L.check()
     assert L.graph_capture_count() == before
     assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(37, 33, 41), (70, 60, 50), (96, 90, 75), (128, 128, 41)])
+@pytest.mark.parametrize("bc,use0", [(L.BC_PERIODIC, 1), (L.BC_SIGNED_LINEAR, 0), (L.BC_COPY, 1)])
+def test_fused_reinit_f32_tile_depths(n, bc, use0, gpu_lib):
+    """FP32 reinitialization at sizes that run 2-, 4-, 8- and 10-plane tiles
+    (on 152 SMs), the last tile of each axis ragged, against the FP64 form
+    (which equals the oracle bit for bit); interior cells, as above (a corner
+    ghost is three extrapolations of 4x to 7x each on top of them)."""
+    import torch
+    fb = (0, n[0] - 1, 0, n[1] - 1, 0, n[2] - 1)
+    gb = tuple(v + (-3, 3)[q % 2] for q, v in enumerate(fb))
+    dx = 2.0 / max(n)
+    X, Y, Z = np.meshgrid(*[(np.arange(-3, m + 3) + 0.5 - 0.5 * m) * dx for m in n], indexing="ij")
+    phi = (np.sqrt(X ** 2 + Y ** 2 + Z ** 2 + 0.01) - 0.5) * (0.5 + (X - 0.3) ** 2 + Y ** 2)
+    t32 = torch.from_numpy(np.ascontiguousarray(phi.T)).cuda().float()
+    t64 = t32.double()
+    for t, precision in ((t32, "f32"), (t64, "f64")):
+        L.reinit_weno5_tvdrk3(t, gb, fb, dx, 0.5 * dx, 3, use_phi0_for_sgn=use0, bc=bc, precision=precision)
+    L.check()
+    assert float((t32.double() - t64)[3:-3, 3:-3, 3:-3].abs().max()) <= 1e-5
