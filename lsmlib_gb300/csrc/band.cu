@@ -49,8 +49,7 @@ void determine_band(const char *name, const R *phi, const Box &gb, const R *seco
   int ob[4];
   int nwrite = 1;
   if (!band_build<R>(call, phd, gb, nbd, nbb, ix, iy, iz, *nlo_index, *nhi_index, outer, *nlo_index_outer,
-                     *nhi_index_outer, width, width_inner, level, lo, hi, ob, nullptr, new_claims(call, nbb), false,
-                     form, &nwrite))
+                     *nhi_index_outer, width, width_inner, level, lo, hi, ob, new_claims(call, nbb), form, &nwrite))
     return;
   put_ints(n_lo, lo.data(), nwrite);
   put_ints(n_hi, hi.data(), nwrite);

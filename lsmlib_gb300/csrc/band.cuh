@@ -1,5 +1,6 @@
 // Narrow-band construction machinery shared by the drop-in entry points
-// (band.cu) and the fused narrow-band stepper (bandflow.cu).
+// (band.cu); the fused narrow-band stepper (bandflow.cuh) uses its ordered
+// compaction.
 //
 // Bit-exact with the reference's serial order:
 //  - level 0 lists cells with |phi| < width in the reference's (k, j, i) sweep
@@ -273,20 +274,8 @@ struct Level0T {
     j = gb.lo[1] + (int)(r / nx);
     i = gb.lo[0] + (int)(r % nx);
   }
-  // FP32 fields compare in FP32 against thresholds rounded so each decision
-  // equals the FP64 one: for a float a, (double)a < width <=> a <= width_lt
-  // (the largest float below width) and (double)a >= width_inner <=>
-  // a >= inner_ge (the smallest float not below width_inner)
-  float width_lt, inner_ge;
-  // when set (nb box == phi's box): the count pass writes every cell's
-  // classification bits into its mark byte (1 level 0, 2 outer minus, 4 outer
-  // plus); the emit pass (Level0Marks) reads them back instead of phi and
-  // leaves the final marks (1 in level 0, 0 elsewhere)
-  U8 *mark_lin = nullptr;
   static constexpr bool kPrefetch = true;
-  __device__ void counted(long long e, int bits) const {
-    if (mark_lin) mark_lin[e] = (U8)bits;
-  }
+  __device__ void counted(long long, int) const {}
   typedef T V;
   __device__ T load(long long e) const { return phi.p[e]; }
   __device__ int flags(long long e) const { return classify(phi.p[e], e); }
@@ -298,33 +287,13 @@ struct Level0T {
       if (a >= width_inner) return v <= R(0) ? 3 : 5;
       return 1;
     }
-    if constexpr (sizeof(T) == 4) {
-      const float v = (float)raw;
-      if (mode == 1) return v >= 0.f ? 1 : 0;
-      if (mode == 2) return v <= 0.f ? 1 : 0;
-      const float a = fabsf(v);
-      if (!(a <= width_lt)) return 0;
-      if (a >= inner_ge) return v <= 0.f ? 3 : 5;
-      return 1;
-    } else {
-      const R v = (R)raw;
-      if (mode == 1) return v >= R(0) ? 1 : 0;
-      if (mode == 2) return v <= R(0) ? 1 : 0;
-      const R a = fabs(v);
-      if (!(a < width)) return 0;
-      if (a >= width_inner) return v <= R(0) ? 3 : 5;
-      return 1;
-    }
-  }
-  void set_widths(double w, double wi) {
-    width = w;
-    width_inner = wi;
-    float f = (float)w;
-    if ((double)f >= w) f = nextafterf(f, -INFINITY);
-    width_lt = f;
-    float g = (float)wi;
-    if ((double)g < wi) g = nextafterf(g, INFINITY);
-    inner_ge = g;
+    const R v = (R)raw;
+    if (mode == 1) return v >= R(0) ? 1 : 0;
+    if (mode == 2) return v <= R(0) ? 1 : 0;
+    const R a = fabs(v);
+    if (!(a < width)) return 0;
+    if (a >= width_inner) return v <= R(0) ? 3 : 5;
+    return 1;
   }
   __device__ void emit(long long e, int bits, long long r0, long long r1, long long r2) const {
     int i, j, k;
@@ -339,53 +308,6 @@ struct Level0T {
 };
 
 typedef Level0T<R> Level0;
-
-// emit pass of a fused-marks level-0 build: the classification comes from the
-// mark bytes the count pass wrote (a quarter of phi's bytes for FP32, an
-// eighth for FP64); each listed cell's byte becomes its final mark 1
-template <class T>
-struct Level0Marks {
-  Level0T<T> z;
-  U8 *marks;
-  static constexpr bool kPrefetch = true;
-  typedef U8 V;
-  __device__ U8 load(long long e) const { return marks[e]; }
-  __device__ int classify(U8 raw, long long) const { return raw; }
-  __device__ int flags(long long e) const { return marks[e]; }
-  __device__ void counted(long long, int) const {}
-  __device__ void emit(long long e, int bits, long long r0, long long r1, long long r2) const {
-    z.emit(e, bits, r0, r1, r2);
-    marks[e] = 1;
-  }
-};
-
-// Level-0 pass of a rebuild inside the narrow-band flow over the previous
-// level-0 list (ox, oy, oz) instead of the grid: between rebuilds the flow
-// writes phi only at level-0 cells, so a cell outside the previous level 0
-// still has |phi| >= width and the new level 0 (and its outer layer) is the
-// ordered sub-sequence of the previous level-0 list whose cells pass the test
-// (the previous list is in the reference's sweep order).  The caller clears
-// the previous band's marks first; each listed cell gets mark 1.
-template <class T>
-struct Level0List {
-  Level0T<T> z;
-  const int *ox, *oy, *oz;
-  static constexpr bool kPrefetch = true;
-  typedef T V;
-  __device__ T load(long long e) const { return z.phi.p[z.phi.off(ox[e], oy[e], oz[e])]; }
-  __device__ int classify(T raw, long long) const { return z.classify(raw, 0); }
-  __device__ int flags(long long e) const { return classify(load(e), e); }
-  __device__ void counted(long long, int) const {}
-  __device__ void emit(long long e, int bits, long long r0, long long r1, long long r2) const {
-    const int i = ox[e], j = oy[e], k = oz[e];
-    z.ix[r0] = i;
-    z.iy[r0] = j;
-    z.iz[r0] = k;
-    if (bits & 2) z.outer[r1] = z.nlo + (int)r0;
-    if (bits & 4) z.outer[(z.nhi_outer - z.nlo_outer) - r2] = z.nlo + (int)r0;
-    z.nb(i, j, k) = 1;
-  }
-};
 
 // every cell of phi's ghost box gets its level-0 mark (1 in the band, 0 out);
 // threads along x and y, each walking kMarkZ planes
@@ -660,20 +582,11 @@ struct BandForm {
 // outer-list bounds {plus lo, plus hi, minus lo, minus hi}, *nwrite (when
 // set) the number of levels the reference writes.  Returns false after
 // recording an error (capacity or CUDA).
-// prev (optional, level-0 selection |phi| < width only): the previous
-// level-0 list {ox, oy, oz, count} of a rebuild inside the narrow-band flow
-// (Level0List); the caller has cleared that band's marks
-struct PrevLevel0 {
-  const int *ox = nullptr, *oy = nullptr, *oz = nullptr;
-  long long n = 0;
-};
-
 template <class T>
 bool band_build(Call &call, const T *phi, const Box &gb, U8 *nbd, const Box &nbb, int *ix, int *iy, int *iz,
                 int nlo, int nhi, int *outer, int nlo_outer, int nhi_outer, double width, double width_inner,
-                int level, std::vector<int> &lo, std::vector<int> &hi, int ob[4], long long *level0_count,
-                int *claim, bool fuse_marks = false, const BandForm<T> &form = BandForm<T>(),
-                int *nwrite = nullptr, const PrevLevel0 *prev = nullptr) {
+                int level, std::vector<int> &lo, std::vector<int> &hi, int ob[4], int *claim,
+                const BandForm<T> &form = BandForm<T>(), int *nwrite = nullptr) {
   const long long cap = (long long)nhi - nlo + 1;
   const long long ocap = (long long)nhi_outer - nlo_outer + 1;
   Level0T<T> z;
@@ -682,7 +595,8 @@ bool band_build(Call &call, const T *phi, const Box &gb, U8 *nbd, const Box &nbb
   z.gb = gb;
   z.nx = gb.n(0);
   z.nxy = gb.n(0) * gb.n(1);
-  z.set_widths(width, width_inner);
+  z.width = width;
+  z.width_inner = width_inner;
   z.ix = ix; z.iy = iy; z.iz = iz;
   z.outer = outer;
   z.nlo = nlo;
@@ -693,41 +607,22 @@ bool band_build(Call &call, const T *phi, const Box &gb, U8 *nbd, const Box &nbb
   z.max_dx = form.max_dx;
   const long long n = gb.size();
   long long tot[3];
-  // fused marks: the count pass writes every cell's level-0 mark (the nb
-  // array has phi's box); only for callers that own the arrays, since the
-  // marks are then written before the capacity check
-  const bool fused = fuse_marks && nbb.lo[0] == gb.lo[0] && nbb.hi[0] == gb.hi[0] && nbb.lo[1] == gb.lo[1] &&
-                     nbb.hi[1] == gb.hi[1] && nbb.lo[2] == gb.lo[2] && nbb.hi[2] == gb.hi[2];
-  const bool from_list = prev && prev->ox && form.l0_mode == 0;
-  if (fused && !from_list) z.mark_lin = nbd;
   Compaction c0;
-  if (from_list) {
-    if (!c0.count(call, Level0List<T>{z, prev->ox, prev->oy, prev->oz}, prev->n, tot)) return false;
-  } else if (!c0.count(call, z, n, tot)) {
-    return false;
-  }
-  z.mark_lin = nullptr;
+  if (!c0.count(call, z, n, tot)) return false;
   if (tot[0] > cap || tot[1] + tot[2] > ocap) {
     set_error(LSMGPU_ERR_CAPACITY, "narrow band (%lld cells) or outer layer (%lld) exceeds the index arrays", tot[0],
               tot[1] + tot[2]);
     return false;
   }
-  if (from_list) {
-    c0.emit(Level0List<T>{z, prev->ox, prev->oy, prev->oz});
-  } else if (fused) {
-    c0.emit(Level0Marks<T>{z, nbd});
-  } else {
-    LSMGPU_LAUNCH(k_mark0<T>,
-                  dim3((unsigned)((gb.n(0) + 31) / 32), (unsigned)((gb.n(1) + 7) / 8),
-                       (unsigned)((gb.n(2) + kMarkZ - 1) / kMarkZ)),
-                  dim3(32, 8), 0, z);
-    c0.emit(z);
-  }
+  LSMGPU_LAUNCH(k_mark0<T>,
+                dim3((unsigned)((gb.n(0) + 31) / 32), (unsigned)((gb.n(1) + 7) / 8),
+                     (unsigned)((gb.n(2) + kMarkZ - 1) / kMarkZ)),
+                dim3(32, 8), 0, z);
+  c0.emit(z);
   lo.assign(level + 1, -1);
   hi.assign(level + 1, -1);
   lo[0] = nlo;
   ob[0] = nhi_outer; ob[1] = nhi_outer; ob[2] = nlo_outer; ob[3] = nlo_outer;
-  if (level0_count) *level0_count = tot[0];
   if (form.bookkeeping != 0) {
     hi[0] = (int)(nlo + tot[0] - 1);
     ob[2] = nlo_outer;

@@ -7,15 +7,21 @@
 //   HJ WENO5 LOCAL -> lsm3dZeroOut/AddNormalVelTermToLSERHSLOCAL ->
 //   (stage 1: lsm3dComputeStableNormalVelDtLOCAL) ->
 //   lsm3dMultiplyCutOffLSERHSLOCAL -> lsm3dTVDRK3StageNLOCAL
-// with one gather kernel per stage (stage 1 is split at the dt reduction),
-// and the band build of band.cuh.  Band levels 1..3 of the stage fields hold
-// phi^n: they are refreshed at every rebuild and never written by a stage.
+// with one gather kernel per stage (stage 1 is split at the dt reduction).
+//
+// The band.  Of LSMLIB's band the flow needs the level-0 cells, |phi| < gamma
+// at a rebuild.  The first build finds them over the grid; since the flow
+// writes phi at level-0 cells only, a later level 0 is the sub-sequence of the
+// previous one that passes the test.  LSMLIB's neighbour levels 1..3 exist so
+// that the stage fields hold phi^n where the stencils reach outside level 0;
+// here the stage fields hold phi at every cell outside level 0 from the start
+// (one copy of phi, then the cells that leave level 0 at a rebuild), so no
+// neighbour level is built.  The list holds one offset per cell, in the
+// reference's sweep order.
 //
 // LSMGPU_BANDFLOW_EXACT selects the FP64 parity arithmetic (this unit is
 // compiled with -fmad=false); the FP32 form uses the fast WENO weights.
 #pragma once
-#include <vector>
-
 #include "band.cuh"
 #include "fused_stage.cuh"
 #include "stencil_math.cuh"
@@ -29,8 +35,7 @@ struct BandArgs {
   View<const R> src;      // stage source (phi^n, u1, u2)
   View<const R> phin;     // phi^n (stages 2, 3)
   View<R> out;            // stage output
-  const int *ix, *iy, *iz;
-  const int *off0;        // padded offset of each level-0 entry (written at each rebuild)
+  const int *off0;        // offset of each level-0 cell in its array
   int n0;                 // level-0 entries (list elements 0..n0-1)
   R dx, a_n, b_n, beta, gamma, cfl;
   // per-call constants of the stencils, divided on the host in R exactly as
@@ -108,8 +113,8 @@ __device__ __forceinline__ R godunov_rhs(const BandArgs<R> &a, R vn, const R gp[
 
 // the RHS of one level-0 cell, before the cut-off; also the cell's H/dx for dt
 template <class R, bool EXACT>
-__device__ __forceinline__ R cell_rhs(const BandArgs<R> &a, int i, int j, int k, R &h_over_dx) {
-  const R *c = a.src.p + a.src.off(i, j, k);
+__device__ __forceinline__ R cell_rhs(const BandArgs<R> &a, long long o, R &h_over_dx) {
+  const R *c = a.src.p + o;
   const long long s[3] = {1, a.src.s1, a.src.s2};
   const R vn = cell_vn<R>(a, c, s);
   // HJ WENO5 plus/minus from the band values of src
@@ -226,11 +231,11 @@ __global__ void k_band_rhs(BandArgs<R> a) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   double h = -1.0e308;
   if (l < a.n0) {
-    const int i = a.ix[l], j = a.iy[l], k = a.iz[l];
+    const long long o = a.off0[l];
     R hd;
-    const R r = cell_rhs<R, EXACT>(a, i, j, k, hd);
+    const R r = cell_rhs<R, EXACT>(a, o, hd);
     h = (double)hd;
-    a.rhs[l] = cutoff<R>(r, a.src(i, j, k), a.beta, a.gamma);
+    a.rhs[l] = cutoff<R>(r, a.src.p[o], a.beta, a.gamma);
   }
   for (int o = 16; o > 0; o >>= 1) h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
   if ((threadIdx.x & 31) == 0) raise_key(a.key, okey(h));
@@ -259,11 +264,11 @@ template <class R, bool EXACT>
 __global__ void k_band_stage(BandArgs<R> a) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= a.n0) return;
-  const int i = a.ix[l], j = a.iy[l], k = a.iz[l];
+  const long long o = a.off0[l];
   R hd;
-  const R us = a.src(i, j, k);
-  const R r = cutoff<R>(cell_rhs<R, EXACT>(a, i, j, k, hd), us, a.beta, a.gamma);
-  a.out(i, j, k) = rk_update<R>(a.stage, a.phin(i, j, k), us, *a.dt, r);
+  const R us = a.src.p[o];
+  const R r = cutoff<R>(cell_rhs<R, EXACT>(a, o, hd), us, a.beta, a.gamma);
+  a.out.p[o] = rk_update<R>(a.stage, a.phin.p[o], us, *a.dt, r);
 }
 
 // FP32 forms of k_band_rhs and k_band_stage on pairs of consecutive list
@@ -331,40 +336,76 @@ static __global__ void k_band_stage_x2(BandArgs<float> a) {
   if (two) a.out.p[o1] = rk_update<float>(a.stage, n1v, us1, dt, cutoff<float>(r.y, us1, a.beta, a.gamma));
 }
 
-// the padded offset of each level-0 entry, for the stage kernels (one 4-byte
-// read per entry instead of three coordinates)
+// The level-0 test |phi| < width in FP64 whatever the field's precision: for
+// a float a, (double)a < width is a <= the largest float below width.
 template <class R>
-__global__ void k_band_offsets(View<const R> v, const int *ix, const int *iy, const int *iz, int n, int *off) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n) return;
-  off[l] = (int)v.off(ix[l], iy[l], iz[l]);
-}
-
-// clears the marks of the listed cells (the previous band, before a rebuild)
-// and copies the level-0 entries (the first n0) to ox, oy, oz
-static __global__ void k_band_retire(U8 *nb, View<const U8> v, const int *ix, const int *iy, const int *iz, int n,
-                                     int n0, int *ox, int *oy, int *oz) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n) return;
-  const int i = ix[l], j = iy[l], k = iz[l];
-  nb[v.off(i, j, k)] = 0;
-  if (l < n0) {
-    ox[l] = i;
-    oy[l] = j;
-    oz[l] = k;
+struct Width {
+  R lim;
+  explicit Width(double w) {
+    if constexpr (sizeof(R) == 4) {
+      lim = (float)w;
+      if ((double)lim >= w) lim = nextafterf(lim, -INFINITY);
+    } else {
+      lim = w;
+    }
   }
-}
+  __device__ __forceinline__ bool in(R v) const {
+    if constexpr (sizeof(R) == 4) return fabsf(v) <= lim;
+    else return below_(v, lim);
+  }
+};
 
-// phi -> u1, u2 at the listed cells
+// Classifiers of the ordered compaction (band.cuh).  First build: every cell
+// of the array in memory order, which is the reference's sweep order.
 template <class R>
-__global__ void k_copy_band(const R *phi, R *u1, R *u2, View<const R> v, const int *ix, const int *iy, const int *iz,
-                            int n) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n) return;
-  const long long o = v.off(ix[l], iy[l], iz[l]);
-  const R p = phi[o];
-  u1[o] = p;
-  u2[o] = p;
+struct FlowGrid {
+  const R *phi;
+  Width<R> width;
+  int *off;
+  static constexpr bool kPrefetch = true;
+  typedef R V;
+  __device__ R load(long long e) const { return phi[e]; }
+  __device__ int classify(R v, long long) const { return width.in(v) ? 1 : 0; }
+  __device__ int flags(long long e) const { return classify(phi[e], e); }
+  __device__ void counted(long long, int) const {}
+  __device__ void emit(long long e, int, long long r0, long long, long long) const { off[r0] = (int)e; }
+};
+
+// Rebuild: the previous list; a cell that leaves level 0 gets phi in the
+// stage fields (in the count pass, which sees each cell once).
+template <class R>
+struct FlowList {
+  const R *phi;
+  Width<R> width;
+  const int *old;
+  int *off;
+  R *u1, *u2;
+  static constexpr bool kPrefetch = true;
+  typedef R V;
+  __device__ R load(long long e) const { return phi[old[e]]; }
+  __device__ int classify(R v, long long) const { return width.in(v) ? 1 : 0; }
+  __device__ int flags(long long e) const { return classify(load(e), e); }
+  __device__ void counted(long long e, int bits) const {
+    if (bits) return;
+    const int o = old[e];
+    u1[o] = u2[o] = phi[o];
+  }
+  __device__ void emit(long long e, int, long long r0, long long, long long) const { off[r0] = old[e]; }
+};
+
+// phi -> u1, u2, the whole array
+template <class R>
+__global__ void __launch_bounds__(256) k_copy_fields(const R *__restrict__ phi, R *__restrict__ u1,
+                                                     R *__restrict__ u2, long long n) {
+  constexpr int kPer = 8;
+  const long long base = (long long)blockIdx.x * (256 * kPer) + threadIdx.x;
+  R v[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+    if (base + 256 * q < n) v[q] = phi[base + 256 * q];
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+    if (base + 256 * q < n) u1[base + 256 * q] = u2[base + 256 * q] = v[q];
 }
 
 template <class R, bool EXACT>
@@ -379,75 +420,50 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, R dx, R a_n
   const long long n = gb.size();
   R *phi = call.inout(phi_user, n);
   R *u1 = call.temp<R>(n), *u2 = call.temp<R>(n);
-  U8 *nb = call.temp<U8>(n);
-  int *ix = call.temp<int>(n), *iy = call.temp<int>(n), *iz = call.temp<int>(n), *outer = call.temp<int>(n);
   constexpr bool packed = !EXACT && sizeof(R) == 4;
   R *rhs = nullptr;  // per level-0 entry; sized at the first build
-  int *off0 = call.temp<int>(n + 1);  // n + 1: the pair loads read an even count
+  int *off0 = nullptr, *off1 = nullptr;  // level-0 lists: this one, and the next rebuild's
   R *dt = call.temp<R>(1);
   unsigned long long *key = call.temp<unsigned long long>(1);
   double *dtl = dt_log ? call.temp<double>(n_steps) : nullptr;
-  int *claim = new_claims(call, gb);  // reused by every rebuild (left unclaimed)
   if (!call.ok()) return lsmgpu_get_last_error(nullptr, 0);
   cudaStream_t s = stream();
-  const int level = 3;
-  std::vector<int> lo, hi;
-  int ob[4];
+  if (dtl) cudaMemsetAsync(dtl, 0, sizeof(double) * n_steps, s);  // steps after the band has emptied
+  const Width<R> width((double)gamma);
   int n0 = 0, nrebuild = 0;
-  // the previous level-0 list of a rebuild (the first build scans the grid)
-  int *ox = nullptr, *oy = nullptr, *oz = nullptr;
   for (int step = 0; step < n_steps; step++) {
     if (step % rebuild_every == 0) {
-      long long c0 = 0;
-      PrevLevel0 prev;
-      if (nrebuild > 0) {
-        // phi changed only at level-0 cells since the last build: the new
-        // band's level 0 is drawn from the old one (Level0List); the old
-        // band's marks are cleared so the breadth-first levels start clean
-        int nlist = 0;
-        for (int lv = 0; lv <= level; lv++)
-          if (hi[lv] + 1 > nlist) nlist = hi[lv] + 1;
-        if (nlist > 0)
-          LSMGPU_LAUNCH(k_band_retire, (unsigned)((nlist + 255) / 256), 256, 0, nb, view((const U8 *)nb, gb), ix, iy,
-                        iz, nlist, n0, ox, oy, oz);
-        prev.ox = ox;
-        prev.oy = oy;
-        prev.oz = oz;
-        prev.n = n0;
+      Compaction c;
+      long long tot[3] = {0, 0, 0};
+      if (nrebuild == 0) {
+        FlowGrid<R> f{phi, width, nullptr};
+        if (!c.count(call, f, n, tot)) return lsmgpu_get_last_error(nullptr, 0);
+        if (tot[0] > 0) {
+          // later lists are sub-sequences of this one; an even number of
+          // elements for the pair loads, a 4-value record per entry pair in
+          // the FP32 form
+          off0 = call.temp<int>(tot[0] + 2);
+          off1 = call.temp<int>(tot[0] + 2);
+          rhs = call.temp<R>(packed ? 2 * tot[0] + 4 : tot[0]);
+          if (!call.ok()) return lsmgpu_get_last_error(nullptr, 0);
+          f.off = off0;
+          c.emit(f);
+          LSMGPU_LAUNCH(k_copy_fields<R>, (unsigned)((n + 2047) / 2048), 256, 0, phi, u1, u2, n);
+        }
+      } else if (n0 > 0) {
+        const FlowList<R> f{phi, width, off0, off1, u1, u2};
+        if (!c.count(call, f, n0, tot)) return lsmgpu_get_last_error(nullptr, 0);
+        c.emit(f);
+        int *t = off0;
+        off0 = off1;
+        off1 = t;
       }
-      if (!band_build<R>(call, phi, gb, nb, gb, ix, iy, iz, 0, (int)(n - 1), outer, 0, (int)(n - 1), (double)gamma,
-                         (double)beta, level, lo, hi, ob, &c0, claim, true, BandForm<R>(), nullptr,
-                         nrebuild > 0 ? &prev : nullptr))
-        return lsmgpu_get_last_error(nullptr, 0);
-      if (nrebuild == 0 && c0 > 0) {
-        // later level-0 lists are sub-sequences of this one
-        ox = call.temp<int>(c0);
-        oy = call.temp<int>(c0);
-        oz = call.temp<int>(c0);
-        // the FP32 form keeps a 4-value record per entry pair
-        rhs = call.temp<R>(packed ? 2 * c0 + 4 : c0);
-        if (!call.ok()) return lsmgpu_get_last_error(nullptr, 0);
-      }
-      n0 = (int)c0;
-      if (band_log) band_log[nrebuild] = c0;
+      n0 = (int)tot[0];
+      if (band_log) band_log[nrebuild] = tot[0];
       nrebuild++;
-      // stage fields hold phi^n on band levels 1..3 (every cell a level-0
-      // stencil reads besides level 0); level-0 cells are written by each
-      // stage before any stage reads them, so only levels 1..3 are copied
-      int nlist = 0;
-      for (int lv = 0; lv <= level; lv++)
-        if (hi[lv] + 1 > nlist) nlist = hi[lv] + 1;
-      if (n0 > 0)
-        LSMGPU_LAUNCH(k_band_offsets<R>, (unsigned)((n0 + 255) / 256), 256, 0, view((const R *)phi, gb), ix, iy, iz,
-                      n0, off0);
-      const int first = n0;  // levels 1..3 follow level 0 in the lists
-      if (n0 > 0 && nlist > first)
-        LSMGPU_LAUNCH(k_copy_band<R>, (unsigned)((nlist - first + 255) / 256), 256, 0, (const R *)phi, u1, u2,
-                      view((const R *)phi, gb), ix + first, iy + first, iz + first, nlist - first);
     }
     if (n0 == 0) continue;
     BandArgs<R> a{};
-    a.ix = ix; a.iy = iy; a.iz = iz;
     a.off0 = off0;
     a.n0 = n0;
     a.dx = dx; a.a_n = a_n; a.b_n = b_n; a.beta = beta; a.gamma = gamma; a.cfl = cfl;
