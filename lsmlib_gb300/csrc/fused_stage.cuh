@@ -329,6 +329,17 @@ __device__ __forceinline__ float pow2_recip(float x) {
 }
 __device__ __forceinline__ float2 pow2_recip2(float2 x) { return make_float2(pow2_recip(x.x), pow2_recip(x.y)); }
 
+// num / den per lane for den a normal number below 2^126: the product with
+// the approximate reciprocal, without the scaling a general quotient carries
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 quot2(float2 num, float2 den) {
+  return mul2(num, make_float2(rcp_ftz(den.x), rcp_ftz(den.y)));
+}
+
 // WENO5-JS on two cells at once, the epsilon-scaled weight form of
 // weno5_fast with the common factors folded: only S/eps enters the weights,
 // so the smoothness indicators are kept as 4 S and epsilon as 12 eps (the
@@ -368,7 +379,7 @@ __device__ __forceinline__ float2 weno5_x2(float2 v1, float2 v2, float2 v3, floa
   const float2 n3 = mul2(mul2(sp(3.f), q12), q12);
   const float2 num = fma2(n1, P1, fma2(n2, P2, mul2(n3, P3)));
   const float2 den = add2(add2(n1, n2), n3);
-  return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+  return quot2(num, den);
 }
 
 // Both one-sided WENO5 values of one axis for two cells: minus side on
@@ -424,7 +435,7 @@ __device__ __forceinline__ void weno5_pm_x2(const float2 D[6], float2 &gp, float
     const float2 n3 = mul2(mul2(sp(3.f), q12), q12);
     const float2 num = fma2(n1, p1, fma2(n2, p2, mul2(n3, p3)));
     const float2 den = add2(add2(n1, n2), n3);  // <= 1e32 < 2^126
-    return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+    return quot2(num, den);
   };
   gm = combine(q1m, q2m, q3m, P1m, A, B);
   gp = combine(q1p, q2p, q3p, P1p, B, A);
