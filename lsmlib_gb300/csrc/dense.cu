@@ -263,17 +263,35 @@ __global__ void k_gradmag(View<const R> px, View<const R> py, View<const R> pz, 
 // kind 1: un = 0.5*(u + u1 + dt*L) (:240-241)
 // kind 2: u2 = 0.75*u + 0.25*(u1 + dt*L) (:403-404)
 // kind 3: un = u/3 + 2/3*(u2 + dt*L) (:490-492)
+// Bound by memory; dt L on the FP64 unit, the products by constants on the
+// integer pipes, which together stay below the memory's time (192^3, stage 2:
+// 71 us with every product on the FP64 unit and one cell per thread).
 template <int KIND>
-__global__ void k_rk(View<R> out, View<const R> a, View<const R> u, View<const R> rhs, Box fb, R dt) {
-  LSMGPU_CELL_INDEX(fb, i, j, k);
-  const R L = rhs(i, j, k);
-  R v;
-  const R w = mul_(dt, L);
-  if (KIND == 0) v = u(i, j, k) + w;
-  if (KIND == 1) v = R(0.5) * (u(i, j, k) + a(i, j, k) + w);
-  if (KIND == 2) v = fma(R(0.25), a(i, j, k) + w, mul_(R(0.75), u(i, j, k)));  // the product by 1/4 is exact
-  if (KIND == 3) v = mul_(R(1.0 / 3.0), u(i, j, k)) + mul_(R(2.0 / 3.0), a(i, j, k) + w);
-  out(i, j, k) = v;
+__global__ void __launch_bounds__(256) k_rk(View<R> out, View<const R> a, View<const R> u, View<const R> rhs, Box fb,
+                                            R dt, int planes) {
+  const int i = fb.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = fb.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
+  const int k0 = first_plane(fb, planes), n = min(planes, fb.hi[2] - k0 + 1);
+  if (i > fb.hi[0] || j > fb.hi[1]) return;
+  R L[kPlanes], U[kPlanes], A[kPlanes];
+#pragma unroll
+  for (int q = 0; q < kPlanes; q++)
+    if (q < n) {
+      L[q] = rhs(i, j, k0 + q);
+      U[q] = u(i, j, k0 + q);
+      if (KIND != 0) A[q] = a(i, j, k0 + q);
+    }
+#pragma unroll
+  for (int q = 0; q < kPlanes; q++)
+    if (q < n) {
+      const R w = dt * L[q];
+      R v;
+      if (KIND == 0) v = U[q] + w;
+      if (KIND == 1) v = R(0.5) * (U[q] + A[q] + w);
+      if (KIND == 2) v = fma(R(0.25), A[q] + w, mul_(R(0.75), U[q]));  // the product by 1/4 is exact
+      if (KIND == 3) v = mul_(R(1.0 / 3.0), U[q]) + mul_(R(2.0 / 3.0), A[q] + w);
+      out(i, j, k0 + q) = v;
+    }
 }
 
 template <int KIND>
@@ -289,22 +307,41 @@ void rk(const char *name, R *out, const Box &ob, const R *a, const Box &ab, cons
   View<const R> U = view((const R *)call.in(u, ub.size()), ub);
   View<const R> L = view((const R *)call.in(rhs, rb.size()), rb);
   if (!call.ok()) return;
-  Grid3 g = cover(fb);
-  LSMGPU_LAUNCH(k_rk<KIND>, g.grid, g.block, 0, O, A, U, L, fb, dt);
+  int planes;
+  const Grid3 g = cover_planes(fb, planes);
+  LSMGPU_LAUNCH(k_rk<KIND>, g.grid, g.block, 0, O, A, U, L, fb, dt, planes);
   call.finish();
 }
 
 // ---- level set RHS terms ------------------------------------------------------
-__global__ void k_fill(View<R> a, Box b, R v) {
-  LSMGPU_CELL_INDEX(b, i, j, k);
-  a(i, j, k) = v;
+__global__ void __launch_bounds__(256) k_zero(R *p, long long n) {
+  const long long base = (long long)blockIdx.x * (256 * kPlanes) + threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kPlanes; q++)
+    if (base + 256 * q < n) p[base + 256 * q] = R(0);
 }
 
-__global__ void k_add_advection(View<R> rhs, View<const R> px, View<const R> py, View<const R> pz,
-                                View<const R> vx, View<const R> vy, View<const R> vz, Box fb) {
-  LSMGPU_CELL_INDEX(fb, i, j, k);
-  rhs(i, j, k) = rhs(i, j, k) - (mul_(vx(i, j, k), px(i, j, k)) + mul_(vy(i, j, k), py(i, j, k)) +
-                                 mul_(vz(i, j, k), pz(i, j, k)));
+// Bound by memory: two products on the FP64 unit beside the three sums, the
+// third on the integer pipes.
+__global__ void __launch_bounds__(256) k_add_advection(View<R> rhs, View<const R> px, View<const R> py,
+                                                       View<const R> pz, View<const R> vx, View<const R> vy,
+                                                       View<const R> vz, Box fb, int planes) {
+  const int i = fb.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = fb.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
+  const int k0 = first_plane(fb, planes), n = min(planes, fb.hi[2] - k0 + 1);
+  if (i > fb.hi[0] || j > fb.hi[1]) return;
+  R r[kPlanes], g[kPlanes][3], v[kPlanes][3];
+#pragma unroll
+  for (int q = 0; q < kPlanes; q++)
+    if (q < n) {
+      const int k = k0 + q;
+      r[q] = rhs(i, j, k);
+      g[q][0] = px(i, j, k); g[q][1] = py(i, j, k); g[q][2] = pz(i, j, k);
+      v[q][0] = vx(i, j, k); v[q][1] = vy(i, j, k); v[q][2] = vz(i, j, k);
+    }
+#pragma unroll
+  for (int q = 0; q < kPlanes; q++)
+    if (q < n) rhs(i, j, k0 + q) = r[q] - (v[q][0] * g[q][0] + v[q][1] * g[q][1] + mul_(v[q][2], g[q][2]));
 }
 
 // vn field (const_vn == false) or constant (const_vn == true)
@@ -418,6 +455,66 @@ struct RedArgs {
 
 constexpr int kRedZ = 8;  // planes a thread walks: fewer blocks to fold, more loads in flight
 
+// an FP32 bound from above on |x| (infinity where FP32 does not reach, and
+// for NaN), and one from below on x (for x < 2^-100: less than any bound)
+__device__ __forceinline__ float above32(R x) {
+  const fpi::W2 w = fpi::words(x);
+  const uint32_t h = w.hi & 0x7fffffffu;
+  if (h >= (1100u << 20)) return INFINITY;
+  const uint32_t f = ((h - (896u << 20)) << 3) | (w.lo >> 29);
+  return h < (923u << 20) ? 0x1p-100f : __uint_as_float(f + 1u);
+}
+__device__ __forceinline__ float below32(R x) {
+  const fpi::W2 w = fpi::words(x);
+  if (w.hi >= (1100u << 20)) return w.hi >= 0x80000000u ? -1.f : 0x1p76f;
+  return w.hi < (923u << 20) ? -1.f : __uint_as_float(((w.hi - (896u << 20)) << 3) | (w.lo >> 29));
+}
+
+// Advection dt (mode 0): the maximum of |u|/dx + |v|/dy + |w|/dz.  A cell
+// whose FP32 bound does not exceed the maximum so far cannot raise it, which
+// settles nearly every cell without FP64 arithmetic (the running maximum of
+// the earlier blocks is the start); the others evaluate the reference's sum.
+// Bound by memory then (384^3: 1.18 ms with every cell in FP64).
+__global__ void __launch_bounds__(256) k_advection_max(RedArgs A, Box ib, unsigned long long *key) {
+  const int i = ib.lo[0] + blockIdx.x * 32 + threadIdx.x;
+  const int j = ib.lo[1] + blockIdx.y * 8 + threadIdx.y;
+  const int k0 = ib.lo[2] + blockIdx.z * kRedZ, n = min(kRedZ, ib.hi[2] - k0 + 1);
+  unsigned long long best = __ldcg(key);
+  float low = below32(okey_inv(best));
+  const float ix = above32(A.ix), iy = above32(A.iy), iz = above32(A.iz);
+  if (i <= ib.hi[0] && j <= ib.hi[1]) {
+    for (int h = 0; h < kRedZ; h += kPlanes) {
+      R u[kPlanes], v[kPlanes], w[kPlanes];
+      bool take[kPlanes];
+#pragma unroll
+      for (int q = 0; q < kPlanes; q++) {
+        const int k = k0 + h + q;
+        take[q] = h + q < n;
+        if (take[q]) {
+          u[q] = A.a(i, j, k);
+          v[q] = A.b(i, j, k);
+          w[q] = A.c(i, j, k);
+          if (A.cv_sgn != 0) take[q] = is_pos_(flip_if_(A.cv(i, j, k), A.cv_sgn < 0));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kPlanes; q++) {
+        if (!take[q]) continue;
+        const float bound =
+            __fmaf_ru(above32(u[q]), ix, __fmaf_ru(above32(v[q]), iy, __fmul_ru(above32(w[q]), iz)));
+        if (bound <= low) continue;
+        const R s = fabs(u[q]) * A.ix + fabs(v[q]) * A.iy + fabs(w[q]) * A.iz;
+        if (fpi::mag(s) <= fpi::kInfBits && okey(s) > best) {  // a NaN exceeds nothing
+          best = okey(s);
+          low = below32(s);
+        }
+      }
+    }
+  }
+  block_max_commit(best, key);
+}
+
+// mode 3: |a - b|; modes 1, 2: the normal velocity's H / dx
 template <int MODE>
 __global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned long long *key) {
   const int i = ib.lo[0] + blockIdx.x * 32 + threadIdx.x;
@@ -432,9 +529,7 @@ __global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned 
         if (!is_pos_(flip_if_(c, A.cv_sgn < 0))) continue;
       }
       R v;
-      if (MODE == 0) {
-        v = mul_(abs_(A.a(i, j, k)), A.ix) + mul_(abs_(A.b(i, j, k)), A.iy) + mul_(abs_(A.c(i, j, k)), A.iz);
-      } else if (MODE == 3) {
+      if (MODE == 3) {
         v = abs_(A.a(i, j, k) - A.b(i, j, k));
       } else {
         const R avn = abs_((MODE == 2) ? A.vn_const : A.vn(i, j, k));
@@ -473,7 +568,8 @@ void reduce_max(Call &call, RedArgs &A, const Box &ib, R *out, R cfl, R init) {
   if (!ib.empty()) {
     const dim3 grd((unsigned)((ib.n(0) + 31) / 32), (unsigned)((ib.n(1) + 7) / 8),
                    (unsigned)((ib.n(2) + kRedZ - 1) / kRedZ));
-    LSMGPU_LAUNCH(k_reduce_max<MODE>, grd, dim3(32, 8), 0, A, ib, key);
+    if constexpr (MODE == 0) LSMGPU_LAUNCH(k_advection_max, grd, dim3(32, 8), 0, A, ib, key);
+    else LSMGPU_LAUNCH(k_reduce_max<MODE>, grd, dim3(32, 8), 0, A, ib, key);
   }
   LSMGPU_LAUNCH(k_finish_scalar, 1, 1, 0, key, dout, MODE, cfl, init);
   call.finish();
@@ -722,8 +818,7 @@ void lsm3dzerooutlevelseteqnrhs_(R *lse_rhs, BOXARG(r)) {
   if (rb.empty()) return;
   View<R> O = view(call.out(lse_rhs, rb.size()), rb);
   if (!call.ok()) return;
-  Grid3 g = cover(rb);
-  LSMGPU_LAUNCH(k_fill, g.grid, g.block, 0, O, rb, R(0));
+  LSMGPU_LAUNCH(k_zero, (unsigned)((rb.size() + 256 * kPlanes - 1) / (256 * kPlanes)), 256, 0, O.p, rb.size());
   call.finish();
 }
 
@@ -742,8 +837,9 @@ void lsm3daddadvectiontermtolserhs_(R *lse_rhs, BOXARG(r), const R *phi_x, const
   View<const R> VX = view((const R *)call.in(vel_x, nv), vb), VY = view((const R *)call.in(vel_y, nv), vb),
                 VZ = view((const R *)call.in(vel_z, nv), vb);
   if (!call.ok()) return;
-  Grid3 g3 = cover(fb);
-  LSMGPU_LAUNCH(k_add_advection, g3.grid, g3.block, 0, O, X, Y, Z, VX, VY, VZ, fb);
+  int planes;
+  const Grid3 g3 = cover_planes(fb, planes);
+  LSMGPU_LAUNCH(k_add_advection, g3.grid, g3.block, 0, O, X, Y, Z, VX, VY, VZ, fb, planes);
   call.finish();
 }
 

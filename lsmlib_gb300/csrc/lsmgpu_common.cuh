@@ -150,14 +150,33 @@ struct Grid3 {
 };
 inline Grid3 cover(const Box &fb, int bx = 32, int by = 4, int bz = 2) {
   Grid3 g;
-  // one plane (a 2D call) or one row (1D): the block's threads go to the
+  // a thin box (a face plane, a 2D or 1D call): the block's threads go to the
   // axes that are there
-  if (fb.n(2) == 1) { by *= bz; bz = 1; }
-  if (fb.n(2) == 1 && fb.n(1) == 1) { bx *= by; by = 1; }
+  const int threads = bx * by * bz;
+  while (bx > 1 && bx / 2 >= fb.n(0)) bx /= 2;
+  if (fb.n(2) == 1) bz = 1;
+  by = threads / (bx * bz);
+  while (by > 1 && by / 2 >= fb.n(1)) by /= 2;
+  if (fb.n(2) > 1) bz = threads / (bx * by) < 64 ? threads / (bx * by) : 64;
+  if (fb.n(2) == 1 && fb.n(1) == 1) bx = threads;
   g.block = dim3(bx, by, bz);
   g.grid = dim3((unsigned)((fb.n(0) + bx - 1) / bx), (unsigned)((fb.n(1) + by - 1) / by),
                 (unsigned)((fb.n(2) + bz - 1) / bz));
   return g;
+}
+
+// The same for memory-bound kernels whose threads take up to kPlanes cells
+// along z, all loads before the arithmetic: `planes` (1 or kPlanes) is passed
+// to the kernel, which starts at first_plane(fb, planes).
+constexpr int kPlanes = 4;
+inline Grid3 cover_planes(const Box &fb, int &planes) {
+  planes = fb.n(2) >= kPlanes ? kPlanes : 1;
+  Box b = fb;
+  b.hi[2] = b.lo[2] + (int)((fb.n(2) + planes - 1) / planes) - 1;
+  return cover(b);
+}
+__device__ __forceinline__ int first_plane(const Box &fb, int planes) {
+  return fb.lo[2] + planes * (int)(blockIdx.z * blockDim.z + threadIdx.z);
 }
 
 #define LSMGPU_CELL_INDEX(fb, i, j, k)                 \
