@@ -16,7 +16,10 @@ binding used by the tests and the benchmark:
 """
 import ctypes
 import json
+import operator
 import os
+import struct
+import threading
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblsmgpu.so")
@@ -101,15 +104,56 @@ _SCALAR_CT = {"real": ctypes.c_double, "double": ctypes.c_double, "int": ctypes.
 
 def _ptr(v):
     """Address of an array argument: numpy array, torch tensor or int."""
-    if v is None:
-        return None
-    if isinstance(v, int):
-        return ctypes.c_void_p(v)
+    a = _address(v)
+    return None if a is None else ctypes.c_void_p(a)
+
+
+_SCALAR_FMT = {"real": "d", "double": "d", "int": "i", "logical": "i", "int1": "B"}
+
+
+class _Plan:
+    """One entry point's call on one library: the function, one buffer for
+    all its scalar arguments (Fortran passes them by reference) and the
+    argument list, whose pointer objects stay while the arrays' addresses and
+    the scalars' values change from call to call."""
+
+    def __init__(self, handle, sym, spec):
+        self.handle, self.spec = handle, spec
+        # a function object of this plan's own (CDLL shares the attribute form)
+        self.fn = handle[sym] if isinstance(handle, ctypes.CDLL) else getattr(handle, sym)
+        self.fn.restype = None
+        self.kinds = [kind for _n, kind, is_arr, _w in spec["args"] if not is_arr]
+        self.names = tuple(name for name, _k, is_arr, _w in spec["args"] if not is_arr)
+        if len(self.names) > 1:
+            self.pick = operator.itemgetter(*self.names)
+        else:
+            self.pick = lambda values: [values[name] for name in self.names]
+        fields = struct.Struct("@" + "".join(_SCALAR_FMT[k] for k in self.kinds))
+        self.pack_into, self.unpack_from = fields.pack_into, fields.unpack_from
+        self.buf = ctypes.create_string_buffer(max(fields.size, 1))
+        base, fmt, self.args, self.arrays = ctypes.addressof(self.buf), "@", [], []
+        for name, kind, is_arr, _w in spec["args"]:
+            pointer = ctypes.c_void_p()
+            self.args.append(pointer)
+            if is_arr:
+                self.arrays.append((pointer, name))
+            else:
+                fmt += _SCALAR_FMT[kind]
+                pointer.value = base + struct.calcsize(fmt) - struct.calcsize(_SCALAR_FMT[kind])
+
+
+def _address(v):
+    """Address of an array argument as an int (None for a null pointer)."""
+    if v is None or isinstance(v, int):
+        return v
     if hasattr(v, "data_ptr"):
-        return ctypes.c_void_p(v.data_ptr())
+        return v.data_ptr()
     if hasattr(v, "ctypes"):
-        return ctypes.c_void_p(v.ctypes.data)
+        return v.ctypes.data
     raise TypeError("unsupported array argument %r" % type(v))
+
+
+_plans = threading.local()
 
 
 def invoke(handle, sym, values, abi=None):
@@ -121,21 +165,30 @@ def invoke(handle, sym, values, abi=None):
     after the call (so outputs such as dt can be read back).
     """
     spec = (abi or ABI)[sym]
-    args, refs = [], {}
-    for name, kind, is_arr, _written in spec["args"]:
-        if name not in values:
-            raise KeyError("%s: missing argument %s" % (sym, name))
-        v = values[name]
-        if is_arr:
-            args.append(_ptr(v))
-        else:
-            r = _SCALAR_CT[kind](v)
-            refs[name] = r
-            args.append(ctypes.byref(r))
-    fn = getattr(handle, sym)
-    fn.restype = None
-    fn(*args)
-    return {k: r.value for k, r in refs.items()}
+    # per thread, and out of the table during the call, so that no two calls
+    # share a plan's buffer; a call that raises drops it
+    plan = _plans.__dict__.pop(sym, None)
+    if plan is None or plan.handle is not handle or plan.spec is not spec:
+        plan = _Plan(handle, sym, spec)
+    try:
+        for pointer, name in plan.arrays:
+            v = values[name]
+            try:
+                pointer.value = v.data_ptr()
+            except AttributeError:
+                pointer.value = _address(v)
+        scalars = plan.pick(values)
+    except KeyError as e:
+        raise KeyError("%s: missing argument %s" % (sym, e.args[0])) from None
+    try:
+        plan.pack_into(plan.buf, 0, *scalars)
+    except struct.error:
+        # a value outside its C type's range: wrapped as ctypes wraps it
+        plan.pack_into(plan.buf, 0, *[_SCALAR_CT[k](v).value for k, v in zip(plan.kinds, scalars)])
+    plan.fn(*plan.args)
+    out = dict(zip(plan.names, plan.unpack_from(plan.buf, 0)))
+    _plans.__dict__[sym] = plan
+    return out
 
 
 # ---------------------------------------------------------------------------
