@@ -6,7 +6,8 @@
 // global work counter, so small and large grids share the machine without a
 // launch per grid; each CTA double-buffers its tiles in shared memory with
 // TMA loads from per-grid tensor maps kept in global memory.  The n_steps x 3
-// stage launches of a call are captured once into a CUDA graph and replayed.
+// stage launches of a call are one CUDA graph, kept for later calls with the
+// same buffers and launch parameters.
 // Each grid gets the tile shape (32 x 8 or 16 x 16 cells of a plane) that
 // pads its x rows least: the 256 threads of a CTA cover one tile plane, and
 // lanes past the row's end idle through the whole tile.  A table of
@@ -44,7 +45,7 @@ using fused::TY;
 struct GridDesc {
   Layout L;
   long long off;  // element offset of this grid's region in each work buffer
-  float vconst[3], inv[3], dt;
+  float vconst[3], inv[3], floor4[3], dt;
   int tile_base;  // first global tile index of this grid
   int ntx, nty, ntz;
   int wide;       // 1: 32 x 8 tiles, 0: 16 x 16 tiles
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(TX * TY) k_batch_stage(const GridDesc *__restr
     for (int d = 0; d < 3; d++) {
       a.vconst[d] = G.vconst[d];
       a.inv[d] = G.inv[d];
+      a.floor4[d] = G.floor4[d];
     }
     a.dt = G.dt;
     a.dx_sq = 0.f;
@@ -137,26 +139,35 @@ __global__ void __launch_bounds__(TX * TY) k_batch_stage(const GridDesc *__restr
     if (G.wide)
       fused::f32_tile<fused::ADV_CONST, TZ_, 32, 8>(tile, a, r.bx * 32, r.by * 8, r.bz * TZ_, tid & 31, tid >> 5);
     else
-      fused::f32_tile<fused::ADV_CONST, TZ_, 16, 16>(tile, a, r.bx * 16, r.by * 16, r.bz * TZ_, tid & 15, tid >> 4);
+      // a warp takes rows two apart: their staged rows lie 48 words apart, so
+      // its halves read different banks (adjacent ones, 24 apart, do not)
+      fused::f32_tile<fused::ADV_CONST, TZ_, 16, 16>(tile, a, r.bx * 16, r.by * 16, r.bz * TZ_, tid & 15,
+                                                     ((tid >> 6) << 2) | ((tid >> 5) & 1) | ((tid >> 3) & 2));
     cur ^= 1;
     t = tn;
   }
 }
 
 // copies between the caller's packed LSMLIB arrays (3 ghost cells per side)
-// and the padded work regions; blockIdx.y is the grid
-__global__ void k_batch_pack(float *work, float *user, const GridDesc *gd, const long long *uoff, int unpack) {
+// and the padded work regions; blockIdx.y is the grid, a warp takes x rows
+// (an index division per row, not per cell)
+__global__ void __launch_bounds__(256) k_batch_pack(float *work, float *user, const GridDesc *gd,
+                                                    const long long *uoff, int unpack) {
   const GridDesc &G = gd[blockIdx.y];
-  const Layout &L = G.L;
-  const long long ux = L.nx + 6, uy = L.ny + 6, uz = L.nz + 6;
-  const long long n = ux * uy * uz;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % ux) - 3, j = (int)((e / ux) % uy) - 3, k = (int)(e / (ux * uy)) - 3;
-    const long long w = G.off + L.idx(i, j, k);
-    if (unpack)
-      user[uoff[blockIdx.y] + e] = work[w];
-    else
-      work[w] = user[uoff[blockIdx.y] + e];
+  const Layout L = G.L;
+  const int ux = L.nx + 6, uy = L.ny + 6;
+  const long long rows = (long long)uy * (L.nz + 6);
+  float *const w0 = work + G.off;
+  float *const u0 = user + uoff[blockIdx.y];
+  for (long long r = blockIdx.x * 8 + threadIdx.x / 32; r < rows; r += gridDim.x * 8) {
+    const int k = (int)(r / uy), j = (int)(r - (long long)k * uy);
+    float *const w = w0 + L.idx(-3, j - 3, k - 3);
+    float *const u = u0 + r * ux;
+    if (unpack) {
+      for (int i = threadIdx.x % 32; i < ux; i += 32) u[i] = w[i];
+    } else {
+      for (int i = threadIdx.x % 32; i < ux; i += 32) w[i] = u[i];
+    }
   }
 }
 
@@ -258,6 +269,7 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
       for (int d = 0; d < 3; d++) {
         G.vconst[d] = vel[3 * g + d];
         G.inv[d] = 1.0f / spacing[3 * g + d];
+        G.floor4[d] = fused::eps_floor4(spacing[3 * g + d]);
       }
       G.dt = dt[g];
       // the shape that pads the x rows less (16-wide on a tie is no better)
@@ -301,8 +313,8 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
   if (!call.ok()) return lsmgpu_get_last_error(nullptr, 0);
   cudaMemcpyAsync(uoff_d, uoff.data(), sizeof(long long) * n_grids, cudaMemcpyHostToDevice, s);
   cudaMemsetAsync(err, 0, sizeof(int), s);
-  cudaMemsetAsync(B, 0, sizeof(float) * b.total, s);
-  cudaMemsetAsync(C, 0, sizeof(float) * b.total, s);
+  // B and C need no initial values: a stage writes every interior cell of its
+  // output and the periodic images that the next stage reads
 
   std::vector<CUtensorMap> tmh(3 * (size_t)n_grids);
   auto encode_all = [&](int tz) -> bool {
@@ -333,9 +345,10 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
 
   auto run_stage = [&](int tz, int stage, int *counter, int blocks) {
-    if (tz == 4) launch_batch_stage<4>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, s);
-    else if (tz == 16) launch_batch_stage<16>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, s);
-    else launch_batch_stage<8>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, s);
+    cudaStream_t q = stream();  // the capturing stream while a graph is captured
+    if (tz == 4) launch_batch_stage<4>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, q);
+    else if (tz == 16) launch_batch_stage<16>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, q);
+    else launch_batch_stage<8>(gd, tm, trd, b, stage, A, B, C, counter, err, 1, blocks, q);
   };
 
   if (want_loop) {
@@ -352,7 +365,7 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
           a.L = G.L;
           a.phi_n = A + G.off;
           a.out = (stage == 1 ? B : (stage == 2 ? C : A)) + G.off;
-          for (int d = 0; d < 3; d++) { a.vconst[d] = G.vconst[d]; a.inv[d] = G.inv[d]; }
+          for (int d = 0; d < 3; d++) { a.vconst[d] = G.vconst[d]; a.inv[d] = G.inv[d]; a.floor4[d] = G.floor4[d]; }
           a.dt = G.dt;
           a.stage = stage;
           a.periodic = 1;
@@ -412,43 +425,20 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
     if (!encode_all(tz)) { call.fail("tensor map encoding failed"); return LSMGPU_ERR_CUDA; }
     const int blocks = per_sm * nsm;
     const long long ncounter = 3LL * n_steps;
-    if (use_graph && n_steps > 0) {
-      // capture on a private stream, ordered after the library stream
-      cudaStream_t cs;
-      cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-      cudaEvent_t ev;
-      cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-      cudaEventRecord(ev, s);
-      cudaStreamWaitEvent(cs, ev, 0);
-      cudaGraph_t graph;
-      cudaGraphExec_t exec;
-      cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-      cudaMemsetAsync(counters, 0, sizeof(int) * ncounter, cs);
-      for (int step = 0; step < n_steps; step++)
-        for (int stage = 1; stage <= 3; stage++) {
-          int *ctr = counters + 3 * step + stage - 1;
-          if (tz == 4) launch_batch_stage<4>(gd, tm, trd, b, stage, A, B, C, ctr, err, 1, blocks, cs);
-          else if (tz == 16) launch_batch_stage<16>(gd, tm, trd, b, stage, A, B, C, ctr, err, 1, blocks, cs);
-          else launch_batch_stage<8>(gd, tm, trd, b, stage, A, B, C, ctr, err, 1, blocks, cs);
-        }
-      cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-      if (ce != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
-        cudaStreamDestroy(cs);
-        call.fail("CUDA graph capture failed");
-        return LSMGPU_ERR_CUDA;
-      }
-      cudaGraphLaunch(exec, cs);
-      cudaEventRecord(ev, cs);
-      cudaStreamWaitEvent(s, ev, 0);
-      cudaStreamSynchronize(cs);
-      cudaGraphExecDestroy(exec);
-      cudaGraphDestroy(graph);
-      cudaEventDestroy(ev);
-      cudaStreamDestroy(cs);
-    } else {
-      cudaMemsetAsync(counters, 0, sizeof(int) * ncounter, s);
+    // all stages of the call, replayed as one CUDA graph when the same buffers
+    // and launch parameters come again (the grids' sizes, velocities and
+    // tensor maps are read from device memory)
+    auto stages = [&]() {
+      cudaMemsetAsync(counters, 0, sizeof(int) * ncounter, stream());
       for (int step = 0; step < n_steps; step++)
         for (int stage = 1; stage <= 3; stage++) run_stage(tz, stage, counters + 3 * step + stage - 1, blocks);
+    };
+    if (n_steps > 0) {
+      GraphKey gk;
+      gk.add((int)0x62617463);  // this call's kind among the cached graphs
+      gk.add(tz); gk.add(blocks); gk.add(n_steps); gk.add(b.ntiles);
+      gk.add(gd); gk.add(tm); gk.add(trd); gk.add(A); gk.add(B); gk.add(C); gk.add(counters); gk.add(err);
+      if (!use_graph || !graph_replay(gk, stages)) stages();
     }
   }
   {

@@ -416,6 +416,8 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   for (int d = 0; d < 3; d++) a.vel[d] = V[d];
   a.vconst[0] = (R)rs.vconst[0]; a.vconst[1] = (R)rs.vconst[1]; a.vconst[2] = (R)rs.vconst[2];
   a.inv[0] = R(1.0) / (R)rs.dx; a.inv[1] = R(1.0) / (R)rs.dy; a.inv[2] = R(1.0) / (R)rs.dz;
+  const double d3[3] = {rs.dx, rs.dy, rs.dz};
+  for (int d = 0; d < 3; d++) a.floor4[d] = (R)eps_floor4((float)d3[d]);
   a.dt = (R)rs.dt;
   {
     R m = rmax(rmax((R)rs.dx, (R)rs.dy), (R)rs.dz);

@@ -61,6 +61,7 @@ struct StageArgs {
   R *out;
   R vconst[3];       // constant velocity (ADV_CONST)
   R inv[3];          // 1/dx, 1/dy, 1/dz
+  R floor4[3];       // FP32 ADV_CONST: eps_floor4 per axis
   R dt, dx_sq;
   int stage;         // 1, 2 or 3
   int use0;          // reinitialization sign from phi0
@@ -69,6 +70,14 @@ struct StageArgs {
                      // the kernel computes in shared memory from the tile
   int *err;
 };
+
+// 4 (1e-36 dx^2): LSMLIB's floor is in units of the divided differences.  Kept
+// a normal number (for dx below 0.06 the floor is larger than LSMLIB's then,
+// which only data below about 1e-19 dx can tell).
+inline float eps_floor4(float dx) {
+  const float f = 4e-36f * dx * dx;
+  return f > 1.5e-38f ? f : 1.5e-38f;
+}
 
 // One-axis extrapolation of LSMLIB's ghost-cell routines
 // (boundary_conditions3d.f:46-462) at distance g from the edge value e, with
@@ -170,28 +179,6 @@ __device__ __forceinline__ float weno5_fast(float v1, float v2, float v3, float 
   q1 *= q1; q2 *= q2; q3 *= q3;
   const float n1 = 0.1f * (q2 * q3), n2 = 0.6f * (q1 * q3), n3 = 0.3f * (q1 * q2);
   return __fdividef(fmaf(n1, p1, fmaf(n2, p2, n3 * p3)), n1 + n2 + n3);
-}
-
-// reinitialization RHS; the FP32 form keeps the FP64 zero tolerance so it
-// approximates the FP64 computation, and uses reciprocal square roots
-template <class R, bool EXACT>
-__device__ __forceinline__ R reinit_term(R pc, const R gp[3], const R gm[3], R dx_sq, bool use0) {
-  if constexpr (EXACT) {
-    return reinit_rhs<R>(pc, gp, gm, dx_sq, use0);
-  } else {
-    float st[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const float u = (pc > 0.f) ? fmaxf(-gp[d], 0.f) : fmaxf(gp[d], 0.f);
-      const float w = (pc > 0.f) ? fmaxf(gm[d], 0.f) : fmaxf(-gm[d], 0.f);
-      st[d] = fmaxf(u, w);
-    }
-    if (!(fabsf(pc) >= 1e-11f)) return 0.f;
-    const float n2 = fmaf(st[0], st[0], fmaf(st[1], st[1], st[2] * st[2]));
-    const float den = use0 ? fmaf(pc, pc, (float)dx_sq) : fmaf(pc, pc, n2 * (float)dx_sq);
-    const float sgn = pc * rsqrtf(den);
-    return sgn * (1.f - sqrtf(n2));
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -322,6 +309,22 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, sp(-1.f), a); }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_approx(x.x), rcp_approx(x.y)); }
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float2 max5(float2 a, float2 b, float2 c, float2 d, float2 e) {
+  return make_float2(max3f(max3f(a.x, b.x, c.x), d.x, e.x), max3f(max3f(a.y, b.y, c.y), d.y, e.y));
+}
+
 // 2^-floor(log2 x) for a positive normal float x, from the exponent bits (no
 // reciprocal instruction).  x * pow2_recip(x) lies in [1, 2).
 __device__ __forceinline__ float pow2_recip(float x) {
@@ -331,14 +334,7 @@ __device__ __forceinline__ float2 pow2_recip2(float2 x) { return make_float2(pow
 
 // num / den per lane for den a normal number below 2^126: the product with
 // the approximate reciprocal, without the scaling a general quotient carries
-__device__ __forceinline__ float rcp_ftz(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float2 quot2(float2 num, float2 den) {
-  return mul2(num, make_float2(rcp_ftz(den.x), rcp_ftz(den.y)));
-}
+__device__ __forceinline__ float2 quot2(float2 num, float2 den) { return mul2(num, rcp2(den)); }
 
 // WENO5-JS on two cells at once, the epsilon-scaled weight form of
 // weno5_fast with the common factors folded: only S/eps enters the weights,
@@ -346,9 +342,7 @@ __device__ __forceinline__ float2 quot2(float2 num, float2 den) {
 // factor 3 goes into the scale), and the weights as 10 d_k prod q_j^2.
 __device__ __forceinline__ float2 weno5_x2(float2 v1, float2 v2, float2 v3, float2 v4, float2 v5) {
   const float2 q1s = mul2(v1, v1), q2s = mul2(v2, v2), q3s = mul2(v3, v3), q4s = mul2(v4, v4), q5s = mul2(v5, v5);
-  float2 m;
-  m.x = fmaxf(fmaxf(fmaxf(q1s.x, q2s.x), fmaxf(q3s.x, q4s.x)), q5s.x);
-  m.y = fmaxf(fmaxf(fmaxf(q1s.y, q2s.y), fmaxf(q3s.y, q4s.y)), q5s.y);
+  const float2 m = max5(q1s, q2s, q3s, q4s, q5s);
   const float2 eps = fma2(sp(12e-6f), m, sp(12e-36f));  // 12 eps
   const float c13 = 1.f / 3.f, c76 = 7.f / 6.f, c116 = 11.f / 6.f, c16 = 1.f / 6.f, c56 = 5.f / 6.f;
   const float2 P1 = fma2(sp(c13), v1, fma2(sp(-c76), v2, mul2(sp(c116), v3)));
@@ -382,6 +376,43 @@ __device__ __forceinline__ float2 weno5_x2(float2 v1, float2 v2, float2 v3, floa
   return quot2(num, den);
 }
 
+// The backward WENO5 value of two cells from phi(c-3 .. c+2), in units of
+// phi (WENO5 is homogeneous of degree one: the caller scales by 1/dx once),
+// as the central candidate plus weighted third differences,
+//   p2 + w1 (p1 - p2) + w3 (p3 - p2),  p1 - p2 = TD(c-2) / 3,
+//   p3 - p2 = TD(c-1) / 6,  TD(s) = t(s) - t(s+1)
+// (the weights sum to 1): 53 packed operations where weno5_x2 with its scaled
+// differences takes 66.  Weights as in reinit_x2.cuh: q_k = S_k / eps + 1;
+// `floor4` is 4 times LSMLIB's floor of epsilon in these units (eps_floor4).
+__device__ __forceinline__ float2 weno5_backward_x2(const float2 x[6], float floor4) {
+  float2 D[5], sq[5];
+#pragma unroll
+  for (int q = 0; q < 5; q++) {
+    D[q] = sub2(x[q + 1], x[q]);
+    sq[q] = mul2(D[q], D[q]);
+  }
+  const float2 s = rcp2(fma2(sp(4e-6f), max5(sq[0], sq[1], sq[2], sq[3], sq[4]), sp(floor4)));  // 1 / (4 eps)
+  // second differences, and the outer parts u of the indicators:
+  // D1 - 4 D2 + 3 D3 = 2 t1 + (D3 - D1), 3 D3 - 4 D4 + D5 = 2 t3 + (D3 - D5)
+  const float2 t1 = fma2(sp(-2.f), D[1], add2(D[0], D[2]));
+  const float2 t2 = fma2(sp(-2.f), D[2], add2(D[1], D[3]));
+  const float2 t3 = fma2(sp(-2.f), D[3], add2(D[2], D[4]));
+  const float2 u1 = fma2(sp(2.f), t1, sub2(D[2], D[0]));
+  const float2 u2 = sub2(D[1], D[3]);
+  const float2 u3 = fma2(sp(2.f), t3, sub2(D[2], D[4]));
+  const float c133 = 13.f / 3.f;
+  const float2 q1 = fma2(fma2(mul2(sp(c133), t1), t1, mul2(u1, u1)), s, sp(1.f));
+  const float2 q2 = fma2(fma2(mul2(sp(c133), t2), t2, mul2(u2, u2)), s, sp(1.f));
+  const float2 q3 = fma2(fma2(mul2(sp(c133), t3), t3, mul2(u3, u3)), s, sp(1.f));
+  const float2 q23 = mul2(q2, q3), q13 = mul2(q1, q3), q12 = mul2(q1, q2);
+  const float2 A = mul2(q23, q23), B = mul2(q13, q13), C = mul2(q12, q12);  // < 3e30
+  // w1 = A / n, w3 = 3 C / n, n = A + 6 B + 3 C
+  const float2 num = fma2(sp(1.5f), mul2(C, sub2(t2, t3)), mul2(A, sub2(t1, t2)));
+  const float2 den = fma2(sp(3.f), A, fma2(sp(18.f), B, mul2(sp(9.f), C)));
+  const float2 p2 = fma2(sp(-1.f / 6.f), t2, mul2(sp(0.5f), add2(D[2], D[3])));
+  return fma2(num, rcp2(den), p2);
+}
+
 // Both one-sided WENO5 values of one axis for two cells: minus side on
 // D(c-2 .. c+2), plus side on D(c+3 .. c-1), given D[0..5] = D(c-2 .. c+3).
 // The two sides share two of their three candidate stencils (plus P2 = minus
@@ -392,11 +423,10 @@ __device__ __forceinline__ void weno5_pm_x2(const float2 D[6], float2 &gp, float
   float2 sq[6];
 #pragma unroll
   for (int i = 0; i < 6; i++) sq[i] = mul2(D[i], D[i]);
-  const float cx = fmaxf(fmaxf(sq[1].x, sq[2].x), fmaxf(sq[3].x, sq[4].x));
-  const float cy = fmaxf(fmaxf(sq[1].y, sq[2].y), fmaxf(sq[3].y, sq[4].y));
+  const float cx = max3f(sq[1].x, sq[2].x, sq[3].x), cy = max3f(sq[1].y, sq[2].y, sq[3].y);
   // 12 eps of each side, its power-of-two scale r and 12 eps r in [1, 2)
-  const float2 em = fma2(sp(12e-6f), make_float2(fmaxf(cx, sq[0].x), fmaxf(cy, sq[0].y)), sp(12e-36f));
-  const float2 ep = fma2(sp(12e-6f), make_float2(fmaxf(cx, sq[5].x), fmaxf(cy, sq[5].y)), sp(12e-36f));
+  const float2 em = fma2(sp(12e-6f), make_float2(max3f(cx, sq[4].x, sq[0].x), max3f(cy, sq[4].y, sq[0].y)), sp(12e-36f));
+  const float2 ep = fma2(sp(12e-6f), make_float2(max3f(cx, sq[4].x, sq[5].x), max3f(cy, sq[4].y, sq[5].y)), sp(12e-36f));
   const float2 rm = pow2_recip2(em), rp = pow2_recip2(ep);
   const float2 emr = mul2(em, rm), epr = mul2(ep, rp);
   const float2 rm3 = mul2(sp(3.f), rm), rp3 = mul2(sp(3.f), rp);
@@ -456,6 +486,9 @@ __device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<floa
   const int kmax = min(TZ_, L.nz - z0);
   const int st[3] = {1, SX_, SX_ * SY_};
   const float2 inv[3] = {sp(a.inv[0]), sp(a.inv[1]), sp(a.inv[2])};
+  // offsets of the column's periodic images along x and y (0: none)
+  const int oi = i < 3 ? L.nx : (i >= L.nx - 3 ? -L.nx : 0);
+  const int oj = j < 3 ? L.ny : (j >= L.ny - 3 ? -L.ny : 0);
 
   for (int tz = 0; tz < kmax; tz += 2) {
     const bool two = tz + 1 < kmax;  // the second lane is a real cell
@@ -464,51 +497,44 @@ __device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<floa
     const int k0 = z0 + tz, k1 = two ? k0 + 1 : k0;
     const long long cell0 = L.idx(i, j, k0), cell1 = L.idx(i, j, k1);
     float2 rhs;
-    if (MODE == REINIT) {
-      float gp0[3], gp1[3], gm0[3], gm1[3];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        float2 a7[7], v[6];  // phi / dx at c-3 .. c+3; scaled D1(c-2 .. c+3) for both cells
-#pragma unroll
-        for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
-#pragma unroll
-        for (int f = 0; f < 6; f++) v[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
-        float2 p, m;
-        weno5_pm_x2(v, p, m);
-        gp0[d] = p.x; gp1[d] = p.y;
-        gm0[d] = m.x; gm1[d] = m.y;
-      }
-      const float pc0 = a.use0 ? a.phi0[cell0] : c0[0];
-      const float pc1 = a.use0 ? a.phi0[cell1] : c1[0];
-      rhs.x = reinit_term<float, false>(pc0, gp0, gm0, a.dx_sq, a.use0 != 0);
-      rhs.y = reinit_term<float, false>(pc1, gp1, gm1, a.dx_sq, a.use0 != 0);
-    } else {
-      float vel0[3], vel1[3];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        vel0[d] = (MODE == ADV_CONST) ? a.vconst[d] : a.vel[d][cell0];
-        vel1[d] = (MODE == ADV_CONST) ? a.vconst[d] : a.vel[d][cell1];
-      }
+    {
       float2 dot = sp(0.f);
+      float vel0[3], vel1[3];
+      if constexpr (MODE == ADV_FIELD) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          vel0[d] = a.vel[d][cell0];
+          vel1[d] = a.vel[d][cell1];
+        }
+      }
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-        // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
-        // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);
-        // the six differences are loaded at fixed offsets and the lane's
-        // stencil is selected in registers
-        float2 a7[7], D[6];
-#pragma unroll
-        for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
-#pragma unroll
-        for (int f = 0; f < 6; f++) D[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
         if constexpr (MODE == ADV_CONST) {
-          // one velocity for the whole grid: the side and the zero cut are
-          // uniform, so the stencil is chosen by a (non-divergent) branch
-          const float u = a.vconst[d];
-          if (fabsf(u) < 1e-11f) continue;
-          const float2 g = u > 0.f ? weno5_x2(D[0], D[1], D[2], D[3], D[4]) : weno5_x2(D[5], D[4], D[3], D[2], D[1]);
-          dot = fma2(sp(u), g, dot);
+          // one velocity for the whole grid: a uniform branch walks the axis
+          // with the velocity's sign; the forward stencil of a negative
+          // velocity is the backward one of the mirrored line, negated, so
+          // v g = |v| g'
+          const float v = a.vconst[d];
+          if (fabsf(v) < 1e-11f) continue;
+          float2 x[6];
+          if (v > 0.f) {
+#pragma unroll
+            for (int q = 0; q < 6; q++) x[q] = make_float2(c0[(q - 3) * st[d]], c1[(q - 3) * st[d]]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 6; q++) x[q] = make_float2(c0[(3 - q) * st[d]], c1[(3 - q) * st[d]]);
+          }
+          dot = fma2(sp(fabsf(v) * a.inv[d]), weno5_backward_x2(x, a.floor4[d]), dot);
         } else {
+          // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
+          // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);
+          // the six differences are loaded at fixed offsets and the lane's
+          // stencil is selected in registers
+          float2 a7[7], D[6];
+#pragma unroll
+          for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
+#pragma unroll
+          for (int f = 0; f < 6; f++) D[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
           const bool b0 = vel0[d] > 0.f, b1 = vel1[d] > 0.f;
           float2 v[5];
 #pragma unroll
@@ -535,26 +561,26 @@ __device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<floa
       else
         u = fma2(sp(1.f / 3.f), un, mul2(sp(2.f / 3.f), fma2(sp(a.dt), rhs, u0)));
     }
-    for (int lane = 0; lane < (two ? 2 : 1); lane++) {
-      const int k = lane ? k1 : k0;
-      const float val = lane ? u.y : u.x;
-      const long long c = L.idx(i, j, k);
-      a.out[c] = val;
-      if (a.periodic) {
-        // the cell's periodic images in the ghost layers (up to 7: each
-        // combination of the axes along which it lies within 3 of a face)
-        const int oi = i < 3 ? L.nx : (i >= L.nx - 3 ? -L.nx : 0);
-        const int oj = j < 3 ? L.ny : (j >= L.ny - 3 ? -L.ny : 0);
-        const int ok = k < 3 ? L.nz : (k >= L.nz - 3 ? -L.nz : 0);
-        if (oi | oj | ok) {
-          const long long sx = oi, sy = L.py * oj, sz = L.pz * ok;
-          if (oi) a.out[c + sx] = val;
-          if (oj) a.out[c + sy] = val;
-          if (ok) a.out[c + sz] = val;
-          if (oi && oj) a.out[c + sx + sy] = val;
-          if (oi && ok) a.out[c + sx + sz] = val;
-          if (oj && ok) a.out[c + sy + sz] = val;
-          if (oi && oj && ok) a.out[c + sx + sy + sz] = val;
+    a.out[cell0] = u.x;
+    if (two) a.out[cell1] = u.y;
+    if (a.periodic) {
+      // the cells' periodic images in the ghost layers (up to 7: each
+      // combination of the axes along which a cell lies within 3 of a face)
+      const bool edge = k0 < 3 || k1 >= L.nz - 3;
+      if ((oi | oj) != 0 || edge) {
+        for (int lane = 0; lane < (two ? 2 : 1); lane++) {
+          const int k = lane ? k1 : k0;
+          const float val = lane ? u.y : u.x;
+          const long long c = lane ? cell1 : cell0;
+          const int ok = k < 3 ? L.nz : (k >= L.nz - 3 ? -L.nz : 0);
+          const long long dx = oi, dy = L.py * oj, dz = L.pz * ok;
+          if (oi) a.out[c + dx] = val;
+          if (oj) a.out[c + dy] = val;
+          if (ok) a.out[c + dz] = val;
+          if (oi && oj) a.out[c + dx + dy] = val;
+          if (oi && ok) a.out[c + dx + dz] = val;
+          if (oj && ok) a.out[c + dy + dz] = val;
+          if (oi && oj && ok) a.out[c + dx + dy + dz] = val;
         }
       }
     }

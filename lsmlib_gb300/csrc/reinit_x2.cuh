@@ -47,18 +47,6 @@ constexpr int RSX = RX + 8, RSY = RY + 6;  // staged tile in x and y
 constexpr int RZ_MAX = 10;        // planes of the deepest tile
 // staged tile of a tz-plane tile: 72 x 14 x (tz + 6) floats
 constexpr size_t reinit_x2_smem(int tz) { return (size_t)RSX * RSY * (tz + 6) * sizeof(float); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, sp(-1.f), a); }
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_approx(x.x), rcp_approx(x.y)); }
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -128,10 +116,6 @@ __device__ __forceinline__ void sides_both(const WQ &w, float2 tda, float2 tdb, 
   const float2 den_p = fma2(sp(6.f), w.q12, fma2(sp(18.f), w.q23, g));
   minus = fma2(num_m, rcp2(den_m), p2m);
   plus = fma2(sp(-1.f), mul2(num_p, rcp2(den_p)), p2p);
-}
-
-__device__ __forceinline__ float2 max5(float2 a, float2 b, float2 c, float2 d, float2 e) {
-  return make_float2(max3f(max3f(a.x, b.x, c.x), d.x, e.x), max3f(max3f(a.y, b.y, c.y), d.y, e.y));
 }
 
 // minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
