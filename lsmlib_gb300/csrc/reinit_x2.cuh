@@ -25,7 +25,8 @@
 //   minus(c) = p2 + w1 (p1 - p2) + w3 (p3 - p2),
 //   p1 - p2 = TD(c-2) / 3,  p3 - p2 = TD(c-1) / 6,
 //   TD(s) = D(s) - 3 D(s+1) + 3 D(s+2) - D(s+3),
-// which is LSMLIB's w1 p1 + w2 p2 + w3 p3 rearranged (the weights sum to 1).
+// which is LSMLIB's w1 p1 + w2 p2 + w3 p3 rearranged (the weights sum to 1),
+// carried doubled.
 // Differences are not divided by dx: WENO5 is homogeneous of degree one in
 // them, so the reconstructed derivatives are scaled once at the end.
 //
@@ -63,22 +64,20 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 //   first triple of a window:  13/3 t^2 + (d0 - 4 d1 + 3 d2)^2
 //   middle triple:             13/3 t^2 + (d0 - d2)^2
 //   last triple:               13/3 t^2 + (3 d0 - 4 d1 + d2)^2
-// (spatial_derivatives3d.f.in:1306-1311; the outer ones are the middle form
-// plus 4 t^2 -/+ 4 t (d0 - d2)).
+// (spatial_derivatives3d.f.in:1306-1311), with d0 - 4 d1 + 3 d2 =
+// 2 t + (d2 - d0) and 3 d0 - 4 d1 + d2 = 2 t - (d2 - d0).
 struct Tri {
   float2 t, s1, s2, s3;
 };
 __device__ __forceinline__ Tri tri_forms(float2 d0, float2 d1, float2 d2) {
   Tri r;
   r.t = fma2(sp(-2.f), d1, add2(d0, d2));
-  const float2 nb = sub2(d2, d0);  // -(d0 - d2)
-  const float2 tt = mul2(sp(13.f / 3.f), r.t);
-  r.s2 = fma2(tt, r.t, mul2(nb, nb));
-  const float2 t4 = mul2(sp(4.f), r.t);
-  const float2 x = fma2(t4, r.t, r.s2);
-  const float2 y = mul2(t4, nb);  // -4 t (d0 - d2)
-  r.s1 = add2(x, y);
-  r.s3 = sub2(x, y);
+  const float2 b = sub2(d2, d0);
+  const float2 T = mul2(mul2(sp(13.f / 3.f), r.t), r.t);
+  const float2 u = fma2(sp(2.f), r.t, b), w = fma2(sp(-2.f), r.t, b);
+  r.s1 = fma2(u, u, T);
+  r.s2 = fma2(b, b, T);
+  r.s3 = fma2(w, w, T);
   return r;
 }
 
@@ -97,38 +96,38 @@ __device__ __forceinline__ WQ window_q(float2 s1, float2 s2, float2 s3, float2 m
   return {mul2(a, a), mul2(b, b), mul2(c, c)};
 }
 
-// minus(c) of window W(c):  p2 + (2 q23 TD(c-2) + 3 q12 TD(c-1)) / (6 (q23 + 6 q13 + 3 q12))
-__device__ __forceinline__ float2 side_minus(const WQ &w, float2 tda, float2 tdb, float2 p2) {
-  const float2 num = fma2(sp(2.f), mul2(w.q23, tda), mul2(sp(3.f), mul2(w.q12, tdb)));
-  const float2 den = fma2(sp(6.f), w.q23, fma2(sp(36.f), w.q13, mul2(sp(18.f), w.q12)));
+// The sides are kept doubled (the factor goes into the 1/dx^2 of |grad phi|^2):
+// with the central candidate 2 p2 = D(c) + D(c+1) - t(c-1) / 3 (minus) or
+// D(c-1) + D(c) - t(c-1) / 3 (plus), A = q23, B = q12, C = q13,
+//   2 minus(c)  = 2 p2 + (A TD(c-2) + 3/2 B TD(c-1)) / (3/2 A + 9 C + 9/2 B)
+//   2 plus(c-1) = 2 p2 - (3/2 A TD(c-2) + B TD(c-1)) / (9/2 A + 9 C + 3/2 B)
+// `a` is TD(c-2), `nb` is -TD(c-1).
+__device__ __forceinline__ float2 side_minus(const WQ &w, float2 a, float2 nb, float2 p2) {
+  const float2 num = fma2(sp(-1.5f), mul2(w.q12, nb), mul2(w.q23, a));
+  const float2 den = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, mul2(sp(9.f), w.q13)));
   return fma2(num, rcp2(den), p2);
 }
-
-// both sides of one window W(c): minus(c) as above and
-// plus(c-1) = p2' - (2 q12 TD(c-1) + 3 q23 TD(c-2)) / (6 (q12 + 6 q13 + 3 q23))
-__device__ __forceinline__ void sides_both(const WQ &w, float2 tda, float2 tdb, float2 p2m, float2 p2p,
-                                           float2 &minus, float2 &plus) {
-  const float2 u = mul2(w.q23, tda), v = mul2(w.q12, tdb);
-  const float2 g = mul2(sp(36.f), w.q13);
-  const float2 num_m = fma2(sp(2.f), u, mul2(sp(3.f), v));
-  const float2 num_p = fma2(sp(3.f), u, mul2(sp(2.f), v));
-  const float2 den_m = fma2(sp(6.f), w.q23, fma2(sp(18.f), w.q12, g));
-  const float2 den_p = fma2(sp(6.f), w.q12, fma2(sp(18.f), w.q23, g));
-  minus = fma2(num_m, rcp2(den_m), p2m);
-  plus = fma2(sp(-1.f), mul2(num_p, rcp2(den_p)), p2p);
+__device__ __forceinline__ void sides_both(const WQ &w, float2 a, float2 nb, float2 p2m, float2 p2p, float2 &minus,
+                                           float2 &plus) {
+  const float2 u = mul2(w.q23, a), v = mul2(w.q12, nb);
+  const float2 g = mul2(sp(9.f), w.q13);
+  const float2 den_m = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, g));
+  const float2 den_p = fma2(sp(1.5f), w.q12, fma2(sp(4.5f), w.q23, g));
+  minus = fma2(fma2(sp(-1.5f), v, u), rcp2(den_m), p2m);
+  plus = fma2(fma2(sp(-1.5f), u, v), rcp2(den_p), p2p);
 }
 
-// minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
+// 2 minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
 __device__ __forceinline__ float2 minus_of_window(const float2 D[5], Tri *mid = nullptr, Tri *last = nullptr) {
   const Tri a0 = tri_forms(D[0], D[1], D[2]), a1 = tri_forms(D[1], D[2], D[3]), a2 = tri_forms(D[2], D[3], D[4]);
   float2 sq[5];
 #pragma unroll
   for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
   const WQ wq = window_q(a0.s1, a1.s2, a2.s3, max5(sq[0], sq[1], sq[2], sq[3], sq[4]));
-  const float2 p2m = fma2(sp(-1.f / 6.f), a1.t, mul2(sp(0.5f), add2(D[2], D[3])));
+  const float2 p2m = fma2(sp(-1.f / 3.f), a1.t, add2(D[2], D[3]));
   if (mid) *mid = a1;
   if (last) *last = a2;
-  return side_minus(wq, sub2(a0.t, a1.t), sub2(a1.t, a2.t), p2m);
+  return side_minus(wq, sub2(a0.t, a1.t), sub2(a2.t, a1.t), p2m);
 }
 
 // periodic images of a cell's new value in the 3 ghost layers (faces, edges,
@@ -236,7 +235,9 @@ static __global__ void __launch_bounds__(256, 3)
   auto ld2 = [&](int sz, int dx, int dy) {
     return *reinterpret_cast<const float2 *>(col + sz * st_z + dy * st_y + dx);
   };
-  const float2 iv2[3] = {sp(a.inv[0] * a.inv[0]), sp(a.inv[1] * a.inv[1]), sp(a.inv[2] * a.inv[2])};
+  // (a quarter of 1/dx^2: the sides are doubled)
+  const float2 iv2[3] = {sp(0.25f * a.inv[0] * a.inv[0]), sp(0.25f * a.inv[1] * a.inv[1]),
+                         sp(0.25f * a.inv[2] * a.inv[2])};
 
   // ---- z march warm-up: the carried state for cell z0 ---------------------
   float2 fz2, dz1, dz2, s1p, s1c, s2c, tk, tdk1, sumk, gmz, pb1, pb2, sqk1, sqk2;
@@ -299,11 +300,10 @@ static __global__ void __launch_bounds__(256, 3)
 #pragma unroll
       for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
       const WQ wq = window_q(b.s1, c.s2, d.s3, max5(sq[0], sq[1], sq[2], sq[3], sq[4]));
-      const float2 c6 = mul2(sp(-1.f / 6.f), c.t);               // t(j) / -6
-      const float2 p2m = fma2(sp(0.5f), add2(D[2], D[3]), c6);  // minus(j+1)
-      const float2 p2p = fma2(sp(0.5f), add2(D[1], D[2]), c6);  // plus(j)
+      const float2 p2m = fma2(sp(-1.f / 3.f), c.t, add2(D[2], D[3]));  // minus(j+1)
+      const float2 p2p = fma2(sp(-1.f / 3.f), c.t, add2(D[1], D[2]));  // plus(j)
       float2 mn;
-      sides_both(wq, sub2(b.t, c.t), sub2(c.t, d.t), p2m, p2p, mn, gpy);
+      sides_both(wq, sub2(b.t, c.t), sub2(d.t, c.t), p2m, p2p, mn, gpy);
       yx[tz & 1][w][lane] = mn;
     }
     // ---- z: window W(k+1) -> plus(k), minus(k+1) -----------------------------
@@ -319,9 +319,8 @@ static __global__ void __launch_bounds__(256, 3)
       const float2 m = make_float2(max3f(pb2.x, pbn.x, sq3.x), max3f(pb2.y, pbn.y, sq3.y));
       const WQ wq = window_q(s1p, s2c, n.s3, m);
       const float2 sumn = add2(dz1, dz2);  // D(k+1) + D(k+2)
-      const float2 c6 = mul2(sp(-1.f / 6.f), tk);
-      const float2 p2m = fma2(sp(0.5f), sumn, c6), p2p = fma2(sp(0.5f), sumk, c6);
-      sides_both(wq, tdk1, tdk, p2m, p2p, gmz, gpz);  // minus(k+1), plus(k)
+      const float2 p2m = fma2(sp(-1.f / 3.f), tk, sumn), p2p = fma2(sp(-1.f / 3.f), tk, sumk);
+      sides_both(wq, tdk1, sub2(n.t, tk), p2m, p2p, gmz, gpz);  // minus(k+1), plus(k)
       fz2 = f3;
       dz1 = dz2;
       dz2 = d3;
@@ -362,12 +361,10 @@ static __global__ void __launch_bounds__(256, 3)
       const float inner = fmaxf(max3f(q0.y, q2.x, q2.y), q4.x);             // sq(i .. i+3)
       const float2 m = make_float2(fmaxf(inner, q0.x), fmaxf(inner, q4.y));
       const WQ wq = window_q(As1, Bs2, C.s3, m);
-      const float2 tda = sub2(At, Bt), tdb = sub2(Bt, C.t);
-      const float2 c6 = mul2(sp(-1.f / 6.f), Bt);
-      const float2 p2m = fma2(sp(0.5f), add2(P2, P3), c6);  // cells i+1, i+2
-      const float2 p2p = fma2(sp(0.5f), add2(P1, P2), c6);  // cells i, i+1
+      const float2 p2m = fma2(sp(-1.f / 3.f), Bt, add2(P2, P3));  // cells i+1, i+2
+      const float2 p2p = fma2(sp(-1.f / 3.f), Bt, add2(P1, P2));  // cells i, i+1
       float2 mn;
-      sides_both(wq, tda, tdb, p2m, p2p, mn, gpx);
+      sides_both(wq, sub2(At, Bt), sub2(C.t, Bt), p2m, p2p, mn, gpx);
       float prev = __shfl_up_sync(0xffffffffu, mn.y, 1);
       if (lane == 0) prev = xedge[0][tz][w];
       gmx = make_float2(prev, mn.x);
