@@ -251,11 +251,12 @@ inline int stage_tz_f64(const Layout &L) {
 
 // Tile depth of the FP32 reinitialization stage (k_reinit_x2).  A grid of
 // fewer 8-plane tiles than SMs is a matter of one tile's latency, about 4 us
-// and 0.95 us per plane: 4 planes, or 2 where 4-plane tiles are fewer than SMs
-// too (37 x 33 x 41: 13.2 -> 7.6 us per stage; 64^3: 13.3 -> 8.8).  Larger
-// grids take 8 or 10 planes, whichever makes the busiest SM's tiles shorter
-// in all, a tile costing one plane beside its own (128^3: 29.5 us with 8, 27.4
-// with 10; 160 x 150 x 140: 44.7 and 48.0; 256^3: 157.6 and 155.6).
+// and 0.8 us per plane: 4 planes, or 2 where 4-plane tiles are fewer than SMs
+// too (37 x 33 x 41: 11.7 us per stage with 8, 7.1 with 2; 64^3: 11.7 and
+// 8.0).  Larger grids take 8 or 10 planes, whichever makes the busiest SM's
+// tiles shorter in all, a tile costing one plane beside its own (128^3: 25.0
+// us with 8, 23.5 with 10; 160 x 150 x 140: 37.7 and 40.8; 192^3: 63.0 and
+// 61.0).
 inline int reinit_tz(const Layout &L) {
   const long long cols = (long long)((L.nx + RX - 1) / RX) * ((L.ny + RY - 1) / RY);
   const int sms = sm_count();

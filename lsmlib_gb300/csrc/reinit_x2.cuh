@@ -276,6 +276,10 @@ static __global__ void __launch_bounds__(256, 3)
   float2 pc_next = pc_src ? *reinterpret_cast<const float2 *>(pc_src + cell0) : sp(0.f);
   float2 un_next = un_src ? *reinterpret_cast<const float2 *>(un_src + cell0) : sp(0.f);
 
+  // four planes per pass: the carried quantities then change names instead of
+  // registers (256^3: 145 us per stage in a rolled loop, 130 with four planes,
+  // 137 with eight)
+#pragma unroll 4
   for (int tz = 0; tz < kmax; tz++) {
     const int k = z0 + tz;
     const int sz = tz + 3;
