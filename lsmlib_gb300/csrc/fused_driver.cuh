@@ -10,6 +10,7 @@
 #pragma once
 
 #include "fused_stage.cuh"
+#include "adv_x2.cuh"
 #include "reinit_x2.cuh"
 #include "lsmgpu_common.cuh"
 #include "../../include/lsmgpu.h"
@@ -195,14 +196,6 @@ void launch_bc(R *buf, const Layout &L, int bc) {
   LSMGPU_LAUNCH(k_ghost_fill<R>, grd, blk, 0, buf, L, bc);
 }
 
-// The FP32 reinitialization stage runs the window-sharing kernel of
-// reinit_x2.cuh (64 x 8 cell tiles); every other form runs k_stage /
-// k_stage_f32 (32 x 8 x TZ tiles).
-template <class R, int MODE, bool EXACT>
-constexpr bool uses_reinit_x2() {
-  return !EXACT && sizeof(R) == 4 && MODE == REINIT;
-}
-
 // SM count of the current device
 inline int sm_count() {
   static int sms_of[64] = {};  // per device, read once
@@ -249,7 +242,7 @@ inline int stage_tz_f64(const Layout &L) {
   return 1;
 }
 
-// Tile depth of the FP32 reinitialization stage (k_reinit_x2).  A grid of
+// Tile depth of k_reinit_x2 and k_adv_x2 (figures: k_reinit_x2).  A grid of
 // fewer 8-plane tiles than SMs is a matter of one tile's latency, about 4 us
 // and 0.8 us per plane: 4 planes, or 2 where 4-plane tiles are fewer than SMs
 // too (37 x 33 x 41: 11.7 us per stage with 8, 7.1 with 2; 64^3: 11.7 and
@@ -266,12 +259,32 @@ inline int reinit_tz(const Layout &L) {
   return planes(10) < planes(8) ? 10 : 8;
 }
 
+// Which stage kernel a grid runs.  FP32 reinitialization: k_reinit_x2.  FP32
+// constant-velocity advection: k_adv_x2, which takes 0.69 of the time of the
+// cell-by-cell k_stage_f32 per covered cell (256^3: 98.6 and 143.9 us per
+// stage) but covers x in rows of 64 cells, not 32.  Where that covers more
+// cells (an odd number of 32-cell halves), k_stage_f32 runs
+//  * a single half (32 x 64 x 64: 5.5 us, 6.3 with k_adv_x2; 32 x 256 x 256:
+//    21.6 and 28.7), unless k_adv_x2 has at most a tile per SM, where its
+//    latency is the shorter one (32^3: 5.5 and 5.1);
+//  * up to one wave of its 4-plane tiles, five per SM (80^3: 9.3 and 12.2; 130
+//    x 64 x 64: 10.5 and 12.2; beyond it, 100^3: 17.8 and 14.5).
+// Both give the same bits.  Every other form runs k_stage or k_stage_f32.
+template <class R, int MODE, bool EXACT>
+bool uses_x2(const Layout &L) {
+  if constexpr (EXACT || sizeof(R) != 4 || MODE == ADV_FIELD) return false;
+  if constexpr (MODE == REINIT) return true;
+  const long long halves = (L.nx + 31) / 32, rows = (L.ny + RY - 1) / RY;
+  if (halves % 2 == 0 || (halves + 1) / 2 * rows * ((L.nz + 1) / 2) <= sm_count()) return true;
+  return halves > 1 && halves * rows * ((L.nz + 3) / 4) > 5LL * sm_count();
+}
+
 // Tensor map of a padded work buffer with the staged box of the stage kernel
 // launch_stage<R, MODE, EXACT> runs.
 template <class R, int MODE, bool EXACT>
 bool encode_stage_tmap(CUtensorMap *m, const R *p, const Layout &L) {
   const long long ex = (long long)L.nx + GX + 3, ey = (long long)L.ny + 2 * GY, ez = (long long)L.nz + 2 * GZ;
-  if constexpr (uses_reinit_x2<R, MODE, EXACT>())
+  if (uses_x2<R, MODE, EXACT>(L))
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, RSX, RSY, reinit_tz(L) + 6);
   if constexpr (!EXACT && sizeof(R) == 4)
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f32(L) + 6);
@@ -288,43 +301,47 @@ template <class R, int MODE, bool EXACT>
 static void launch_stage(const CUtensorMap &tm, const StageArgs<R> &a, bool prepare_only = false) {
   const Layout &L = a.L;
   static bool attr_set = false;
-  if constexpr (uses_reinit_x2<R, MODE, EXACT>()) {
+  auto want_smem = [](auto kern, size_t bytes) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  auto grid = [&](int tx, int ty, int tz) {
+    return dim3((unsigned)((L.nx + tx - 1) / tx), (unsigned)((L.ny + ty - 1) / ty), (unsigned)((L.nz + tz - 1) / tz));
+  };
+  constexpr size_t kPlane = (size_t)SX * SY * sizeof(R);
+  if constexpr (!EXACT && sizeof(R) == 4) {
+    // FP32 form: packed cell pairs, tile depth per grid
     if (!attr_set) {
-      cudaFuncSetAttribute(k_reinit_x2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)reinit_x2_smem(RZ_MAX));
+      if constexpr (MODE == REINIT)
+        for (auto k : {k_reinit_x2<false>, k_reinit_x2<true>}) want_smem(k, reinit_x2_smem(RZ_MAX));
+      if constexpr (MODE == ADV_CONST)
+        for (int q = 0; q < 8; q++) {
+          const float v[3] = {q & 1 ? -1.f : 1.f, q & 2 ? -1.f : 1.f, q & 4 ? -1.f : 1.f};
+          want_smem(adv_x2_kernel(v), reinit_x2_smem(RZ_MAX));
+        }
+      if constexpr (MODE != REINIT) {
+        want_smem(k_stage_f32<MODE, 8>, kPlane * 14);
+        want_smem(k_stage_f32<MODE, 4>, kPlane * 10);
+      }
       attr_set = true;
     }
     if (prepare_only) return;
-    const int tz = reinit_tz(L);
-    dim3 grd((unsigned)((L.nx + RX - 1) / RX), (unsigned)((L.ny + RY - 1) / RY), (unsigned)((L.nz + tz - 1) / tz));
-    k_reinit_x2<<<grd, dim3(32, RY), reinit_x2_smem(tz), stream()>>>(tm, a, tz);
-    note_launch();
-    return;
-  }
-  dim3 blk(TX, TY);
-  if (!attr_set) {
-    if constexpr (!EXACT && sizeof(R) == 4) {
-      cudaFuncSetAttribute(k_stage_f32<MODE, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)((size_t)SX * SY * 14 * sizeof(float)));
-      cudaFuncSetAttribute(k_stage_f32<MODE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)((size_t)SX * SY * 10 * sizeof(float)));
-    } else {
-      cudaFuncSetAttribute(k_stage<R, MODE, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)((size_t)SX * SY * SZ * sizeof(R)));
+    if (uses_x2<R, MODE, EXACT>(L)) {
+      StageX2 kern = nullptr;
+      if constexpr (MODE == REINIT) kern = a.periodic ? k_reinit_x2<true> : k_reinit_x2<false>;
+      if constexpr (MODE == ADV_CONST) kern = adv_x2_kernel(a.vconst);
+      const int tz = reinit_tz(L);
+      kern<<<grid(RX, RY, tz), dim3(32, RY), reinit_x2_smem(tz), stream()>>>(tm, a, tz);
+    } else if constexpr (MODE != REINIT) {
+      const int tz = stage_tz_f32(L);
+      const auto kern = tz == 4 ? k_stage_f32<MODE, 4> : k_stage_f32<MODE, 8>;
+      kern<<<grid(TX, TY, tz), dim3(TX, TY), kPlane * (tz + 6), stream()>>>(tm, a);
     }
-    attr_set = true;
-  }
-  if (prepare_only) return;
-  if constexpr (!EXACT && sizeof(R) == 4) {
-    // FP32 form: the packed cell-pair kernel, tile depth per grid
-    const int tz = stage_tz_f32(L);
-    dim3 grd((unsigned)((L.nx + TX - 1) / TX), (unsigned)((L.ny + TY - 1) / TY), (unsigned)((L.nz + tz - 1) / tz));
-    const size_t smem = (size_t)SX * SY * (tz + 6) * sizeof(float);
-    if (tz == 4) k_stage_f32<MODE, 4><<<grd, blk, smem, stream()>>>(tm, a);
-    else k_stage_f32<MODE, 8><<<grd, blk, smem, stream()>>>(tm, a);
   } else {
+    if (!attr_set) want_smem(k_stage<R, MODE, EXACT>, kPlane * SZ);
+    attr_set = true;
+    if (prepare_only) return;
     const int tz = stage_tz_f64(L);
-    dim3 grd((unsigned)((L.nx + TX - 1) / TX), (unsigned)((L.ny + TY - 1) / TY), (unsigned)((L.nz + tz - 1) / tz));
-    k_stage<R, MODE, EXACT><<<grd, blk, (size_t)SX * SY * (tz + 6) * sizeof(R), stream()>>>(tm, a, tz);
+    k_stage<R, MODE, EXACT><<<grid(TX, TY, tz), dim3(TX, TY), kPlane * (tz + 6), stream()>>>(tm, a, tz);
   }
   note_launch();
 }

@@ -376,41 +376,122 @@ __device__ __forceinline__ float2 weno5_x2(float2 v1, float2 v2, float2 v3, floa
   return quot2(num, den);
 }
 
-// The backward WENO5 value of two cells from phi(c-3 .. c+2), in units of
-// phi (WENO5 is homogeneous of degree one: the caller scales by 1/dx once),
-// as the central candidate plus weighted third differences,
-//   p2 + w1 (p1 - p2) + w3 (p3 - p2),  p1 - p2 = TD(c-2) / 3,
-//   p3 - p2 = TD(c-1) / 6,  TD(s) = t(s) - t(s+1)
-// (the weights sum to 1): 53 packed operations where weno5_x2 with its scaled
-// differences takes 66.  Weights as in reinit_x2.cuh: q_k = S_k / eps + 1;
-// `floor4` is 4 times LSMLIB's floor of epsilon in these units (eps_floor4).
-__device__ __forceinline__ float2 weno5_backward_x2(const float2 x[6], float floor4) {
-  float2 D[5], sq[5];
-#pragma unroll
-  for (int q = 0; q < 5; q++) {
-    D[q] = sub2(x[q + 1], x[q]);
-    sq[q] = mul2(D[q], D[q]);
-  }
-  const float2 s = rcp2(fma2(sp(4e-6f), max5(sq[0], sq[1], sq[2], sq[3], sq[4]), sp(floor4)));  // 1 / (4 eps)
-  // second differences, and the outer parts u of the indicators:
-  // D1 - 4 D2 + 3 D3 = 2 t1 + (D3 - D1), 3 D3 - 4 D4 + D5 = 2 t3 + (D3 - D5)
-  const float2 t1 = fma2(sp(-2.f), D[1], add2(D[0], D[2]));
-  const float2 t2 = fma2(sp(-2.f), D[2], add2(D[1], D[3]));
-  const float2 t3 = fma2(sp(-2.f), D[3], add2(D[2], D[4]));
-  const float2 u1 = fma2(sp(2.f), t1, sub2(D[2], D[0]));
-  const float2 u2 = sub2(D[1], D[3]);
-  const float2 u3 = fma2(sp(2.f), t3, sub2(D[2], D[4]));
-  const float c133 = 13.f / 3.f;
-  const float2 q1 = fma2(fma2(mul2(sp(c133), t1), t1, mul2(u1, u1)), s, sp(1.f));
-  const float2 q2 = fma2(fma2(mul2(sp(c133), t2), t2, mul2(u2, u2)), s, sp(1.f));
-  const float2 q3 = fma2(fma2(mul2(sp(c133), t3), t3, mul2(u3, u3)), s, sp(1.f));
-  const float2 q23 = mul2(q2, q3), q13 = mul2(q1, q3), q12 = mul2(q1, q2);
-  const float2 A = mul2(q23, q23), B = mul2(q13, q13), C = mul2(q12, q12);  // < 3e30
-  // w1 = A / n, w3 = 3 C / n, n = A + 6 B + 3 C
-  const float2 num = fma2(sp(1.5f), mul2(C, sub2(t2, t3)), mul2(A, sub2(t1, t2)));
-  const float2 den = fma2(sp(3.f), A, fma2(sp(18.f), B, mul2(sp(9.f), C)));
-  const float2 p2 = fma2(sp(-1.f / 6.f), t2, mul2(sp(0.5f), add2(D[2], D[3])));
+// A triple of consecutive differences (d0, d1, d2): its second difference t
+// and the three smoothness-indicator forms it takes in a window, times 4:
+//   first triple of a window:  13/3 t^2 + (d0 - 4 d1 + 3 d2)^2
+//   middle triple:             13/3 t^2 + (d0 - d2)^2
+//   last triple:               13/3 t^2 + (3 d0 - 4 d1 + d2)^2
+// (spatial_derivatives3d.f.in:1306-1311), with d0 - 4 d1 + 3 d2 =
+// 2 t + (d2 - d0) and 3 d0 - 4 d1 + d2 = 2 t - (d2 - d0).
+struct Tri {
+  float2 t, s1, s2, s3;
+};
+__device__ __forceinline__ Tri tri_forms(float2 d0, float2 d1, float2 d2) {
+  Tri r;
+  r.t = fma2(sp(-2.f), d1, add2(d0, d2));
+  const float2 b = sub2(d2, d0);
+  const float2 T = mul2(mul2(sp(13.f / 3.f), r.t), r.t);
+  const float2 u = fma2(sp(2.f), r.t, b), w = fma2(sp(-2.f), r.t, b);
+  r.s1 = fma2(u, u, T);
+  r.s2 = fma2(b, b, T);
+  r.s3 = fma2(w, w, T);
+  return r;
+}
+
+// Weight products of a window from its three indicator forms (x4) and the
+// maximum squared difference m: q_k = 4 S_k / (4 eps) + 1 = (S_k + eps) / eps,
+// eps = 1e-6 m + 1e-36 (LSMLIB's, spatial_derivatives3d.f.in:1296, in units
+// of the unscaled differences, or with the floor scaled to them, floor4 / 4);
+// only ratios of the q_k enter the weights.
+// 1 <= q_k < 4e7, so the squared products stay below 3e30.
+struct WQ {
+  float2 q23, q13, q12;  // (q2 q3)^2, (q1 q3)^2, (q1 q2)^2
+};
+__device__ __forceinline__ WQ window_q(float2 s1, float2 s2, float2 s3, float2 m, float floor4 = 4e-36f) {
+  const float2 s = rcp2(fma2(sp(4e-6f), m, sp(floor4)));  // 1 / (4 eps), finite: floor4 is a normal number
+  const float2 q1 = fma2(s1, s, sp(1.f)), q2 = fma2(s2, s, sp(1.f)), q3 = fma2(s3, s, sp(1.f));
+  const float2 a = mul2(q2, q3), b = mul2(q1, q3), c = mul2(q1, q2);
+  return {mul2(a, a), mul2(b, b), mul2(c, c)};
+}
+
+// The sides are kept doubled (the factor goes into the 1/dx^2 of |grad phi|^2):
+// with the central candidate 2 p2 = D(c) + D(c+1) - t(c-1) / 3 (minus) or
+// D(c-1) + D(c) - t(c-1) / 3 (plus), A = q23, B = q12, C = q13,
+//   2 minus(c)  = 2 p2 + (A TD(c-2) + 3/2 B TD(c-1)) / (3/2 A + 9 C + 9/2 B)
+//   2 plus(c-1) = 2 p2 - (3/2 A TD(c-2) + B TD(c-1)) / (9/2 A + 9 C + 3/2 B)
+// `a` is TD(c-2), `nb` is -TD(c-1).
+__device__ __forceinline__ float2 side_minus(const WQ &w, float2 a, float2 nb, float2 p2) {
+  const float2 num = fma2(sp(-1.5f), mul2(w.q12, nb), mul2(w.q23, a));
+  const float2 den = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, mul2(sp(9.f), w.q13)));
   return fma2(num, rcp2(den), p2);
+}
+__device__ __forceinline__ void sides_both(const WQ &w, float2 a, float2 nb, float2 p2m, float2 p2p, float2 &minus,
+                                           float2 &plus) {
+  const float2 u = mul2(w.q23, a), v = mul2(w.q12, nb);
+  const float2 g = mul2(sp(9.f), w.q13);
+  const float2 den_m = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, g));
+  const float2 den_p = fma2(sp(1.5f), w.q12, fma2(sp(4.5f), w.q23, g));
+  minus = fma2(fma2(sp(-1.5f), v, u), rcp2(den_m), p2m);
+  plus = fma2(fma2(sp(-1.5f), u, v), rcp2(den_p), p2p);
+}
+
+// 2 minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
+__device__ __forceinline__ float2 minus_of_window(const float2 D[5], float floor4 = 4e-36f, Tri *mid = nullptr,
+                                                  Tri *last = nullptr) {
+  const Tri a0 = tri_forms(D[0], D[1], D[2]), a1 = tri_forms(D[1], D[2], D[3]), a2 = tri_forms(D[2], D[3], D[4]);
+  float2 sq[5];
+#pragma unroll
+  for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
+  const WQ wq = window_q(a0.s1, a1.s2, a2.s3, max5(sq[0], sq[1], sq[2], sq[3], sq[4]), floor4);
+  const float2 p2m = fma2(sp(-1.f / 3.f), a1.t, add2(D[2], D[3]));
+  if (mid) *mid = a1;
+  if (last) *last = a2;
+  return side_minus(wq, sub2(a0.t, a1.t), sub2(a2.t, a1.t), p2m);
+}
+
+// Periodic images of a cell's new value in the 3 ghost layers along y and z
+// (and their x images), for a cell within 3 of a y or z face; its image along
+// x alone is written by the caller.  dx, dy, dz: the element offsets of the
+// cell's image along each axis (0: none).  Not inlined: the stage loop then
+// keeps none of its index arithmetic.
+static __device__ __noinline__ void write_yz_images(float *c, int dx, long long dy, long long dz, float val) {
+  if (dy) c[dy] = val;
+  if (dz) c[dz] = val;
+  if (dx && dy) c[dx + dy] = val;
+  if (dx && dz) c[dx + dz] = val;
+  if (dy && dz) c[dy + dz] = val;
+  if (dx && dy && dz) c[dx + dy + dz] = val;
+}
+// index offset of the periodic image of index i of n (0: none)
+__device__ __forceinline__ int image_of(int i, int n) { return i < 3 ? n : (i >= n - 3 ? -n : 0); }
+
+// Stores the pair (u.x, u.y) of a row at out + cell (the second cell where
+// `two`), with its periodic images: those along x are two predicated stores
+// (px0, px1: image_of of both cells; every row of a tile column at an x face
+// has such cells), the others concern whole rows and planes (j and k are the
+// warp's).
+__device__ __forceinline__ void store_pair(float *out, const Layout &L, long long cell, float2 u, bool two, int px0,
+                                           int px1, int py, int pz) {
+  float *c = out + cell;
+  if (two) *reinterpret_cast<float2 *>(c) = u;
+  else c[0] = u.x;
+  if (px0) c[px0] = u.x;
+  if (px1) c[1 + px1] = u.y;
+  if ((py | pz) != 0) {
+    const long long dy = L.py * py, dz = L.pz * pz;
+    write_yz_images(c, px0, dy, dz, u.x);
+    if (two) write_yz_images(c + 1, px1, dy, dz, u.y);
+  }
+}
+
+// 2 minus(c) of two cells from phi(c-3 .. c+2), in units of phi (WENO5 is
+// homogeneous of degree one: the caller scales by 1/(2 dx) once); 51 packed
+// operations where weno5_x2 with its scaled differences takes 66.
+__device__ __forceinline__ float2 weno5_backward_x2(const float2 x[6], float floor4) {
+  float2 D[5];
+#pragma unroll
+  for (int q = 0; q < 5; q++) D[q] = sub2(x[q + 1], x[q]);
+  return minus_of_window(D, floor4);
 }
 
 // Both one-sided WENO5 values of one axis for two cells: minus side on
@@ -524,7 +605,7 @@ __device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<floa
 #pragma unroll
             for (int q = 0; q < 6; q++) x[q] = make_float2(c0[(3 - q) * st[d]], c1[(3 - q) * st[d]]);
           }
-          dot = fma2(sp(fabsf(v) * a.inv[d]), weno5_backward_x2(x, a.floor4[d]), dot);
+          dot = fma2(sp(0.5f * fabsf(v) * a.inv[d]), weno5_backward_x2(x, a.floor4[d]), dot);
         } else {
           // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
           // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);

@@ -59,97 +59,11 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return r;
 }
 
-// A triple of consecutive differences (d0, d1, d2): its second difference t
-// and the three smoothness-indicator forms it takes in a window, times 4:
-//   first triple of a window:  13/3 t^2 + (d0 - 4 d1 + 3 d2)^2
-//   middle triple:             13/3 t^2 + (d0 - d2)^2
-//   last triple:               13/3 t^2 + (3 d0 - 4 d1 + d2)^2
-// (spatial_derivatives3d.f.in:1306-1311), with d0 - 4 d1 + 3 d2 =
-// 2 t + (d2 - d0) and 3 d0 - 4 d1 + d2 = 2 t - (d2 - d0).
-struct Tri {
-  float2 t, s1, s2, s3;
-};
-__device__ __forceinline__ Tri tri_forms(float2 d0, float2 d1, float2 d2) {
-  Tri r;
-  r.t = fma2(sp(-2.f), d1, add2(d0, d2));
-  const float2 b = sub2(d2, d0);
-  const float2 T = mul2(mul2(sp(13.f / 3.f), r.t), r.t);
-  const float2 u = fma2(sp(2.f), r.t, b), w = fma2(sp(-2.f), r.t, b);
-  r.s1 = fma2(u, u, T);
-  r.s2 = fma2(b, b, T);
-  r.s3 = fma2(w, w, T);
-  return r;
-}
-
-// Weight products of a window from its three indicator forms (x4) and the
-// maximum squared difference m: q_k = 4 S_k / (4 eps) + 1 = (S_k + eps) / eps,
-// eps = 1e-6 m + 1e-36 (LSMLIB's, spatial_derivatives3d.f.in:1296, in units
-// of the unscaled differences); only ratios of the q_k enter the weights.
-// 1 <= q_k < 4e7, so the squared products stay below 3e30.
-struct WQ {
-  float2 q23, q13, q12;  // (q2 q3)^2, (q1 q3)^2, (q1 q2)^2
-};
-__device__ __forceinline__ WQ window_q(float2 s1, float2 s2, float2 s3, float2 m) {
-  const float2 s = rcp2(fma2(sp(4e-6f), m, sp(4e-36f)));  // 1 / (4 eps), finite: 4 eps >= 4e-36
-  const float2 q1 = fma2(s1, s, sp(1.f)), q2 = fma2(s2, s, sp(1.f)), q3 = fma2(s3, s, sp(1.f));
-  const float2 a = mul2(q2, q3), b = mul2(q1, q3), c = mul2(q1, q2);
-  return {mul2(a, a), mul2(b, b), mul2(c, c)};
-}
-
-// The sides are kept doubled (the factor goes into the 1/dx^2 of |grad phi|^2):
-// with the central candidate 2 p2 = D(c) + D(c+1) - t(c-1) / 3 (minus) or
-// D(c-1) + D(c) - t(c-1) / 3 (plus), A = q23, B = q12, C = q13,
-//   2 minus(c)  = 2 p2 + (A TD(c-2) + 3/2 B TD(c-1)) / (3/2 A + 9 C + 9/2 B)
-//   2 plus(c-1) = 2 p2 - (3/2 A TD(c-2) + B TD(c-1)) / (9/2 A + 9 C + 3/2 B)
-// `a` is TD(c-2), `nb` is -TD(c-1).
-__device__ __forceinline__ float2 side_minus(const WQ &w, float2 a, float2 nb, float2 p2) {
-  const float2 num = fma2(sp(-1.5f), mul2(w.q12, nb), mul2(w.q23, a));
-  const float2 den = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, mul2(sp(9.f), w.q13)));
-  return fma2(num, rcp2(den), p2);
-}
-__device__ __forceinline__ void sides_both(const WQ &w, float2 a, float2 nb, float2 p2m, float2 p2p, float2 &minus,
-                                           float2 &plus) {
-  const float2 u = mul2(w.q23, a), v = mul2(w.q12, nb);
-  const float2 g = mul2(sp(9.f), w.q13);
-  const float2 den_m = fma2(sp(1.5f), w.q23, fma2(sp(4.5f), w.q12, g));
-  const float2 den_p = fma2(sp(1.5f), w.q12, fma2(sp(4.5f), w.q23, g));
-  minus = fma2(fma2(sp(-1.5f), v, u), rcp2(den_m), p2m);
-  plus = fma2(fma2(sp(-1.5f), u, v), rcp2(den_p), p2p);
-}
-
-// 2 minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
-__device__ __forceinline__ float2 minus_of_window(const float2 D[5], Tri *mid = nullptr, Tri *last = nullptr) {
-  const Tri a0 = tri_forms(D[0], D[1], D[2]), a1 = tri_forms(D[1], D[2], D[3]), a2 = tri_forms(D[2], D[3], D[4]);
-  float2 sq[5];
-#pragma unroll
-  for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
-  const WQ wq = window_q(a0.s1, a1.s2, a2.s3, max5(sq[0], sq[1], sq[2], sq[3], sq[4]));
-  const float2 p2m = fma2(sp(-1.f / 3.f), a1.t, add2(D[2], D[3]));
-  if (mid) *mid = a1;
-  if (last) *last = a2;
-  return side_minus(wq, sub2(a0.t, a1.t), sub2(a2.t, a1.t), p2m);
-}
-
-// periodic images of a cell's new value in the 3 ghost layers (faces, edges,
-// corners), written by the thread that computes the cell (not inlined: the
-// stage loop then keeps none of its index arithmetic when it is not used)
-static __device__ __noinline__ void write_periodic_images(float *out, const Layout &L, int i, int j, int k, float val) {
-  const int oi = i < 3 ? L.nx : (i >= L.nx - 3 ? -L.nx : 0);
-  const int oj = j < 3 ? L.ny : (j >= L.ny - 3 ? -L.ny : 0);
-  const int ok = k < 3 ? L.nz : (k >= L.nz - 3 ? -L.nz : 0);
-  if (!(oi | oj | ok)) return;
-  const long long c = L.idx(i, j, k), sx = oi, sy = L.py * oj, sz = L.pz * ok;
-  if (oi) out[c + sx] = val;
-  if (oj) out[c + sy] = val;
-  if (ok) out[c + sz] = val;
-  if (oi && oj) out[c + sx + sy] = val;
-  if (oi && ok) out[c + sx + sz] = val;
-  if (oj && ok) out[c + sy + sz] = val;
-  if (oi && oj && ok) out[c + sx + sy + sz] = val;
-}
-
-// (static: each translation unit including this header has its own instance,
+// (PERIODIC: the stage also writes the periodic images; an instance of its own
+// because that code in the other one costs it registers, 142 us per stage.
+// static: each translation unit including this header has its own instance,
 // as with the other stage kernels; 80 registers for three CTAs per SM)
+template <bool PERIODIC>
 static __global__ void __launch_bounds__(256, 3)
     k_reinit_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a, int tzn) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -198,7 +112,7 @@ static __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int q = 0; q < 5; q++) D[q] = sub2(p[q + 1], p[q]);
     Tri a1, a2;
-    const float2 mv = minus_of_window(D, &a1, &a2);  // a1 = tri(x0-1), a2 = tri(x0)
+    const float2 mv = minus_of_window(D, 4e-36f, &a1, &a2);  // a1 = tri(x0-1), a2 = tri(x0)
     const float2 v[6] = {mv, a1.s1, a2.s1, a2.s2, a1.t, a2.t};
 #pragma unroll
     for (int q = 0; q < 6; q++) {
@@ -229,6 +143,9 @@ static __global__ void __launch_bounds__(256, 3)
   const bool row_live = j < L.ny;
   const bool two = i + 1 < L.nx;
   const bool live = row_live && i < L.nx;
+  // offsets of the periodic images of the pair's cells along x and y
+  const int px0 = PERIODIC ? image_of(i, L.nx) : 0, px1 = PERIODIC && two ? image_of(i + 1, L.nx) : 0;
+  const int py = PERIODIC ? image_of(j, L.ny) : 0;
   const int sx = 2 * lane + 4, sy = w + 3;
   const int kmax = min(tzn, L.nz - z0);
   const float *col = tile + sy * st_y + sx;  // (i, j) column, plane index sz
@@ -249,7 +166,7 @@ static __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int q = 0; q < 5; q++) D[q] = sub2(p[q + 1], p[q]);
     Tri a1, a2;
-    gmz = minus_of_window(D, &a1, &a2);  // minus(z0); a1 = tri(z0-1), a2 = tri(z0)
+    gmz = minus_of_window(D, 4e-36f, &a1, &a2);  // minus(z0); a1 = tri(z0-1), a2 = tri(z0)
     float2 sq[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
@@ -276,10 +193,11 @@ static __global__ void __launch_bounds__(256, 3)
   float2 pc_next = pc_src ? *reinterpret_cast<const float2 *>(pc_src + cell0) : sp(0.f);
   float2 un_next = un_src ? *reinterpret_cast<const float2 *>(un_src + cell0) : sp(0.f);
 
-  // four planes per pass: the carried quantities then change names instead of
-  // registers (256^3: 145 us per stage in a rolled loop, 130 with four planes,
-  // 137 with eight)
-#pragma unroll 4
+  // several planes per pass: the carried quantities then change names instead
+  // of registers (256^3, us per stage, 3 / 4 / 5 / 8 planes: 141 / 136 / 134 /
+  // 133, with the periodic images 148 / 144 / 139 / 162; rolled: 145)
+  constexpr int kRun = PERIODIC ? 5 : 8;
+#pragma unroll kRun
   for (int tz = 0; tz < kmax; tz++) {
     const int k = z0 + tz;
     const int sz = tz + 3;
@@ -405,16 +323,12 @@ static __global__ void __launch_bounds__(256, 3)
       u = fma2(sp(1.f / 3.f), un, mul2(sp(2.f / 3.f), fma2(sp(a.dt), rhs, u0)));  // :490-492
     }
     if (live) {
-      if (two) {
+      if constexpr (PERIODIC) {
+        store_pair(a.out, L, cell, u, two, px0, px1, py, image_of(k, L.nz));
+      } else if (two) {
         *reinterpret_cast<float2 *>(a.out + cell) = u;
       } else {
         a.out[cell] = u.x;
-      }
-      // (the writer returns at once for a cell with no image; a boundary
-      // test here measured 5% slower stages, through the loop's code)
-      if (a.periodic) {
-        write_periodic_images(a.out, L, i, j, k, u.x);
-        if (two) write_periodic_images(a.out, L, i + 1, j, k, u.y);
       }
     }
   }

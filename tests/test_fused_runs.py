@@ -199,3 +199,27 @@ def test_fused_reinit_f32_tile_depths(n, bc, use0, gpu_lib):
         L.reinit_weno5_tvdrk3(t, gb, fb, dx, 0.5 * dx, 3, use_phi0_for_sgn=use0, bc=bc, precision=precision)
     L.check()
     assert float((t32.double() - t64)[3:-3, 3:-3, 3:-3].abs().max()) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(24, 23, 25), (37, 33, 41), (70, 40, 39), (130, 61, 50), (96, 101, 100), (128, 128, 41)])
+@pytest.mark.parametrize("v", [(0.3, -0.4, 0.5), (-0.3, 0.4, -0.5), (0.0, -0.6, 0.2), (-0.5, -0.3, -0.4),
+                               (0.5, 0.3, 0.4), (-0.2, 0.0, 0.6), (0.4, 0.5, -0.3), (0.4, -0.5, -0.3),
+                               (-0.6, -0.2, 0.0)])
+@pytest.mark.parametrize("bc", [L.BC_PERIODIC, L.BC_LINEAR])
+def test_fused_advect_f32_constant_velocity_signs(n, v, bc, gpu_lib):
+    """FP32 constant-velocity advection for every sign triple, at sizes whose
+    rows run as 64- and as 32-cell tiles, the last tile of each axis ragged,
+    against the FP64 form (which equals the oracle bit for bit)."""
+    import torch
+    fb = (0, n[0] - 1, 0, n[1] - 1, 0, n[2] - 1)
+    gb = tuple(q + (-3, 3)[s % 2] for s, q in enumerate(fb))
+    dx = 2.0 / max(n)
+    X, Y, Z = np.meshgrid(*[2 * np.pi * (np.arange(-3, m + 3) + 0.5) / m for m in n], indexing="ij")
+    phi = np.sin(X) * np.cos(Y) + 0.4 * np.cos(2 * Z + 0.3) * np.sin(Y)
+    t32 = torch.from_numpy(np.ascontiguousarray(phi.T)).cuda().float()
+    t64 = t32.double()
+    for t, precision in ((t32, "f32"), (t64, "f64")):
+        L.advect_weno5_tvdrk3(t, gb, fb, dx, 0.5 * dx, 3, vel_const=v, bc=bc, precision=precision)
+    L.check()
+    assert float((t32.double() - t64)[3:-3, 3:-3, 3:-3].abs().max()) <= 1e-5
