@@ -168,15 +168,13 @@ int lsmgpu_band_flow_weno5_tvdrk3_f32(float *phi, const int *gb, const int *fb, 
  * one array, grid g occupying (nx+6)(ny+6)(nz+6) values (3 ghost cells per
  * side, column-major) from phi + offsets[g]; dims holds (nx, ny, nz) per grid,
  * vel the constant velocity (u, v, w) per grid, spacing (dx, dy, dz) per grid
- * and dt one step per grid.  Each TVD-RK3 stage of all grids is one
- * persistent kernel launch pulling 32 x 8 x TZ tiles from a work counter; the
- * n_steps x 3 launches are captured in a CUDA graph.  TZ and the CTAs per SM
- * are picked by an autotuner on the first call for a batch shape.  Periodic
- * boundaries only (bc = LSMGPU_BC_PERIODIC).  flags: LSMGPU_BATCH_LOOP runs
- * one single-grid launch per grid per stage instead (for comparison),
- * LSMGPU_BATCH_NO_GRAPH launches without a graph, LSMGPU_BATCH_TZ(n) forces
- * tile depth n (4, 8 or 16) and skips the autotuner.  The result is the same
- * in every mode. */
+ * and dt one step per grid.  Each TVD-RK3 stage of all grids is one kernel
+ * launch over a table of their tiles; the n_steps x 3 launches are captured
+ * in a CUDA graph.  Periodic boundaries only (bc = LSMGPU_BC_PERIODIC).
+ * flags: LSMGPU_BATCH_LOOP runs one single-grid launch per grid per stage
+ * instead (for comparison), LSMGPU_BATCH_NO_GRAPH launches without a graph,
+ * LSMGPU_BATCH_TZ(n) sets the depth of the deepest tile (even, 8 at most; by
+ * the batch's size otherwise).  The result is the same in every mode. */
 #define LSMGPU_BATCH_LOOP 1
 #define LSMGPU_BATCH_NO_GRAPH 2
 #define LSMGPU_BATCH_TZ(n) ((n) << 8)

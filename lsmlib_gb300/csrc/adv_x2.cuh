@@ -1,25 +1,29 @@
-// FP32 constant-velocity advection stage on the x cell pairs and the z march
-// of reinit_x2.cuh.
+// FP32 constant-velocity advection on the x cell pairs and the z march of
+// reinit_x2.cuh: the stage kernel of single grids, and the tile routine that
+// the batched kernel (batched.cu) shares with it.
 //
-// The velocity's sign is the same for every cell, so of each window only one
-// side is needed: minus(c) of W(c) where the component is positive, plus(c) of
-// W(c+1) where it is negative.  The kernel is instantiated for the eight sign
-// triples (OX, OY, OZ: 1 where the component is negative, the window's offset
-// from the cell).  With one window per cell and axis there is nothing to hand
-// between rows, so the plane loop has no barrier:
-//  * z: the thread marches up its column and carries the last two triples'
+// The velocity's sign is the same for every cell of a grid, and the forward
+// value of a negative velocity is the backward one of the mirrored line,
+// negated, so v g = |v| g'.  The callers therefore lay the grid out mirrored
+// along each axis of negative velocity (flip bits of the copies into and out
+// of the work layout) and these kernels know one direction: v >= 0, the minus
+// side of one window per cell and axis.  Every rounding is symmetric, so the
+// bits are those of the unmirrored formulas.  With nothing to hand between
+// rows, the plane loop has no barrier:
+//  * z: the thread marches along its column and carries the last two triples'
 //    forms (one new triple per cell);
 //  * x: a thread owns two x-neighbouring cells as the lanes of the packed
 //    instructions and takes the forms of the two triples before its own from
-//    the previous lane (the first lane from a per-tile prologue);
+//    the previous lane (the first lane of a row from a per-tile prologue);
 //  * y: the row's three triples, evaluated in place.
-// Bound by FMA issue: about 130 packed operations per cell pair, where the
-// cell-by-cell tile (adv tile of fused_stage.cuh) takes 165 and as many again
-// in loads, selection and per-tile set-up.  The arithmetic is that tile's
-// (minus_of_window, and its mirror image for the plus side), operation for
-// operation, so both give the same bits.  Measured per stage, periodic, with
-// this kernel and before it: 37 x 33 x 41 5.3 and 5.8 us, 128^3 18.3 and 23.0,
-// 256^3 98.6 and 143.
+// Bound by the issue of FP32 and data-movement instructions (62% and 38% of
+// their pipes at 64% of the issue slots): about 130 packed operations per cell
+// pair, where a cell-by-cell tile took 165 and as many again in loads,
+// selection and set-up.  Measured us per periodic stage, the cell-by-cell tile
+// / one kernel per sign triple on 64 x 8 tiles / this kernel: 37 x 33 x 41 4.5
+// / 5.3 / 4.0, 128^3 21.2 / 18.3 / 17.2, 256^3 140 / 98.6 / 97.9, 32 x 256 x
+// 256 21.6 / 21.6 / 17.6.  (Signed strides for the two axes that need no
+// mirrored lanes: 128^3 18.7, 256^3 109.)
 #pragma once
 
 #include "reinit_x2.cuh"
@@ -27,103 +31,81 @@
 namespace lsmgpu {
 namespace fused {
 
-// 2 minus(c) (PLUS = 0) or 2 plus(c-1) (PLUS = 1) of window W(c): its weight
-// products, TD(c-2), -TD(c-1), t(c-1) and D(c-1), D(c), D(c+1)
-template <int PLUS>
-__device__ __forceinline__ float2 one_side(const WQ &w, float2 a, float2 nb, float2 t, float2 dm, float2 d0,
-                                           float2 dp) {
-  if constexpr (PLUS == 0) {
-    return side_minus(w, a, nb, fma2(sp(-1.f / 3.f), t, add2(d0, dp)));
-  } else {
-    const float2 num = fma2(sp(-1.5f), mul2(w.q23, a), mul2(w.q12, nb));
-    const float2 den = fma2(sp(1.5f), w.q12, fma2(sp(4.5f), w.q23, mul2(sp(9.f), w.q13)));
-    return fma2(num, rcp2(den), fma2(sp(-1.f / 3.f), t, add2(dm, d0)));
-  }
-}
+// the axes along which a grid of velocity v is laid out mirrored, bit d
+template <class R>
+inline int mirrored_axes(const R v[3]) { return (v[0] < 0 ? 1 : 0) | (v[1] < 0 ? 2 : 0) | (v[2] < 0 ? 4 : 0); }
 
-template <int OX, int OY, int OZ>
-static __global__ void __launch_bounds__(256, 3)
-    k_adv_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a, int tzn) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  float *tile = reinterpret_cast<float *>(smem_raw);
-  __shared__ __align__(8) uint64_t bar;
-  // per (plane, row): s1 and t of triple x0-2+OX, s1, s2 and t of x0-1+OX
-  __shared__ float xedge[5][RZ_MAX][RY];
-  const int lane = threadIdx.x, w = threadIdx.y;
-  const int tid = lane + 32 * w;
-  const int x0 = blockIdx.x * RX, y0 = blockIdx.y * RY, z0 = blockIdx.z * tzn;
+// a tile's rows are W cells wide; T threads, two cells each, cover a plane of it
+template <int W, int T>
+struct AdvTile {
+  static constexpr int LX = W / 2;        // threads of a row
+  static constexpr int ROWS = T / LX;     // rows
+  static constexpr int SXW = W + 8, SYW = ROWS + 6;  // staged plane
+  static constexpr size_t smem(int tz) { return (size_t)SXW * SYW * (tz + 6) * sizeof(float); }
+};
+
+// One tile of W x ROWS x tzn cells at (x0, y0, z0) whose haloed input is in
+// `tile`; `xedge`: 5 x DEPTH x ROWS floats of shared memory.  All T threads call
+// it (it has a barrier); tzn is even, at most DEPTH.
+template <int W, int T, int DEPTH, int UNROLL>
+__device__ __forceinline__ void adv_tile(const float *tile, float *xedge, const StageArgs<float> &a, int x0, int y0,
+                                         int z0, int tzn, int tid) {
+  using Q = AdvTile<W, T>;
   const Layout &L = a.L;
-
-  if (tid == 0) {
-    prefetch_tmap(&tm);
-    mbar_init(&bar, 1);
-    fence_barrier_init();
-  }
-  __syncthreads();
-  if (tid == 0) {
-    mbar_arrive_expect_tx(&bar, (uint32_t)reinit_x2_smem(tzn));
-    tma_load_3d(tile, &tm, x0 + GX - 4, y0 + GY - 3, z0 + GZ - 3, &bar);
-  }
-  if (!mbar_wait(&bar, 0, kMaxPolls)) {
-    if (tid == 0) atomicExch(a.err, LSMGPU_ERR_TIMEOUT);
-    mbar_wait(&bar, 0, kMaxPolls);  // let an in-flight copy land before exit
-    return;
-  }
-  if (a.ghost) {
-    fill_face_ghosts<float>(tile, RSX, RSY, tzn + 6, x0 - 4, y0 - 3, z0 - 3, L, a.ghost);
-    __syncthreads();
-  }
-
-  const int st_y = RSX, st_z = RSX * RSY;
-  // ---- prologue: the forms before the tile's first cell, two planes a thread --
-  if (tid < RY * tzn / 2) {
-    const int pw = tid % RY, pz = 2 * (tid / RY);
-    const float *r0 = tile + ((pz + 3) * RSY + pw + 3) * RSX, *r1 = r0 + st_z;
-    float2 p[5], D[4];  // phi(x0-3+OX ..), D(x0-2+OX ..)
+  constexpr int st_y = Q::SXW, st_z = Q::SXW * Q::SYW;
+  const int lx = tid % Q::LX;
+  // rows of 16 cells: a half-warp takes rows two apart, whose staged words lie
+  // in different banks (48 words apart; adjacent rows are 24 apart)
+  const int w = W == 16 ? ((tid >> 5) << 2) | ((tid >> 4) & 1) | ((tid >> 2) & 2) : tid / Q::LX;
+  constexpr int es = Q::ROWS * DEPTH;  // one quantity's part of xedge
+  // ---- prologue: per (plane, row) s1 and t of triple x0-2, s1, s2 and t of
+  // x0-1; two planes a thread
+  for (int e = tid; e < Q::ROWS * tzn / 2; e += T) {
+    const int pw = e % Q::ROWS, pz = 2 * (e / Q::ROWS);
+    const float *r0 = tile + (pz + 3) * st_z + (pw + 3) * st_y, *r1 = r0 + st_z;
+    float2 p[5], D[4];  // phi(x0-3 ..), D(x0-2 ..)
 #pragma unroll
-    for (int q = 0; q < 5; q++) p[q] = make_float2(r0[q + 1 + OX], r1[q + 1 + OX]);
+    for (int q = 0; q < 5; q++) p[q] = make_float2(r0[q + 1], r1[q + 1]);
 #pragma unroll
     for (int q = 0; q < 4; q++) D[q] = sub2(p[q + 1], p[q]);
     const Tri t2 = tri_forms(D[0], D[1], D[2]), t1 = tri_forms(D[1], D[2], D[3]);
     const float2 v[5] = {t2.s1, t2.t, t1.s1, t1.s2, t1.t};
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      xedge[q][pz][pw] = v[q].x;
-      xedge[q][pz + 1][pw] = v[q].y;
+      xedge[q * es + pz * Q::ROWS + pw] = v[q].x;
+      xedge[q * es + (pz + 1) * Q::ROWS + pw] = v[q].y;
     }
   }
   __syncthreads();
 
   // Rows and lanes outside the grid compute on tile padding and store nothing
   // (whole warps of such rows leave).
-  const int i = x0 + 2 * lane, j = y0 + w;
-  if (j >= L.ny) return;
+  const int i = x0 + 2 * lx, j = y0 + w;
+  if (!__any_sync(0xffffffffu, j < L.ny)) return;
+  const bool live = i < L.nx && j < L.ny;
   const bool two = i + 1 < L.nx;
-  const bool live = i < L.nx;
   // offsets of the periodic images of the pair's cells along x and y
   const int px0 = a.periodic ? image_of(i, L.nx) : 0, px1 = a.periodic && two ? image_of(i + 1, L.nx) : 0;
   const int py = a.periodic ? image_of(j, L.ny) : 0;
   const int kmax = min(tzn, L.nz - z0);
-  const float *col = tile + (w + 3) * st_y + 2 * lane + 4;  // (i, j) column, plane index sz
-  auto ld2 = [&](int sz, int dx, int dy) {
-    return *reinterpret_cast<const float2 *>(col + sz * st_z + dy * st_y + dx);
-  };
+  const float *col = tile + 3 * st_z + (w + 3) * st_y + 2 * lx + 4;  // cell (i, j) of the first plane
+  const float *edge = xedge + w;
+  auto ld2 = [](const float *p) { return *reinterpret_cast<const float2 *>(p); };
   // |v| / (2 dx) per axis; 0 where |v| is below the reference's zero tolerance
   float wv[3];
 #pragma unroll
-  for (int d = 0; d < 3; d++) wv[d] = fabsf(a.vconst[d]) < 1e-11f ? 0.f : 0.5f * fabsf(a.vconst[d]) * a.inv[d];
-  // the backward value of the line walked with the velocity's sign: -plus
-  auto add_axis = [&](float2 dot, int d, int neg, float2 g) {
-    const float2 r = fma2(sp(neg ? -wv[d] : wv[d]), g, dot);
+  for (int d = 0; d < 3; d++) wv[d] = a.vconst[d] < 1e-11f ? 0.f : 0.5f * a.vconst[d] * a.inv[d];
+  auto add_axis = [&](float2 dot, int d, float2 g) {
+    const float2 r = fma2(sp(wv[d]), g, dot);
     return wv[d] != 0.f ? r : dot;
   };
 
-  // ---- z march: the carried state for the window of cell z0, c = z0 + OZ ------
-  float2 fl, dm, d0, d1, s1a, s1b, s2b, ta, tb, pm2, pm1, sq0, sq1;
+  // ---- z march: the carried state for the window of the first cell c ----------
+  float2 fl, d0, d1, s1a, s1b, s2b, ta, tb, pm2, pm1, sq0, sq1;
   {
     float2 p[5], D[4], sq[4];  // phi(c-3 .. c+1), D(c-2 .. c+1)
 #pragma unroll
-    for (int q = 0; q < 5; q++) p[q] = ld2(q + OZ, 0, 0);
+    for (int q = 0; q < 5; q++) p[q] = ld2(col + (q - 3) * st_z);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       D[q] = sub2(p[q + 1], p[q]);
@@ -131,7 +113,6 @@ static __global__ void __launch_bounds__(256, 3)
     }
     const Tri t2 = tri_forms(D[0], D[1], D[2]), t1 = tri_forms(D[1], D[2], D[3]);
     fl = p[4];
-    dm = D[1];
     d0 = D[2];
     d1 = D[3];
     s1a = t2.s1;
@@ -146,79 +127,58 @@ static __global__ void __launch_bounds__(256, 3)
   }
 
   const float *un_src = a.stage == 1 ? nullptr : a.phi_n;
-  const long long cell0 = L.idx(live ? i : 0, j, z0);
-  float2 un_next = un_src ? *reinterpret_cast<const float2 *>(un_src + cell0) : sp(0.f);
+  long long cell = L.idx(live ? i : 0, live ? j : 0, z0);
+  float2 un_next = un_src ? ld2(un_src + cell) : sp(0.f);
 
-  // (unrolled: the carried quantities change names instead of registers; 256^3,
-  // 2 planes per pass 100.6 us per stage, 8 planes 98.6, 10 with two CTAs per SM
-  // 105.4)
-#pragma unroll 8
+  // (unrolled: the carried quantities change names instead of registers)
+#pragma unroll UNROLL
   for (int tz = 0; tz < kmax; tz++) {
-    const int k = z0 + tz;
-    const int sz = tz + 3;
-    const long long cell = cell0 + (long long)tz * L.pz;
     const float2 un = un_next;  // read one plane ahead of its use
-    if (tz + 1 < kmax && un_src) un_next = *reinterpret_cast<const float2 *>(un_src + cell + L.pz);
-    const float2 u0 = ld2(sz, 0, 0);  // phi(i), phi(i+1)
+    if (tz + 1 < kmax && un_src) un_next = ld2(un_src + cell + L.pz);
+    const float2 u0 = ld2(col);  // phi(i), phi(i+1)
     float2 gx, gy, gz;
-    // ---- x: windows W(c), W(c+1), c = i + OX ------------------------------------
+    // ---- x: windows W(i), W(i+1) ------------------------------------------------
     {
-      // P_s = (D(s), D(s+1)) for s = c-2 .. c+2
-      float2 P0, P1, P2, P3, P4;
-      if constexpr (OX == 1) {
-        const float2 e0 = ld2(sz, -2, 0), e2 = ld2(sz, 2, 0), e3 = ld2(sz, 4, 0);
-        const float2 o0 = make_float2(e0.y, u0.x), o1 = make_float2(u0.y, e2.x), o2 = make_float2(e2.y, e3.x);
-        P0 = sub2(o0, e0); P1 = sub2(u0, o0); P2 = sub2(o1, u0); P3 = sub2(e2, o1); P4 = sub2(o2, e2);
-      } else {
-        const float2 e0 = ld2(sz, -4, 0), e1 = ld2(sz, -2, 0), e3 = ld2(sz, 2, 0);
-        const float2 o0 = make_float2(e0.y, e1.x), o1 = make_float2(e1.y, u0.x), o2 = make_float2(u0.y, e3.x);
-        P0 = sub2(e1, o0); P1 = sub2(o1, e1); P2 = sub2(u0, o1); P3 = sub2(o2, u0); P4 = sub2(e3, o2);
-      }
-      const Tri C = tri_forms(P2, P3, P4);  // (tri(c), tri(c+1))
-      // (tri(c-2), tri(c-1)) are the previous lane's C
+      const float2 e0 = ld2(col - 4), e1 = ld2(col - 2), e3 = ld2(col + 2);
+      const float2 o0 = make_float2(e0.y, e1.x), o1 = make_float2(e1.y, u0.x), o2 = make_float2(u0.y, e3.x);
+      // P_s = (D(s), D(s+1)) for s = i-2 .. i+2
+      const float2 P0 = sub2(e1, o0), P2 = sub2(u0, o1), P3 = sub2(o2, u0), P4 = sub2(e3, o2);
+      const Tri C = tri_forms(P2, P3, P4);  // (tri(i), tri(i+1))
+      // (tri(i-2), tri(i-1)) are the previous lane's C
       float a_s1x = __shfl_up_sync(0xffffffffu, C.s1.x, 1), a_s1y = __shfl_up_sync(0xffffffffu, C.s1.y, 1);
       float a_s2y = __shfl_up_sync(0xffffffffu, C.s2.y, 1);
       float a_tx = __shfl_up_sync(0xffffffffu, C.t.x, 1), a_ty = __shfl_up_sync(0xffffffffu, C.t.y, 1);
-      if (lane == 0) {
-        a_s1x = xedge[0][tz][w];
-        a_tx = xedge[1][tz][w];
-        a_s1y = xedge[2][tz][w];
-        a_s2y = xedge[3][tz][w];
-        a_ty = xedge[4][tz][w];
+      if (lx == 0) {
+        a_s1x = edge[0];
+        a_tx = edge[es];
+        a_s1y = edge[2 * es];
+        a_s2y = edge[3 * es];
+        a_ty = edge[4 * es];
       }
       const float2 At = make_float2(a_tx, a_ty), Bt = make_float2(a_ty, C.t.x);
-      const float2 q0 = mul2(P0, P0), q2 = mul2(P2, P2), q4 = mul2(P4, P4);  // sq(c-2 .. c+3)
+      const float2 q0 = mul2(P0, P0), q2 = mul2(P2, P2), q4 = mul2(P4, P4);  // sq(i-2 .. i+3)
       const float inner = fmaxf(max3f(q0.y, q2.x, q2.y), q4.x);
       const float2 m = make_float2(fmaxf(inner, q0.x), fmaxf(inner, q4.y));
       const WQ wq = window_q(make_float2(a_s1x, a_s1y), make_float2(a_s2y, C.s2.x), C.s3, m, a.floor4[0]);
-      gx = one_side<OX>(wq, sub2(At, Bt), sub2(C.t, Bt), Bt, P1, P2, P3);
+      gx = side_minus(wq, sub2(At, Bt), sub2(C.t, Bt), fma2(sp(-1.f / 3.f), Bt, add2(P2, P3)));
     }
-    // ---- y: window W(c), c = j + OY ---------------------------------------------
+    // ---- y: window W(j) ---------------------------------------------------------
     {
-      float2 r[6], D[5];  // phi(c-3 .. c+2)
-#pragma unroll
-      for (int q = 0; q < 6; q++) r[q] = (q + OY == 3) ? u0 : ld2(sz, 0, q - 3 + OY);
-#pragma unroll
-      for (int q = 0; q < 5; q++) D[q] = sub2(r[q + 1], r[q]);
-      const Tri t2 = tri_forms(D[0], D[1], D[2]), t1 = tri_forms(D[1], D[2], D[3]), t0 = tri_forms(D[2], D[3], D[4]);
-      float2 sq[5];
-#pragma unroll
-      for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
-      const WQ wq = window_q(t2.s1, t1.s2, t0.s3, max5(sq[0], sq[1], sq[2], sq[3], sq[4]), a.floor4[1]);
-      gy = one_side<OY>(wq, sub2(t2.t, t1.t), sub2(t0.t, t1.t), t1.t, D[1], D[2], D[3]);
+      const float2 r[6] = {ld2(col - 3 * st_y), ld2(col - 2 * st_y), ld2(col - st_y), u0, ld2(col + st_y),
+                           ld2(col + 2 * st_y)};
+      gy = weno5_backward_x2(r, a.floor4[1]);
     }
-    // ---- z: window W(c), c = k + OZ ----------------------------------------------
+    // ---- z: window W(k), c = k ----------------------------------------------------
     {
-      const float2 f = ld2(sz + 2 + OZ, 0, 0);  // phi(c+2)
+      const float2 f = ld2(col + 2 * st_z);  // phi(c+2)
       const float2 d2 = sub2(f, fl);
       const float2 sq2 = mul2(d2, d2);
       const Tri n = tri_forms(d0, d1, d2);  // tri(c)
       const float2 pmn = make_float2(fmaxf(sq0.x, sq1.x), fmaxf(sq0.y, sq1.y));
       const float2 m = make_float2(max3f(pm2.x, pmn.x, sq2.x), max3f(pm2.y, pmn.y, sq2.y));
       const WQ wq = window_q(s1a, s2b, n.s3, m, a.floor4[2]);
-      gz = one_side<OZ>(wq, sub2(ta, tb), sub2(n.t, tb), tb, dm, d0, d1);
+      gz = side_minus(wq, sub2(ta, tb), sub2(n.t, tb), fma2(sp(-1.f / 3.f), tb, add2(d0, d1)));
       fl = f;
-      dm = d0;
       d0 = d1;
       d1 = d2;
       s1a = s1b;
@@ -231,22 +191,55 @@ static __global__ void __launch_bounds__(256, 3)
       sq0 = sq1;
       sq1 = sq2;
     }
-    const float2 dot = add_axis(add_axis(add_axis(sp(0.f), 0, OX, gx), 1, OY, gy), 2, OZ, gz);
+    const float2 dot = add_axis(add_axis(add_axis(sp(0.f), 0, gx), 1, gy), 2, gz);
     const float2 rhs = make_float2(-dot.x, -dot.y);
     float2 u = fma2(sp(a.dt), rhs, u0);  // tvd_runge_kutta3d.f:78
     if (a.stage == 2) u = fma2(sp(0.75f), un, mul2(sp(0.25f), u));                  // :403-404
     else if (a.stage == 3) u = fma2(sp(1.f / 3.f), un, mul2(sp(2.f / 3.f), u));  // :490-492
-    if (live) store_pair(a.out, L, cell, u, two, px0, px1, py, a.periodic ? image_of(k, L.nz) : 0);
+    if (live) store_pair(a.out, L, cell, u, two, px0, px1, py, a.periodic ? image_of(z0 + tz, L.nz) : 0);
+    col += st_z;
+    edge += Q::ROWS;
+    cell += L.pz;
   }
 }
 
-// the instance for a velocity's signs
-using StageX2 = void (*)(const CUtensorMap, StageArgs<float>, int);
-inline StageX2 adv_x2_kernel(const float v[3]) {
-  static const StageX2 k[8] = {k_adv_x2<0, 0, 0>, k_adv_x2<1, 0, 0>, k_adv_x2<0, 1, 0>, k_adv_x2<1, 1, 0>,
-                             k_adv_x2<0, 0, 1>, k_adv_x2<1, 0, 1>, k_adv_x2<0, 1, 1>, k_adv_x2<1, 1, 1>};
-  return k[(v[0] < 0.f ? 1 : 0) | (v[1] < 0.f ? 2 : 0) | (v[2] < 0.f ? 4 : 0)];
+// the stage kernel of a single grid: tiles of W x ROWS x tzn cells
+constexpr int kAdvThreads = 256;
+template <int W>
+static __global__ void __launch_bounds__(kAdvThreads, 3)
+    k_adv_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a, int tzn) {
+  using Q = AdvTile<W, kAdvThreads>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  float *tile = reinterpret_cast<float *>(smem_raw);
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ float xedge[5 * RZ_MAX * Q::ROWS];
+  const int tid = threadIdx.x + 32 * threadIdx.y;
+  const int x0 = blockIdx.x * W, y0 = blockIdx.y * Q::ROWS, z0 = blockIdx.z * tzn;
+  if (tid == 0) {
+    prefetch_tmap(&tm);
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (tid == 0) {
+    mbar_arrive_expect_tx(&bar, (uint32_t)Q::smem(tzn));
+    tma_load_3d(tile, &tm, x0 + GX - 4, y0 + GY - 3, z0 + GZ - 3, &bar);
+  }
+  if (!mbar_wait(&bar, 0, kMaxPolls)) {
+    if (tid == 0) atomicExch(a.err, LSMGPU_ERR_TIMEOUT);
+    mbar_wait(&bar, 0, kMaxPolls);  // let an in-flight copy land before exit
+    return;
+  }
+  if (a.ghost) {
+    fill_face_ghosts<float>(tile, Q::SXW, Q::SYW, tzn + 6, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
+    __syncthreads();
+  }
+  adv_tile<W, kAdvThreads, RZ_MAX, 8>(tile, xedge, a, x0, y0, z0, tzn, tid);
 }
+
+// the instance for a row length
+using StageX2 = void (*)(const CUtensorMap, StageArgs<float>, int);
+inline StageX2 adv_x2_kernel(int w) { return w == 64 ? k_adv_x2<64> : (w == 32 ? k_adv_x2<32> : k_adv_x2<16>); }
 
 }  // namespace fused
 }  // namespace lsmgpu

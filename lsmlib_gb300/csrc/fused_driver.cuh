@@ -28,19 +28,22 @@ namespace fused {
 constexpr int kPackZ = 8;
 
 // dst2 (optional) receives the same values (the phi0 copy of the
-// reinitialization's sign form)
+// reinitialization's sign form); bit d of `flip`: the layout is mirrored
+// along axis d
+__device__ __forceinline__ int maybe_mirrored(int i, int n, bool flip) { return flip ? n - 1 - i : i; }
 template <class R>
-__global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int jlo, int klo, R *dst2 = nullptr) {
+__global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int jlo, int klo, R *dst2 = nullptr,
+                       int flip = 0) {
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) - GX;
   const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y) - GY;
   const int k0 = (int)(blockIdx.z * kPackZ) - GZ;
   if (i > L.nx + 2 || j > L.ny + 2) return;
-  const int gi = i + ilo, gj = j + jlo;
+  const int gi = maybe_mirrored(i, L.nx, flip & 1) + ilo, gj = maybe_mirrored(j, L.ny, flip & 2) + jlo;
   const bool in_xy = gi >= gb.lo[0] && gi <= gb.hi[0] && gj >= gb.lo[1] && gj <= gb.hi[1];
   R v[kPackZ];
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
-    const int gk = k0 + q + klo;
+    const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
     v[q] = (in_xy && gk >= gb.lo[2] && gk <= gb.hi[2]) ? src(gi, gj, gk) : R(0);
   }
 #pragma unroll
@@ -53,12 +56,12 @@ __global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int
 }
 
 template <class R>
-__global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, int jlo, int klo) {
+__global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, int jlo, int klo, int flip = 0) {
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) - 3;
   const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y) - 3;
   const int k0 = (int)(blockIdx.z * kPackZ) - 3;
   if (i > L.nx + 2 || j > L.ny + 2) return;
-  const int gi = i + ilo, gj = j + jlo;
+  const int gi = maybe_mirrored(i, L.nx, flip & 1) + ilo, gj = maybe_mirrored(j, L.ny, flip & 2) + jlo;
   if (!(gi >= gb.lo[0] && gi <= gb.hi[0] && gj >= gb.lo[1] && gj <= gb.hi[1])) return;
   R v[kPackZ];
 #pragma unroll
@@ -66,7 +69,7 @@ __global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, i
     if (k0 + q <= L.nz + 2) v[q] = src[L.idx(i, j, k0 + q)];
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
-    const int gk = k0 + q + klo;
+    const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
     if (k0 + q <= L.nz + 2 && gk >= gb.lo[2] && gk <= gb.hi[2]) dst(gi, gj, gk) = v[q];
   }
 }
@@ -250,33 +253,41 @@ inline int stage_tz_f64(const Layout &L) {
 // tiles shorter in all, a tile costing one plane beside its own (128^3: 25.0
 // us with 8, 23.5 with 10; 160 x 150 x 140: 37.7 and 40.8; 192^3: 63.0 and
 // 61.0).
-inline int reinit_tz(const Layout &L) {
-  const long long cols = (long long)((L.nx + RX - 1) / RX) * ((L.ny + RY - 1) / RY);
+inline int x2_tz(long long cols, int nz) {
   const int sms = sm_count();
-  auto tiles = [&](int tz) { return cols * ((L.nz + tz - 1) / tz); };
+  auto tiles = [&](int tz) { return cols * ((nz + tz - 1) / tz); };
   if (tiles(8) < sms) return tiles(4) < sms ? 2 : 4;
   auto planes = [&](int tz) { return (tiles(tz) + sms - 1) / sms * (tz + 1); };
   return planes(10) < planes(8) ? 10 : 8;
 }
 
-// Which stage kernel a grid runs.  FP32 reinitialization: k_reinit_x2.  FP32
-// constant-velocity advection: k_adv_x2, which takes 0.69 of the time of the
-// cell-by-cell k_stage_f32 per covered cell (256^3: 98.6 and 143.9 us per
-// stage) but covers x in rows of 64 cells, not 32.  Where that covers more
-// cells (an odd number of 32-cell halves), k_stage_f32 runs
-//  * a single half (32 x 64 x 64: 5.5 us, 6.3 with k_adv_x2; 32 x 256 x 256:
-//    21.6 and 28.7), unless k_adv_x2 has at most a tile per SM, where its
-//    latency is the shorter one (32^3: 5.5 and 5.1);
-//  * up to one wave of its 4-plane tiles, five per SM (80^3: 9.3 and 12.2; 130
-//    x 64 x 64: 10.5 and 12.2; beyond it, 100^3: 17.8 and 14.5).
-// Both give the same bits.  Every other form runs k_stage or k_stage_f32.
+// The tiles of k_reinit_x2 (64 x 8 cells of a plane) and k_adv_x2.  The
+// latter's 512 cells are 64 x 8, 32 x 16 or 16 x 32, whichever covers the
+// fewest cells of the plane, the widest of equals (us per stage, 64 x 8 and
+// the rule's choice: 80^3 9.3 and 7.2, 130 x 64 x 64 10.5 and 7.3, 100^3 14.5
+// and 13.3).
+struct TileX2 {
+  int w, h, tz;
+  size_t smem() const { return (size_t)(w + 8) * (h + 6) * (tz + 6) * sizeof(float); }
+};
+template <int MODE>
+TileX2 tile_x2(const Layout &L) {
+  TileX2 t{0, 0, 0};
+  long long best = 0;
+  for (int w = RX; w >= (MODE == REINIT ? RX : 16); w /= 2) {
+    const int h = 512 / w;
+    const long long cols = (long long)((L.nx + w - 1) / w) * ((L.ny + h - 1) / h);
+    if (best == 0 || cols < best) t = TileX2{w, h, 0}, best = cols;
+  }
+  t.tz = x2_tz(best, L.nz);
+  return t;
+}
+
+// FP32 reinitialization and constant-velocity advection run k_reinit_x2 and
+// k_adv_x2; every other form runs k_stage or k_stage_f32.
 template <class R, int MODE, bool EXACT>
-bool uses_x2(const Layout &L) {
-  if constexpr (EXACT || sizeof(R) != 4 || MODE == ADV_FIELD) return false;
-  if constexpr (MODE == REINIT) return true;
-  const long long halves = (L.nx + 31) / 32, rows = (L.ny + RY - 1) / RY;
-  if (halves % 2 == 0 || (halves + 1) / 2 * rows * ((L.nz + 1) / 2) <= sm_count()) return true;
-  return halves > 1 && halves * rows * ((L.nz + 3) / 4) > 5LL * sm_count();
+constexpr bool uses_x2() {
+  return !EXACT && sizeof(R) == 4 && MODE != ADV_FIELD;
 }
 
 // Tensor map of a padded work buffer with the staged box of the stage kernel
@@ -284,8 +295,10 @@ bool uses_x2(const Layout &L) {
 template <class R, int MODE, bool EXACT>
 bool encode_stage_tmap(CUtensorMap *m, const R *p, const Layout &L) {
   const long long ex = (long long)L.nx + GX + 3, ey = (long long)L.ny + 2 * GY, ez = (long long)L.nz + 2 * GZ;
-  if (uses_x2<R, MODE, EXACT>(L))
-    return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, RSX, RSY, reinit_tz(L) + 6);
+  if constexpr (uses_x2<R, MODE, EXACT>()) {
+    const TileX2 t = tile_x2<MODE>(L);
+    return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, t.w + 8, t.h + 6, t.tz + 6);
+  }
   if constexpr (!EXACT && sizeof(R) == 4)
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f32(L) + 6);
   return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f64(L) + 6);
@@ -308,34 +321,31 @@ static void launch_stage(const CUtensorMap &tm, const StageArgs<R> &a, bool prep
     return dim3((unsigned)((L.nx + tx - 1) / tx), (unsigned)((L.ny + ty - 1) / ty), (unsigned)((L.nz + tz - 1) / tz));
   };
   constexpr size_t kPlane = (size_t)SX * SY * sizeof(R);
-  if constexpr (!EXACT && sizeof(R) == 4) {
-    // FP32 form: packed cell pairs, tile depth per grid
+  if constexpr (uses_x2<R, MODE, EXACT>()) {
     if (!attr_set) {
       if constexpr (MODE == REINIT)
         for (auto k : {k_reinit_x2<false>, k_reinit_x2<true>}) want_smem(k, reinit_x2_smem(RZ_MAX));
       if constexpr (MODE == ADV_CONST)
-        for (int q = 0; q < 8; q++) {
-          const float v[3] = {q & 1 ? -1.f : 1.f, q & 2 ? -1.f : 1.f, q & 4 ? -1.f : 1.f};
-          want_smem(adv_x2_kernel(v), reinit_x2_smem(RZ_MAX));
-        }
-      if constexpr (MODE != REINIT) {
-        want_smem(k_stage_f32<MODE, 8>, kPlane * 14);
-        want_smem(k_stage_f32<MODE, 4>, kPlane * 10);
-      }
+        for (int w = 16; w <= 64; w *= 2) want_smem(adv_x2_kernel(w), TileX2{w, 512 / w, RZ_MAX}.smem());
       attr_set = true;
     }
     if (prepare_only) return;
-    if (uses_x2<R, MODE, EXACT>(L)) {
-      StageX2 kern = nullptr;
-      if constexpr (MODE == REINIT) kern = a.periodic ? k_reinit_x2<true> : k_reinit_x2<false>;
-      if constexpr (MODE == ADV_CONST) kern = adv_x2_kernel(a.vconst);
-      const int tz = reinit_tz(L);
-      kern<<<grid(RX, RY, tz), dim3(32, RY), reinit_x2_smem(tz), stream()>>>(tm, a, tz);
-    } else if constexpr (MODE != REINIT) {
-      const int tz = stage_tz_f32(L);
-      const auto kern = tz == 4 ? k_stage_f32<MODE, 4> : k_stage_f32<MODE, 8>;
-      kern<<<grid(TX, TY, tz), dim3(TX, TY), kPlane * (tz + 6), stream()>>>(tm, a);
+    const TileX2 t = tile_x2<MODE>(L);
+    StageX2 kern = nullptr;
+    if constexpr (MODE == REINIT) kern = a.periodic ? k_reinit_x2<true> : k_reinit_x2<false>;
+    if constexpr (MODE == ADV_CONST) kern = adv_x2_kernel(t.w);
+    kern<<<grid(t.w, t.h, t.tz), dim3(32, 8), t.smem(), stream()>>>(tm, a, t.tz);
+  } else if constexpr (!EXACT && sizeof(R) == 4) {
+    // packed cell pairs, tile depth per grid
+    if (!attr_set) {
+      want_smem(k_stage_f32<8>, kPlane * 14);
+      want_smem(k_stage_f32<4>, kPlane * 10);
+      attr_set = true;
     }
+    if (prepare_only) return;
+    const int tz = stage_tz_f32(L);
+    const auto kern = tz == 4 ? k_stage_f32<4> : k_stage_f32<8>;
+    kern<<<grid(TX, TY, tz), dim3(TX, TY), kPlane * (tz + 6), stream()>>>(tm, a);
   } else {
     if (!attr_set) want_smem(k_stage<R, MODE, EXACT>, kPlane * SZ);
     attr_set = true;
@@ -354,7 +364,7 @@ void add_stage_args(GraphKey &key, const StageArgs<R> &a) {
   key.add(a.phi_n); key.add(a.phi0);
   for (int d = 0; d < 3; d++) key.add(a.vel[d]);
   key.add(a.out);
-  for (int d = 0; d < 3; d++) { key.add(a.vconst[d]); key.add(a.inv[d]); }
+  for (int d = 0; d < 3; d++) { key.add(a.vconst[d]); key.add(a.inv[d]); key.add(a.floor4[d]); }
   key.add(a.dt); key.add(a.dx_sq);
   key.add(a.stage); key.add(a.use0); key.add(a.periodic); key.add(a.ghost);
   key.add(a.err);
@@ -407,11 +417,14 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   // by the stage (periodic images) or computed by the next stage's loader
   cudaStream_t s = stream();
   cudaMemsetAsync(err, 0, sizeof(int), s);
+  // k_adv_x2 takes velocities that are not negative
+  const int flip = (!EXACT && sizeof(R) == 4 && rs.mode == ADV_CONST) ? mirrored_axes(rs.vconst) : 0;
   {
     const dim3 blk = pack_block(), grd = pack_grid(nx, ny, nz, GX);
     // the phi0 copy of the sign form (read at interior cells only) is
     // written by the same pass
-    LSMGPU_LAUNCH(k_pack<R>, grd, blk, 0, A, L, view((const R *)phi_d, gb), gb, fb.lo[0], fb.lo[1], fb.lo[2], P0);
+    LSMGPU_LAUNCH(k_pack<R>, grd, blk, 0, A, L, view((const R *)phi_d, gb), gb, fb.lo[0], fb.lo[1], fb.lo[2], P0,
+                  flip);
     if (rs.mode == ADV_FIELD)
       for (int d = 0; d < 3; d++)
         LSMGPU_LAUNCH(k_pack<R>, grd, blk, 0, V[d], L, view(vel_d[d], vb), vb, fb.lo[0], fb.lo[1], fb.lo[2]);
@@ -432,7 +445,7 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   a.L = L;
   a.phi0 = P0;
   for (int d = 0; d < 3; d++) a.vel[d] = V[d];
-  a.vconst[0] = (R)rs.vconst[0]; a.vconst[1] = (R)rs.vconst[1]; a.vconst[2] = (R)rs.vconst[2];
+  for (int d = 0; d < 3; d++) a.vconst[d] = (R)(flip >> d & 1 ? -rs.vconst[d] : rs.vconst[d]);
   a.inv[0] = R(1.0) / (R)rs.dx; a.inv[1] = R(1.0) / (R)rs.dy; a.inv[2] = R(1.0) / (R)rs.dz;
   const double d3[3] = {rs.dx, rs.dy, rs.dz};
   for (int d = 0; d < 3; d++) a.floor4[d] = (R)eps_floor4((float)d3[d]);
@@ -489,7 +502,7 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   if (!graph_replay(key, steps)) steps();
   {
     const dim3 blk = pack_block(), grd = pack_grid(nx, ny, nz, 3);
-    LSMGPU_LAUNCH(k_unpack<R>, grd, blk, 0, view(phi_d, gb), gb, A, L, fb.lo[0], fb.lo[1], fb.lo[2]);
+    LSMGPU_LAUNCH(k_unpack<R>, grd, blk, 0, view(phi_d, gb), gb, A, L, fb.lo[0], fb.lo[1], fb.lo[2], flip);
   }
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);

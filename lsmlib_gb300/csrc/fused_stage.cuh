@@ -552,82 +552,59 @@ __device__ __forceinline__ void weno5_pm_x2(const float2 D[6], float2 &gp, float
   gp = combine(q1p, q2p, q3p, P1p, B, A);
 }
 
-// Computes one TX_ x TY_ x TZ_ tile whose haloed input ((TX_ + 8) x (TY_ + 6)
-// x (TZ_ + 6)) is in `tile`, the calling thread at (tx, ty) of the tile;
-// shared by the single-grid kernel (32 x 8 tiles) and the batched persistent
-// kernel (32 x 8 or 16 x 16 tiles per grid, TZ_ from its autotuner).
-template <int MODE, int TZ_ = TZ, int TX_ = TX, int TY_ = TY>
-__device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<float> &a, int x0, int y0, int z0,
-                                         int tx, int ty) {
-  constexpr int SX_ = TX_ + 8, SY_ = TY_ + 6;
+// Computes one TX x TY x TZ_ tile of a field-velocity advection stage whose
+// haloed input ((TX + 8) x (TY + 6) x (TZ_ + 6)) is in `tile`, the calling
+// thread at (tx, ty) of the tile, two z-neighbouring cells at a time.
+template <int TZ_>
+__device__ __forceinline__ void adv_field_tile(const float *tile, const StageArgs<float> &a, int x0, int y0, int z0,
+                                               int tx, int ty) {
   const Layout &L = a.L;
   const int i = x0 + tx, j = y0 + ty;
   if (i >= L.nx || j >= L.ny) return;
   const int sx = tx + 4, sy = ty + 3;
   const int kmax = min(TZ_, L.nz - z0);
-  const int st[3] = {1, SX_, SX_ * SY_};
+  const int st[3] = {1, SX, SX * SY};
   const float2 inv[3] = {sp(a.inv[0]), sp(a.inv[1]), sp(a.inv[2])};
   // offsets of the column's periodic images along x and y (0: none)
-  const int oi = i < 3 ? L.nx : (i >= L.nx - 3 ? -L.nx : 0);
-  const int oj = j < 3 ? L.ny : (j >= L.ny - 3 ? -L.ny : 0);
+  const int oi = image_of(i, L.nx), oj = image_of(j, L.ny);
 
   for (int tz = 0; tz < kmax; tz += 2) {
     const bool two = tz + 1 < kmax;  // the second lane is a real cell
-    const float *c0 = tile + ((tz + 3) * SY_ + sy) * SX_ + sx;
-    const float *c1 = two ? c0 + SX_ * SY_ : c0;
+    const float *c0 = tile + ((tz + 3) * SY + sy) * SX + sx;
+    const float *c1 = two ? c0 + SX * SY : c0;
     const int k0 = z0 + tz, k1 = two ? k0 + 1 : k0;
     const long long cell0 = L.idx(i, j, k0), cell1 = L.idx(i, j, k1);
     float2 rhs;
     {
       float2 dot = sp(0.f);
       float vel0[3], vel1[3];
-      if constexpr (MODE == ADV_FIELD) {
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-          vel0[d] = a.vel[d][cell0];
-          vel1[d] = a.vel[d][cell1];
-        }
+      for (int d = 0; d < 3; d++) {
+        vel0[d] = a.vel[d][cell0];
+        vel1[d] = a.vel[d][cell1];
       }
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-        if constexpr (MODE == ADV_CONST) {
-          // one velocity for the whole grid: a uniform branch walks the axis
-          // with the velocity's sign; the forward stencil of a negative
-          // velocity is the backward one of the mirrored line, negated, so
-          // v g = |v| g'
-          const float v = a.vconst[d];
-          if (fabsf(v) < 1e-11f) continue;
-          float2 x[6];
-          if (v > 0.f) {
+        // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
+        // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);
+        // the six differences are loaded at fixed offsets and the lane's
+        // stencil is selected in registers
+        float2 a7[7], D[6];
 #pragma unroll
-            for (int q = 0; q < 6; q++) x[q] = make_float2(c0[(q - 3) * st[d]], c1[(q - 3) * st[d]]);
-          } else {
+        for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
 #pragma unroll
-            for (int q = 0; q < 6; q++) x[q] = make_float2(c0[(3 - q) * st[d]], c1[(3 - q) * st[d]]);
-          }
-          dot = fma2(sp(0.5f * fabsf(v) * a.inv[d]), weno5_backward_x2(x, a.floor4[d]), dot);
-        } else {
-          // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
-          // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);
-          // the six differences are loaded at fixed offsets and the lane's
-          // stencil is selected in registers
-          float2 a7[7], D[6];
+        for (int f = 0; f < 6; f++) D[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
+        const bool b0 = vel0[d] > 0.f, b1 = vel1[d] > 0.f;
+        float2 v[5];
 #pragma unroll
-          for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
-#pragma unroll
-          for (int f = 0; f < 6; f++) D[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
-          const bool b0 = vel0[d] > 0.f, b1 = vel1[d] > 0.f;
-          float2 v[5];
-#pragma unroll
-          for (int q = 0; q < 5; q++) {
-            v[q].x = b0 ? D[q].x : D[5 - q].x;
-            v[q].y = b1 ? D[q].y : D[5 - q].y;
-          }
-          float2 g = weno5_x2(v[0], v[1], v[2], v[3], v[4]);
-          if (fabsf(vel0[d]) < 1e-11f) g.x = 0.f;
-          if (fabsf(vel1[d]) < 1e-11f) g.y = 0.f;
-          dot = fma2(make_float2(vel0[d], vel1[d]), g, dot);
+        for (int q = 0; q < 5; q++) {
+          v[q].x = b0 ? D[q].x : D[5 - q].x;
+          v[q].y = b1 ? D[q].y : D[5 - q].y;
         }
+        float2 g = weno5_x2(v[0], v[1], v[2], v[3], v[4]);
+        if (fabsf(vel0[d]) < 1e-11f) g.x = 0.f;
+        if (fabsf(vel1[d]) < 1e-11f) g.y = 0.f;
+        dot = fma2(make_float2(vel0[d], vel1[d]), g, dot);
       }
       rhs = make_float2(-dot.x, -dot.y);
     }
@@ -670,7 +647,7 @@ __device__ __forceinline__ void f32_tile(const float *tile, const StageArgs<floa
 
 // 32 x 8 x TZ_ tiles; the steppers launch TZ_ = 8, or 4 where 4-plane tiles
 // fill the machine's waves better (fused_driver.cuh, stage_tz_f32)
-template <int MODE, int TZ_ = TZ>
+template <int TZ_>
 __global__ void __launch_bounds__(TX * TY) k_stage_f32(const __grid_constant__ CUtensorMap tm, StageArgs<float> a) {
   constexpr int SZ_ = TZ_ + 6;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -698,7 +675,7 @@ __global__ void __launch_bounds__(TX * TY) k_stage_f32(const __grid_constant__ C
     fill_face_ghosts<float>(tile, SX, SY, SZ_, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
     __syncthreads();
   }
-  f32_tile<MODE, TZ_>(tile, a, x0, y0, z0, tx, ty);
+  adv_field_tile<TZ_>(tile, a, x0, y0, z0, tx, ty);
 }
 
 }  // namespace fused

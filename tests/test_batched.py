@@ -72,3 +72,38 @@ def test_batch_fp32_against_fp64_oracle(gpu_lib):
                             float(dt[g]), 2, L.BC_PERIODIC, vel=v)
         got = buf[offsets[g]:offsets[g] + f.size].reshape(f.shape, order="F")
         assert np.max(np.abs(got[3:-3, 3:-3, 3:-3] - want[3:-3, 3:-3, 3:-3])) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flags", [0, L.batch_tz(2), L.batch_tz(8)])
+def test_batch_tile_shapes_and_velocity_signs(flags, gpu_lib):
+    """Grids at the edges of both tile shapes (32 x 8 and 16 x 16 cells) and of
+    the tile depths, every sign triple of the velocity, zero components among
+    them, against the FP64 stepper (equal to the oracle bit for bit)."""
+    import torch
+    sides = [(6, 6, 6), (16, 16, 8), (17, 16, 9), (32, 8, 10), (33, 9, 17), (48, 15, 16), (47, 17, 7), (64, 7, 25),
+             (65, 33, 6), (15, 65, 18), (96, 31, 33)]
+    signs = [(1, 1, 1), (-1, 1, 1), (1, -1, 1), (1, 1, -1), (-1, -1, 1), (-1, 1, -1), (1, -1, -1), (-1, -1, -1),
+             (0, -1, 1), (-1, 0, -1), (1, 1, 0)]
+    rng = np.random.default_rng(3)
+    dims = np.array(sides)
+    vel = np.array(signs) * rng.uniform(0.2, 1.0, size=(len(sides), 3))
+    spacing = 2.0 / dims
+    dt = 0.5 / (np.abs(vel) / spacing).sum(axis=1)
+    fields, offsets, off = [], [], 0
+    for g, n in enumerate(sides):
+        X, Y, Z = np.meshgrid(*[2 * np.pi * (np.arange(-3, m + 3) + 0.5) / m for m in n], indexing="ij")
+        f = np.asfortranarray((np.sin(X) * np.cos(Y) + 0.4 * np.cos(Z + 0.3 * g)).astype(np.float32))
+        fields.append(f)
+        offsets.append(off)
+        off += f.size
+    buf = pack(fields, np.array(offsets))
+    L.advect_batch_weno5_tvdrk3(buf, np.array(offsets), dims, vel, spacing, dt, 3, flags=flags)
+    for g, n in enumerate(sides):
+        gb = tuple(v for m in n for v in (-3, m + 2))
+        fb = tuple(v for m in n for v in (0, m - 1))
+        t = torch.from_numpy(np.ascontiguousarray(fields[g].astype(np.float64).T)).cuda()
+        L.advect_weno5_tvdrk3(t, gb, fb, float(spacing[g, 0]), float(dt[g]), 3, vel_const=tuple(map(float, vel[g])),
+                              bc=L.BC_PERIODIC, dy=float(spacing[g, 1]), dz=float(spacing[g, 2]))
+        got = buf[offsets[g]:offsets[g] + fields[g].size].reshape(fields[g].shape, order="F")
+        assert np.max(np.abs(got - t.cpu().numpy().T)) <= 1e-5, g
