@@ -41,6 +41,11 @@ struct AdvTile {
   static constexpr int LX = W / 2;        // threads of a row
   static constexpr int ROWS = T / LX;     // rows
   static constexpr int SXW = W + 8, SYW = ROWS + 6;  // staged plane
+  // a thread's row; rows of 16 cells: a half-warp takes rows two apart, whose
+  // staged words lie in different banks (48 words apart; adjacent rows are 24)
+  __device__ static __forceinline__ int row(int tid) {
+    return W == 16 ? ((tid >> 5) << 2) | ((tid >> 4) & 1) | ((tid >> 2) & 2) : tid / LX;
+  }
   static constexpr size_t smem(int tz) { return (size_t)SXW * SYW * (tz + 6) * sizeof(float); }
 };
 
@@ -54,9 +59,7 @@ __device__ __forceinline__ void adv_tile(const float *tile, float *xedge, const 
   const Layout &L = a.L;
   constexpr int st_y = Q::SXW, st_z = Q::SXW * Q::SYW;
   const int lx = tid % Q::LX;
-  // rows of 16 cells: a half-warp takes rows two apart, whose staged words lie
-  // in different banks (48 words apart; adjacent rows are 24 apart)
-  const int w = W == 16 ? ((tid >> 5) << 2) | ((tid >> 4) & 1) | ((tid >> 2) & 2) : tid / Q::LX;
+  const int w = Q::row(tid);
   constexpr int es = Q::ROWS * DEPTH;  // one quantity's part of xedge
   // ---- prologue: per (plane, row) s1 and t of triple x0-2, s1, s2 and t of
   // x0-1; two planes a thread
@@ -203,16 +206,122 @@ __device__ __forceinline__ void adv_tile(const float *tile, float *xedge, const 
   }
 }
 
+// ---------------------------------------------------------------------------
+// advection by a velocity field
+// ---------------------------------------------------------------------------
+// One tile of a stage with a velocity per cell: the upwind side is chosen per
+// cell (a lane), so every cell evaluates its own three windows, from the six
+// scaled differences D1(c-2 .. c+3) of each axis.  A thread owns two
+// x-neighbouring cells, as above, which makes the tile's loads, the velocity's
+// and the result's 64 bits wide, and marches along z, carrying that axis'
+// differences (one new one per cell); the next plane's velocity and phi^n are
+// read a plane ahead.  Same bits as evaluating each cell on its own.  Bound by
+// issue: the three windows are 220 packed operations per cell pair and their
+// selection 60 moves.  us per stage, two z-neighbouring cells per thread of a
+// 32 x 8 tile / this: 64^3 5.96 / 5.4, 100^3 19.3 / 14.4, 192^3 76 / 62, 256^3
+// 167 / 133.  (Four CTAs per SM at 64 registers; three at 80: 192^3 65, 256^3
+// 138.  Planes unrolled by 1 / 4: 192^3 gradient 1% slower.)
+template <int W, int T, int UNROLL>
+__device__ __forceinline__ void adv_field_tile(const float *tile, const StageArgs<float> &a, int x0, int y0, int z0,
+                                               int tzn, int tid) {
+  using Q = AdvTile<W, T>;
+  const Layout &L = a.L;
+  constexpr int st_y = Q::SXW, st_z = Q::SXW * Q::SYW;
+  const int lx = tid % Q::LX, w = Q::row(tid);
+  const int i = x0 + 2 * lx, j = y0 + w;
+  if (i >= L.nx || j >= L.ny) return;
+  const bool two = i + 1 < L.nx;
+  const int px0 = a.periodic ? image_of(i, L.nx) : 0, px1 = a.periodic && two ? image_of(i + 1, L.nx) : 0;
+  const int py = a.periodic ? image_of(j, L.ny) : 0;
+  const int kmax = min(tzn, L.nz - z0);
+  const float *col = tile + 3 * st_z + (w + 3) * st_y + 2 * lx + 4;  // cell (i, j) of the first plane
+  auto ld2 = [](const float *p) { return *reinterpret_cast<const float2 *>(p); };
+  const float2 ix = sp(a.inv[0]), iy = sp(a.inv[1]), iz = sp(a.inv[2]);
+  auto diff = [](float2 lo, float2 hi) { return fma2(sp(-1.f), lo, hi); };
+  // the upwind value from the differences (spatial_derivatives3d.f.in:2756-2812):
+  // D1(c-2 .. c+2) for v > 0, D1(c+3 .. c-1) otherwise, 0 where |v| < zero_tol
+  auto upwind = [](const float2 D[6], float2 vel) {
+    const bool b0 = vel.x > 0.f, b1 = vel.y > 0.f;
+    float2 v[5];
+#pragma unroll
+    for (int q = 0; q < 5; q++) v[q] = make_float2(b0 ? D[q].x : D[5 - q].x, b1 ? D[q].y : D[5 - q].y);
+    float2 g = weno5_x2(v[0], v[1], v[2], v[3], v[4]);
+    if (fabsf(vel.x) < 1e-11f) g.x = 0.f;
+    if (fabsf(vel.y) < 1e-11f) g.y = 0.f;
+    return g;
+  };
+
+  // z march: D1(z0-2 .. z0+2) and the scaled phi(z0+2)
+  float2 Dz[6], zl;
+  {
+    float2 p[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) p[q] = mul2(ld2(col + (q - 3) * st_z), iz);
+#pragma unroll
+    for (int q = 0; q < 5; q++) Dz[q + 1] = diff(p[q], p[q + 1]);
+    zl = p[5];
+  }
+  const float *un_src = a.stage == 1 ? nullptr : a.phi_n;
+  long long cell = L.idx(i, j, z0);
+  float2 vn[3], un_next = un_src ? ld2(un_src + cell) : sp(0.f);
+#pragma unroll
+  for (int d = 0; d < 3; d++) vn[d] = ld2(a.vel[d] + cell);
+#pragma unroll UNROLL
+  for (int tz = 0; tz < kmax; tz++) {
+    const float2 vx = vn[0], vy = vn[1], vz = vn[2], un = un_next;
+    if (tz + 1 < kmax) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) vn[d] = ld2(a.vel[d] + cell + L.pz);
+      if (un_src) un_next = ld2(un_src + cell + L.pz);
+    }
+    const float2 u0 = ld2(col);  // phi(i), phi(i+1)
+    float2 dot = sp(0.f), D[6];
+    {
+      const float2 e0 = mul2(ld2(col - 4), ix), e1 = mul2(ld2(col - 2), ix), e2 = mul2(u0, ix);
+      const float2 e3 = mul2(ld2(col + 2), ix), e4 = mul2(ld2(col + 4), ix);
+      // (phi(s), phi(s+1)) for s = i-3, i-1, i+1, i+3
+      const float2 o0 = make_float2(e0.y, e1.x), o1 = make_float2(e1.y, e2.x), o2 = make_float2(e2.y, e3.x);
+      const float2 o3 = make_float2(e3.y, e4.x);
+      D[0] = diff(o0, e1); D[1] = diff(e1, o1); D[2] = diff(o1, e2);
+      D[3] = diff(e2, o2); D[4] = diff(o2, e3); D[5] = diff(e3, o3);
+      dot = fma2(vx, upwind(D, vx), dot);
+    }
+    {
+      float2 p[7];
+#pragma unroll
+      for (int q = 0; q < 7; q++) p[q] = mul2(q == 3 ? u0 : ld2(col + (q - 3) * st_y), iy);
+#pragma unroll
+      for (int q = 0; q < 6; q++) D[q] = diff(p[q], p[q + 1]);
+      dot = fma2(vy, upwind(D, vy), dot);
+    }
+    {
+      const float2 p = mul2(ld2(col + 3 * st_z), iz);
+#pragma unroll
+      for (int q = 0; q < 5; q++) Dz[q] = Dz[q + 1];
+      Dz[5] = diff(zl, p);
+      zl = p;
+      dot = fma2(vz, upwind(Dz, vz), dot);
+    }
+    const float2 rhs = make_float2(-dot.x, -dot.y);
+    float2 u = fma2(sp(a.dt), rhs, u0);  // tvd_runge_kutta3d.f:78
+    if (a.stage == 2) u = fma2(sp(0.75f), un, mul2(sp(0.25f), u));                  // :403-404
+    else if (a.stage == 3) u = fma2(sp(1.f / 3.f), un, mul2(sp(2.f / 3.f), u));  // :490-492
+    store_pair(a.out, L, cell, u, two, px0, px1, py, a.periodic ? image_of(z0 + tz, L.nz) : 0);
+    col += st_z;
+    cell += L.pz;
+  }
+}
+
 // the stage kernel of a single grid: tiles of W x ROWS x tzn cells
 constexpr int kAdvThreads = 256;
-template <int W>
-static __global__ void __launch_bounds__(kAdvThreads, 3)
+template <int W, bool FIELD>
+static __global__ void __launch_bounds__(kAdvThreads, FIELD ? 4 : 3)
     k_adv_x2(const __grid_constant__ CUtensorMap tm, StageArgs<float> a, int tzn) {
   using Q = AdvTile<W, kAdvThreads>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *tile = reinterpret_cast<float *>(smem_raw);
   __shared__ __align__(8) uint64_t bar;
-  __shared__ float xedge[5 * RZ_MAX * Q::ROWS];
+  __shared__ float xedge[FIELD ? 1 : 5 * RZ_MAX * Q::ROWS];
   const int tid = threadIdx.x + 32 * threadIdx.y;
   const int x0 = blockIdx.x * W, y0 = blockIdx.y * Q::ROWS, z0 = blockIdx.z * tzn;
   if (tid == 0) {
@@ -234,12 +343,16 @@ static __global__ void __launch_bounds__(kAdvThreads, 3)
     fill_face_ghosts<float>(tile, Q::SXW, Q::SYW, tzn + 6, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
     __syncthreads();
   }
-  adv_tile<W, kAdvThreads, RZ_MAX, 8>(tile, xedge, a, x0, y0, z0, tzn, tid);
+  if constexpr (FIELD) adv_field_tile<W, kAdvThreads, 2>(tile, a, x0, y0, z0, tzn, tid);
+  else adv_tile<W, kAdvThreads, RZ_MAX, 8>(tile, xedge, a, x0, y0, z0, tzn, tid);
 }
 
 // the instance for a row length
 using StageX2 = void (*)(const CUtensorMap, StageArgs<float>, int);
-inline StageX2 adv_x2_kernel(int w) { return w == 64 ? k_adv_x2<64> : (w == 32 ? k_adv_x2<32> : k_adv_x2<16>); }
+template <bool FIELD>
+inline StageX2 adv_x2_kernel(int w) {
+  return w == 64 ? k_adv_x2<64, FIELD> : (w == 32 ? k_adv_x2<32, FIELD> : k_adv_x2<16, FIELD>);
+}
 
 }  // namespace fused
 }  // namespace lsmgpu

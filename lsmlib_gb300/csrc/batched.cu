@@ -276,7 +276,7 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
 
   if (want_loop) {
     // comparison mode: one single-grid stage launch per grid per stage
-    const auto kern = fused::adv_x2_kernel(kLoopW);
+    const auto kern = fused::adv_x2_kernel<false>(kLoopW);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)AdvTile<kLoopW, fused::kAdvThreads>::smem(kDepth));
     for (int step = 0; step < n_steps; step++)

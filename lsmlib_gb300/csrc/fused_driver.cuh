@@ -214,23 +214,6 @@ inline int sm_count() {
   }
   return sms;
 }
-// Tile depth of the FP32 k_stage_f32 launches of a grid: 8, or 4 where the
-// 4-plane tiles fill whole waves of resident CTAs at least 10% better (a
-// partly filled last wave costs a whole one; five CTAs per SM at either
-// depth; a grid of less than one wave gets twice the CTAs).  At 128^3, 1024
-// 8-plane tiles are 1.35 waves on 152 SMs, 2048 4-plane tiles 2.7; at 192^3
-// and 256^3 both depths fill their waves equally and 8 is kept.
-inline int stage_tz_f32(const Layout &L) {
-  const long long slots = 5LL * sm_count();
-  const long long cols = (long long)((L.nx + TX - 1) / TX) * ((L.ny + TY - 1) / TY);
-  auto eff = [&](int tz) {
-    const long long tiles = cols * ((L.nz + tz - 1) / tz);
-    const long long waves = (tiles + slots - 1) / slots;
-    return (double)L.nz / ((double)waves * slots * tz / (double)cols);  // used fraction of the wave slots
-  };
-  return eff(4) > 1.1 * eff(8) ? 4 : 8;
-}
-
 // Tile depth of the FP64 k_stage launches: the arithmetic of one plane takes
 // far longer than its share of the tile load, so shallow tiles cost nothing
 // and only the tail of the launch matters: 4 planes where the grid still has
@@ -245,62 +228,74 @@ inline int stage_tz_f64(const Layout &L) {
   return 1;
 }
 
-// Tile depth of k_reinit_x2 and k_adv_x2 (figures: k_reinit_x2).  A grid of
-// fewer 8-plane tiles than SMs is a matter of one tile's latency, about 4 us
-// and 0.8 us per plane: 4 planes, or 2 where 4-plane tiles are fewer than SMs
-// too (37 x 33 x 41: 11.7 us per stage with 8, 7.1 with 2; 64^3: 11.7 and
-// 8.0).  Larger grids take 8 or 10 planes, whichever makes the busiest SM's
-// tiles shorter in all, a tile costing one plane beside its own (128^3: 25.0
-// us with 8, 23.5 with 10; 160 x 150 x 140: 37.7 and 40.8; 192^3: 63.0 and
-// 61.0).
-inline int x2_tz(long long cols, int nz) {
-  const int sms = sm_count();
-  auto tiles = [&](int tz) { return cols * ((nz + tz - 1) / tz); };
-  if (tiles(8) < sms) return tiles(4) < sms ? 2 : 4;
-  auto planes = [&](int tz) { return (tiles(tz) + sms - 1) / sms * (tz + 1); };
-  return planes(10) < planes(8) ? 10 : 8;
-}
-
-// The tiles of k_reinit_x2 (64 x 8 cells of a plane) and k_adv_x2.  The
-// latter's 512 cells are 64 x 8, 32 x 16 or 16 x 32, whichever covers the
-// fewest cells of the plane, the widest of equals (us per stage, 64 x 8 and
-// the rule's choice: 80^3 9.3 and 7.2, 130 x 64 x 64 10.5 and 7.3, 100^3 14.5
-// and 13.3).
+// Tiles of the FP32 stage kernels: w x h cells of a plane (512), tz planes.
 struct TileX2 {
   int w, h, tz;
   size_t smem() const { return (size_t)(w + 8) * (h + 6) * (tz + 6) * sizeof(float); }
 };
-template <int MODE>
-TileX2 tile_x2(const Layout &L) {
-  TileX2 t{0, 0, 0};
-  long long best = 0;
-  for (int w = RX; w >= (MODE == REINIT ? RX : 16); w /= 2) {
-    const int h = 512 / w;
-    const long long cols = (long long)((L.nx + w - 1) / w) * ((L.ny + h - 1) / h);
-    if (best == 0 || cols < best) t = TileX2{w, h, 0}, best = cols;
-  }
-  t.tz = x2_tz(best, L.nz);
-  return t;
+
+// k_reinit_x2 (64 x 8 cells).  A grid of fewer 8-plane tiles than SMs is a
+// matter of one tile's latency, about 4 us and 0.8 us per plane: 4 planes, or
+// 2 where 4-plane tiles are fewer than SMs too (37 x 33 x 41: 11.7 us per
+// stage with 8, 7.1 with 2; 64^3: 11.7 and 8.0).  Larger grids take 8 or 10
+// planes, whichever makes the busiest SM's tiles shorter in all, a tile
+// costing one plane beside its own (128^3: 25.0 us with 8, 23.5 with 10; 160 x
+// 150 x 140: 37.7 and 40.8; 192^3: 63.0 and 61.0).
+inline TileX2 reinit_tile(const Layout &L) {
+  const long long cols = (long long)((L.nx + RX - 1) / RX) * ((L.ny + RY - 1) / RY);
+  const int sms = sm_count();
+  auto tiles = [&](int tz) { return cols * ((L.nz + tz - 1) / tz); };
+  auto planes = [&](int tz) { return (tiles(tz) + sms - 1) / sms * (tz + 1); };
+  int tz = planes(10) < planes(8) ? 10 : 8;
+  if (tiles(8) < sms) tz = tiles(4) < sms ? 2 : 4;
+  return TileX2{RX, RY, tz};
 }
 
-// FP32 reinitialization and constant-velocity advection run k_reinit_x2 and
-// k_adv_x2; every other form runs k_stage or k_stage_f32.
-template <class R, int MODE, bool EXACT>
-constexpr bool uses_x2() {
-  return !EXACT && sizeof(R) == 4 && MODE != ADV_FIELD;
+// k_adv_x2: rows of 64, 32 or 16 cells and 2 to 10 planes, the pair with the
+// shortest run of the busiest SM: the first of its n tiles at a lone tile's
+// latency, the others at the rate of an SM with all its CTAs, in us
+//   constant velocity  2.5 + 0.69 tz  and  0.41 + 0.39 tz,
+//   velocity field     2.5 + 0.85 tz  and  0.24 + 0.59 tz,
+// fitted to 24^3 and 256^3 at each depth.  Measured against it, constant
+// velocity: 100^3 64 x 8 x 4 13.2 (13.2), x 8 14.2 (15.2); 75 x 120 x 61 16 x
+// 32 x 2 8.6 (8.7), x 10 10.0 (10.4); field: 100^3 64 x 8 x 2 14.4 (15.5), x 8
+// 18.6 (19.2); 128^3 64 x 8 x 4 20.5 (21.4), x 8 23.2 (24.1); 192^3 62.6 (62.9)
+// and 63.2 (63.6).
+inline TileX2 adv_tile_of(const Layout &L, bool field) {
+  const float lone = field ? 0.85f : 0.69f, tile = field ? 0.24f : 0.41f, plane = field ? 0.59f : 0.39f;
+  const int sms = sm_count();
+  TileX2 t{RX, RY, 8};
+  float best = INFINITY;
+  for (int w = RX; w >= 16; w /= 2) {
+    const int h = 512 / w;
+    const long long cols = (long long)((L.nx + w - 1) / w) * ((L.ny + h - 1) / h);
+    for (int tz = RZ_MAX; tz >= 2; tz -= 2) {
+      const long long zt = (L.nz + tz - 1) / tz;
+      if (zt > 65535) continue;
+      const float cost = 2.5f + lone * tz + (float)((cols * zt + sms - 1) / sms - 1) * (tile + plane * tz);
+      if (cost < best) t = TileX2{w, h, tz}, best = cost;
+    }
+  }
+  return t;
 }
+template <int MODE>
+TileX2 tile_x2(const Layout &L) {
+  return MODE == REINIT ? reinit_tile(L) : adv_tile_of(L, MODE == ADV_FIELD);
+}
+
+// The FP32 forms run k_reinit_x2 and k_adv_x2, the FP64 ones k_stage.
+template <class R, bool EXACT>
+constexpr bool uses_x2() { return !EXACT && sizeof(R) == 4; }
 
 // Tensor map of a padded work buffer with the staged box of the stage kernel
 // launch_stage<R, MODE, EXACT> runs.
 template <class R, int MODE, bool EXACT>
 bool encode_stage_tmap(CUtensorMap *m, const R *p, const Layout &L) {
   const long long ex = (long long)L.nx + GX + 3, ey = (long long)L.ny + 2 * GY, ez = (long long)L.nz + 2 * GZ;
-  if constexpr (uses_x2<R, MODE, EXACT>()) {
+  if constexpr (uses_x2<R, EXACT>()) {
     const TileX2 t = tile_x2<MODE>(L);
     return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, t.w + 8, t.h + 6, t.tz + 6);
   }
-  if constexpr (!EXACT && sizeof(R) == 4)
-    return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f32(L) + 6);
   return encode_tmap_3d(m, p, sizeof(R), ex, ey, ez, L.py, L.pz, SX, SY, stage_tz_f64(L) + 6);
 }
 
@@ -321,31 +316,21 @@ static void launch_stage(const CUtensorMap &tm, const StageArgs<R> &a, bool prep
     return dim3((unsigned)((L.nx + tx - 1) / tx), (unsigned)((L.ny + ty - 1) / ty), (unsigned)((L.nz + tz - 1) / tz));
   };
   constexpr size_t kPlane = (size_t)SX * SY * sizeof(R);
-  if constexpr (uses_x2<R, MODE, EXACT>()) {
+  if constexpr (uses_x2<R, EXACT>()) {
     if (!attr_set) {
       if constexpr (MODE == REINIT)
         for (auto k : {k_reinit_x2<false>, k_reinit_x2<true>}) want_smem(k, reinit_x2_smem(RZ_MAX));
-      if constexpr (MODE == ADV_CONST)
-        for (int w = 16; w <= 64; w *= 2) want_smem(adv_x2_kernel(w), TileX2{w, 512 / w, RZ_MAX}.smem());
+      else
+        for (int w = 16; w <= 64; w *= 2)
+          want_smem(adv_x2_kernel<MODE == ADV_FIELD>(w), TileX2{w, 512 / w, RZ_MAX}.smem());
       attr_set = true;
     }
     if (prepare_only) return;
     const TileX2 t = tile_x2<MODE>(L);
     StageX2 kern = nullptr;
     if constexpr (MODE == REINIT) kern = a.periodic ? k_reinit_x2<true> : k_reinit_x2<false>;
-    if constexpr (MODE == ADV_CONST) kern = adv_x2_kernel(t.w);
+    else kern = adv_x2_kernel<MODE == ADV_FIELD>(t.w);
     kern<<<grid(t.w, t.h, t.tz), dim3(32, 8), t.smem(), stream()>>>(tm, a, t.tz);
-  } else if constexpr (!EXACT && sizeof(R) == 4) {
-    // packed cell pairs, tile depth per grid
-    if (!attr_set) {
-      want_smem(k_stage_f32<8>, kPlane * 14);
-      want_smem(k_stage_f32<4>, kPlane * 10);
-      attr_set = true;
-    }
-    if (prepare_only) return;
-    const int tz = stage_tz_f32(L);
-    const auto kern = tz == 4 ? k_stage_f32<4> : k_stage_f32<8>;
-    kern<<<grid(TX, TY, tz), dim3(TX, TY), kPlane * (tz + 6), stream()>>>(tm, a);
   } else {
     if (!attr_set) want_smem(k_stage<R, MODE, EXACT>, kPlane * SZ);
     attr_set = true;

@@ -552,131 +552,5 @@ __device__ __forceinline__ void weno5_pm_x2(const float2 D[6], float2 &gp, float
   gp = combine(q1p, q2p, q3p, P1p, B, A);
 }
 
-// Computes one TX x TY x TZ_ tile of a field-velocity advection stage whose
-// haloed input ((TX + 8) x (TY + 6) x (TZ_ + 6)) is in `tile`, the calling
-// thread at (tx, ty) of the tile, two z-neighbouring cells at a time.
-template <int TZ_>
-__device__ __forceinline__ void adv_field_tile(const float *tile, const StageArgs<float> &a, int x0, int y0, int z0,
-                                               int tx, int ty) {
-  const Layout &L = a.L;
-  const int i = x0 + tx, j = y0 + ty;
-  if (i >= L.nx || j >= L.ny) return;
-  const int sx = tx + 4, sy = ty + 3;
-  const int kmax = min(TZ_, L.nz - z0);
-  const int st[3] = {1, SX, SX * SY};
-  const float2 inv[3] = {sp(a.inv[0]), sp(a.inv[1]), sp(a.inv[2])};
-  // offsets of the column's periodic images along x and y (0: none)
-  const int oi = image_of(i, L.nx), oj = image_of(j, L.ny);
-
-  for (int tz = 0; tz < kmax; tz += 2) {
-    const bool two = tz + 1 < kmax;  // the second lane is a real cell
-    const float *c0 = tile + ((tz + 3) * SY + sy) * SX + sx;
-    const float *c1 = two ? c0 + SX * SY : c0;
-    const int k0 = z0 + tz, k1 = two ? k0 + 1 : k0;
-    const long long cell0 = L.idx(i, j, k0), cell1 = L.idx(i, j, k1);
-    float2 rhs;
-    {
-      float2 dot = sp(0.f);
-      float vel0[3], vel1[3];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        vel0[d] = a.vel[d][cell0];
-        vel1[d] = a.vel[d][cell1];
-      }
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        // per lane: the backward stencil D1(c-2..c+2) for v > 0, the forward
-        // stencil D1(c+3..c-1) otherwise (spatial_derivatives3d.f.in:2756-2812);
-        // the six differences are loaded at fixed offsets and the lane's
-        // stencil is selected in registers
-        float2 a7[7], D[6];
-#pragma unroll
-        for (int q = -3; q <= 3; q++) a7[q + 3] = mul2(make_float2(c0[q * st[d]], c1[q * st[d]]), inv[d]);
-#pragma unroll
-        for (int f = 0; f < 6; f++) D[f] = fma2(sp(-1.f), a7[f], a7[f + 1]);
-        const bool b0 = vel0[d] > 0.f, b1 = vel1[d] > 0.f;
-        float2 v[5];
-#pragma unroll
-        for (int q = 0; q < 5; q++) {
-          v[q].x = b0 ? D[q].x : D[5 - q].x;
-          v[q].y = b1 ? D[q].y : D[5 - q].y;
-        }
-        float2 g = weno5_x2(v[0], v[1], v[2], v[3], v[4]);
-        if (fabsf(vel0[d]) < 1e-11f) g.x = 0.f;
-        if (fabsf(vel1[d]) < 1e-11f) g.y = 0.f;
-        dot = fma2(make_float2(vel0[d], vel1[d]), g, dot);
-      }
-      rhs = make_float2(-dot.x, -dot.y);
-    }
-    const float2 u0 = make_float2(c0[0], c1[0]);
-    float2 u;
-    if (a.stage == 1) {
-      u = fma2(sp(a.dt), rhs, u0);
-    } else {
-      const float2 un = make_float2(a.phi_n[cell0], a.phi_n[cell1]);
-      if (a.stage == 2)
-        u = fma2(sp(0.75f), un, mul2(sp(0.25f), fma2(sp(a.dt), rhs, u0)));
-      else
-        u = fma2(sp(1.f / 3.f), un, mul2(sp(2.f / 3.f), fma2(sp(a.dt), rhs, u0)));
-    }
-    a.out[cell0] = u.x;
-    if (two) a.out[cell1] = u.y;
-    if (a.periodic) {
-      // the cells' periodic images in the ghost layers (up to 7: each
-      // combination of the axes along which a cell lies within 3 of a face)
-      const bool edge = k0 < 3 || k1 >= L.nz - 3;
-      if ((oi | oj) != 0 || edge) {
-        for (int lane = 0; lane < (two ? 2 : 1); lane++) {
-          const int k = lane ? k1 : k0;
-          const float val = lane ? u.y : u.x;
-          const long long c = lane ? cell1 : cell0;
-          const int ok = k < 3 ? L.nz : (k >= L.nz - 3 ? -L.nz : 0);
-          const long long dx = oi, dy = L.py * oj, dz = L.pz * ok;
-          if (oi) a.out[c + dx] = val;
-          if (oj) a.out[c + dy] = val;
-          if (ok) a.out[c + dz] = val;
-          if (oi && oj) a.out[c + dx + dy] = val;
-          if (oi && ok) a.out[c + dx + dz] = val;
-          if (oj && ok) a.out[c + dy + dz] = val;
-          if (oi && oj && ok) a.out[c + dx + dy + dz] = val;
-        }
-      }
-    }
-  }
-}
-
-// 32 x 8 x TZ_ tiles; the steppers launch TZ_ = 8, or 4 where 4-plane tiles
-// fill the machine's waves better (fused_driver.cuh, stage_tz_f32)
-template <int TZ_>
-__global__ void __launch_bounds__(TX * TY) k_stage_f32(const __grid_constant__ CUtensorMap tm, StageArgs<float> a) {
-  constexpr int SZ_ = TZ_ + 6;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  float *tile = reinterpret_cast<float *>(smem_raw);
-  __shared__ __align__(8) uint64_t bar;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int tid = tx + TX * ty;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ_;
-  if (tid == 0) {
-    prefetch_tmap(&tm);
-    mbar_init(&bar, 1);
-    fence_barrier_init();
-  }
-  __syncthreads();
-  if (tid == 0) {
-    mbar_arrive_expect_tx(&bar, (uint32_t)(SX * SY * SZ_ * sizeof(float)));
-    tma_load_3d(tile, &tm, x0 + GX - 4, y0 + GY - 3, z0 + GZ - 3, &bar);
-  }
-  if (!mbar_wait(&bar, 0, kMaxPolls)) {
-    if (tid == 0) atomicExch(a.err, LSMGPU_ERR_TIMEOUT);
-    mbar_wait(&bar, 0, kMaxPolls);
-    return;
-  }
-  if (a.ghost) {
-    fill_face_ghosts<float>(tile, SX, SY, SZ_, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
-    __syncthreads();
-  }
-  adv_field_tile<TZ_>(tile, a, x0, y0, z0, tx, ty);
-}
-
 }  // namespace fused
 }  // namespace lsmgpu

@@ -223,3 +223,28 @@ def test_fused_advect_f32_constant_velocity_signs(n, v, bc, gpu_lib):
         L.advect_weno5_tvdrk3(t, gb, fb, dx, 0.5 * dx, 3, vel_const=v, bc=bc, precision=precision)
     L.check()
     assert float((t32.double() - t64)[3:-3, 3:-3, 3:-3].abs().max()) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(6, 7, 8), (24, 23, 25), (37, 33, 41), (75, 40, 61), (16, 70, 50), (130, 61, 50), (128, 128, 41)])
+@pytest.mark.parametrize("bc", [L.BC_PERIODIC, L.BC_LINEAR])
+def test_fused_advect_f32_field_tiles(n, bc, gpu_lib):
+    """FP32 advection by a velocity field that changes sign inside the tiles
+    (and is zero in places), at sizes whose rows run as 64-, 32- and 16-cell
+    tiles of several depths, the last tile of each axis ragged, against the
+    FP64 form (which equals the oracle bit for bit)."""
+    import torch
+    fb = (0, n[0] - 1, 0, n[1] - 1, 0, n[2] - 1)
+    gb = tuple(q + (-3, 3)[s % 2] for s, q in enumerate(fb))
+    dx = 2.0 / max(n)
+    X, Y, Z = np.meshgrid(*[2 * np.pi * (np.arange(-3, m + 3) + 0.5) / m for m in n], indexing="ij")
+    phi = np.sin(X) * np.cos(Y) + 0.4 * np.cos(2 * Z + 0.3) * np.sin(Y)
+    vel = [0.5 * np.sin(Y + 0.2) * np.cos(Z), -0.4 * np.cos(X) * np.sin(Z + 0.1), 0.3 * np.sin(X + Y)]
+    vel = [np.where(np.abs(v) < 0.05, 0.0, v) for v in vel]
+    t32 = torch.from_numpy(np.ascontiguousarray(phi.T)).cuda().float()
+    t64 = t32.double()
+    v32 = [torch.from_numpy(np.ascontiguousarray(v.T)).cuda().float() for v in vel]
+    for t, precision, v in ((t32, "f32", v32), (t64, "f64", [q.double() for q in v32])):
+        L.advect_weno5_tvdrk3(t, gb, fb, dx, 0.5 * dx, 3, vel=v, vel_gb=gb, bc=bc, precision=precision)
+    L.check()
+    assert float((t32.double() - t64)[3:-3, 3:-3, 3:-3].abs().max()) <= 1e-5
