@@ -368,7 +368,7 @@ struct Width {
       lim = (float)w;
       if ((double)lim >= w) lim = nextafterf(lim, -INFINITY);
     } else {
-      lim = w;
+      lim = w > 0.0 ? w : 0.0;  // (below_ takes a width that is not negative)
     }
   }
   __device__ __forceinline__ bool in(R v) const {

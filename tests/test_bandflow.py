@@ -94,3 +94,14 @@ def test_band_flow_f32_within_tolerance(gpu_lib):
     assert np.max(np.abs(np.asarray(want_dt) - dts)) <= 1e-5 * max(want_dt)
     band = np.abs(phi) < ARGS["gamma"]
     assert np.max(np.abs(want - got.astype(np.float64))[band]) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("gamma", [0.0, -3 * DX, float("nan")])
+def test_band_without_cells_leaves_phi(precision, gamma, gpu_lib):
+    """|phi| < gamma holds nowhere for a width that is not positive."""
+    phi = spheres_phi().astype(np.float64 if precision == "f64" else np.float32)
+    got = phi.copy(order="F")
+    dts, counts = L.band_flow_weno5_tvdrk3(got, GB, FB, DX, 4, 2, gamma, ARGS["beta"], precision=precision)
+    assert list(counts) == [0, 0] and np.array_equal(got, phi)
