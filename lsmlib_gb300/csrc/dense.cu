@@ -90,7 +90,7 @@ __device__ __forceinline__ AxisCell axis_cell(const Box &fb, unsigned axes) {
   return a;
 }
 
-__global__ void __launch_bounds__(256, 5) k_hj_pm_weno5(Out3 plus, Out3 minus, View<const R> phi, Box fb, unsigned axes,
+__global__ void __launch_bounds__(256, 6) k_hj_pm_weno5(Out3 plus, Out3 minus, View<const R> phi, Box fb, unsigned axes,
                                                         R ix, R iy, R iz) {
   const AxisCell a = axis_cell(fb, axes);
   if (!a.in) return;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256, 5) k_hj_pm_weno5(Out3 plus, Out3 minus, V
 // the minus side of the mirrored line, negated (every rounding is symmetric),
 // so a lane walks its line with the stride's sign and lanes of both sides run
 // the same reconstruction.
-__global__ void __launch_bounds__(256, 5) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx,
+__global__ void __launch_bounds__(256, 7) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx,
                                                             View<const R> vy, View<const R> vz, Box fb, unsigned axes,
                                                             R ix, R iy, R iz) {
   const AxisCell a = axis_cell(fb, axes);

@@ -217,14 +217,14 @@ inline int sm_count() {
 // Tile depth of the FP64 k_stage launches: the arithmetic of one plane takes
 // far longer than its share of the tile load, so shallow tiles cost nothing
 // and only the tail of the launch matters: 4 planes where the grid still has
-// 16 tiles per resident CTA slot (four per SM), else 2, else 1.  (8 where 4
+// 64 tiles per SM, else 2, else 1 (with 96 per SM the same times).  (8 where 4
 // would exceed the grid's z extent limit.)
 inline int stage_tz_f64(const Layout &L) {
-  const long long slots = 4LL * sm_count();
+  const long long enough = 64LL * sm_count();
   const long long cols = (long long)((L.nx + TX - 1) / TX) * ((L.ny + TY - 1) / TY);
   if (L.nz > 4 * 65535) return 8;
   for (int tz = 4; tz > 1; tz /= 2)
-    if (cols * ((L.nz + tz - 1) / tz) >= 16 * slots) return tz;
+    if (cols * ((L.nz + tz - 1) / tz) >= enough) return tz;
   return 1;
 }
 

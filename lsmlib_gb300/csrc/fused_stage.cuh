@@ -187,9 +187,12 @@ __device__ __forceinline__ float weno5_fast(float v1, float v2, float v3, float 
 // The FP64 stage.  Bound by its arithmetic (weno64.cuh: the FP64 pipe with the
 // integer pipes close behind), so the tile only has to be there in time: tiles
 // of `tz` planes (1 to 4, chosen by the launcher so that the last wave of
-// tiles is a small part of the run), four CTAs per SM at 64 registers.
+// tiles is a small part of the run), six CTAs per SM at 40 registers
+// (reinitialization 121 x 118 x 109, 5 steps: four 10.27 ms, five 10.04, six
+// 9.95, seven 10.14; field advection 111 x 104 x 92: five 3.95, six 3.87,
+// seven 3.93).
 template <class R, int MODE, bool EXACT>
-__global__ void __launch_bounds__(TX * TY, MODE == REINIT ? 4 : 5) k_stage(const __grid_constant__ CUtensorMap tm, StageArgs<R> a, int tzn) {
+__global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CUtensorMap tm, StageArgs<R> a, int tzn) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R *tile = reinterpret_cast<R *>(smem_raw);
   __shared__ __align__(8) uint64_t bar;

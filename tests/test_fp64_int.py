@@ -84,3 +84,21 @@ def test_dropin_elementwise_on_all_scales(sym, kind, gpu_lib):
             assert H.same(want[k], got[k]), (name, k)
         for k in wsc:
             assert wsc[k] == gsc[k] or (wsc[k] != wsc[k] and gsc[k] != gsc[k]), (name, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-6, 1e-9, 1e-11, 1e-13, 1e-15, 1e-18, 1e-30])
+@pytest.mark.parametrize("sym", ["lsm3dhjweno5_", "lsm3dupwindhjweno5_"])
+def test_dropin_weno5_around_the_floor_of_epsilon(sym, scale, gpu_lib):
+    """Differences whose 1e-6 v^2 lies on either side of 2^55 times the floor
+    of epsilon (where its addition is left out), and below the floor."""
+    vals = H.dense_case(sym, seed=5)
+    rng = np.random.default_rng(23)
+    phi = H.rough_field(rng, H.GB)
+    vals["phi"] = np.asfortranarray(phi * scale * 10.0 ** rng.uniform(-1, 1, size=phi.shape))
+    want, _ = H.run(H.oracle(), sym, vals)
+    got, _ = H.run(gpu_lib, sym, vals)
+    L.check()
+    for name in H.written_names(sym):
+        if name in got and not name.startswith("d"):
+            assert H.same(want[name], got[name]), name
