@@ -340,7 +340,7 @@ static __global__ void __launch_bounds__(kAdvThreads, FIELD ? 4 : 3)
     return;
   }
   if (a.ghost) {
-    fill_face_ghosts<float>(tile, Q::SXW, Q::SYW, tzn + 6, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
+    fill_face_ghosts<float, W, Q::ROWS>(tile, tzn, x0, y0, z0, a.L, a.ghost, tid);
     __syncthreads();
   }
   if constexpr (FIELD) adv_field_tile<W, kAdvThreads, 2>(tile, a, x0, y0, z0, tzn, tid);

@@ -96,57 +96,60 @@ __device__ __forceinline__ R extrap(R e, R n, int g, int kind) {
 // (boundary_conditions3d.f:46-462): identical values to a fill of the
 // stored array, whose faces are written x, then y, then z, because a face
 // ghost of an axis is written only by that axis' pass from interior cells.
-// (Edge and corner ghosts are read by no axis-aligned stencil.)  Tile cell
-// (a, b, c) holds interior cell (ox + a, oy + b, oz + c).
-// The faces write disjoint cells and read only interior ones, so they are
-// filled in any order; a tile inside the domain on every axis has none (one
-// uniform test).  Threads cover each face plane in 2D (x along threadIdx.x,
-// the other axis along threadIdx.y) and walk the ghost layers, so no index
-// is decomposed by division.  Not inlined, so the stage kernels' register
-// allocation does not depend on it.
-template <class R>
-__device__ __noinline__ void fill_face_ghosts(R *tile, int sdx, int sdy, int sdz, int ox, int oy, int oz, const Layout &L,
-                                 int kind) {
-  if (ox >= 0 && ox + sdx <= L.nx && oy >= 0 && oy + sdy <= L.ny && oz >= 0 && oz + sdz <= L.nz) return;
-  const int sxy = sdx * sdy;
-  // one face: ghost layers 1..3 of axis AX below (up = 0) or above (up = 1)
-  auto face = [&](auto ax_tag, int up) {
-    constexpr int AX = decltype(ax_tag)::value;
-    const int n0 = L.nx, n1 = L.ny, n2 = L.nz;
-    const int nax = AX == 0 ? n0 : (AX == 1 ? n1 : n2);
-    // ranges: ghost layers along AX, interior along the other two, clipped to the tile
-    int lo0 = AX == 0 ? (up ? n0 : -3) : 0, hi0 = AX == 0 ? (up ? n0 + 2 : -1) : n0 - 1;
-    int lo1 = AX == 1 ? (up ? n1 : -3) : 0, hi1 = AX == 1 ? (up ? n1 + 2 : -1) : n1 - 1;
-    int lo2 = AX == 2 ? (up ? n2 : -3) : 0, hi2 = AX == 2 ? (up ? n2 + 2 : -1) : n2 - 1;
-    lo0 = max(lo0, ox); hi0 = min(hi0, ox + sdx - 1);
-    lo1 = max(lo1, oy); hi1 = min(hi1, oy + sdy - 1);
-    lo2 = max(lo2, oz); hi2 = min(hi2, oz + sdz - 1);
-    if (lo0 > hi0 || lo1 > hi1 || lo2 > hi2) return;
-    const int e_at = up ? nax - 1 : 0, n_at = up ? nax - 2 : 1;
-    const int st = AX == 0 ? 1 : (AX == 1 ? sdx : sxy);
-    // plane axes: (1, 2) for an x face, (0, 2) for y, (0, 1) for z
-    constexpr int PA = AX == 0 ? 1 : 0, PB = AX == 2 ? 1 : 2;
-    const int loA = PA == 0 ? lo0 : lo1, hiA = PA == 0 ? hi0 : hi1;
-    const int loB = PB == 1 ? lo1 : lo2, hiB = PB == 1 ? hi1 : hi2;
-    const int loG = AX == 0 ? lo0 : (AX == 1 ? lo1 : lo2), hiG = AX == 0 ? hi0 : (AX == 1 ? hi1 : hi2);
-    // both values of a line are read once, before its ghost cells are written
-    for (int pb = loB + (int)threadIdx.y; pb <= hiB; pb += blockDim.y)
-      for (int pa = loA + (int)threadIdx.x; pa <= hiA; pa += blockDim.x) {
-        const int c0 = AX == 0 ? e_at : pa;
-        const int c1 = AX == 1 ? e_at : (PA == 1 ? pa : pb);
-        const int c2 = AX == 2 ? e_at : pb;
-        R *edge = tile + (c0 - ox) + (c1 - oy) * sdx + (c2 - oz) * sxy;
-        const R e = *edge, n = edge[(n_at - e_at) * st];
-        for (int g = loG; g <= hiG; g++) edge[(g - e_at) * st] = extrap(e, n, up ? g - e_at : -g, kind);
-      }
+// (Edge and corner ghosts are read by no axis-aligned stencil.)
+// Only the lines that the tile's own cells read are filled (x ghosts of its
+// rows, y and z ghosts of its columns), one per thread and pass of 256
+// threads: on small grids the stage is the latency of an edge tile.  The faces
+// write disjoint cells and read only interior ones, so they are filled in any
+// order; a tile inside the domain on every axis has none (one uniform test).
+// Not inlined, so the stage kernels' register allocation does not depend on it.
+// us per reinitialization stage with the whole halo's lines filled face by face
+// / with these: FP32 37 x 33 x 41 5.8 / 4.9, 128^3 21.2 / 19.8, 256^3 129 / 121;
+// FP64 121 x 118 x 109 662 / 637.
+template <class R, int W, int H>
+__device__ __noinline__ void fill_face_ghosts(R *tile, int tzn, int x0, int y0, int z0, const Layout &L, int kind,
+                                              int tid) {
+  constexpr int sy = W + 8, sz = sy * (H + 6), T = 256;
+  if (x0 >= 3 && x0 + W + 3 <= L.nx && y0 >= 3 && y0 + H + 3 <= L.ny && z0 >= 3 && z0 + tzn + 3 <= L.nz) return;
+  R *const cells = tile + 4 + 3 * sy + 3 * sz;  // cell (x0, y0, z0)
+  // ghost layers 1 .. n beyond the edge cell, away from the interior along `out`
+  auto line = [&](R *edge, int out, int n) {
+    const R e = edge[0], in = edge[-out];
+#pragma unroll
+    for (int g = 1; g <= 3; g++)
+      if (g <= n) edge[g * out] = extrap(e, in, g, kind);
   };
-  // only the faces the tile crosses
-  if (ox < 0) face(std::integral_constant<int, 0>{}, 0);
-  if (ox + sdx > L.nx) face(std::integral_constant<int, 0>{}, 1);
-  if (oy < 0) face(std::integral_constant<int, 1>{}, 0);
-  if (oy + sdy > L.ny) face(std::integral_constant<int, 1>{}, 1);
-  if (oz < 0) face(std::integral_constant<int, 2>{}, 0);
-  if (oz + sdz > L.nz) face(std::integral_constant<int, 2>{}, 1);
+  const int kx = min(W, L.nx - x0), ky = min(H, L.ny - y0), kz = min(tzn, L.nz - z0);  // own cells
+  // layers below and above that the tile reads, and the edge cells' offsets
+  const int bx = 3 - x0, by = 3 - y0, bz = 3 - z0;
+  const int ax = x0 + W + 3 - L.nx, ay = y0 + H + 3 - L.ny, az = z0 + tzn + 3 - L.nz;
+  if (bx > 0 || ax > 0)
+    for (int e = tid; e < H * kz; e += T) {
+      const int y = e % H, z = e / H;
+      R *row = cells + y * sy + z * sz;
+      if (y < ky) {
+        if (bx > 0) line(row - x0, -1, bx);
+        if (ax > 0) line(row + L.nx - 1 - x0, 1, ax);
+      }
+    }
+  if (by > 0 || ay > 0)
+    for (int e = tid; e < W * kz; e += T) {
+      const int x = e % W, z = e / W;
+      R *col = cells + x + z * sz;
+      if (x < kx) {
+        if (by > 0) line(col - y0 * sy, -sy, by);
+        if (ay > 0) line(col + (L.ny - 1 - y0) * sy, sy, ay);
+      }
+    }
+  if (bz > 0 || az > 0)
+    for (int e = tid; e < W * ky; e += T) {
+      const int x = e % W, y = e / W;
+      R *col = cells + x + y * sy;
+      if (x < kx) {
+        if (bz > 0) line(col - z0 * sz, -sz, bz);
+        if (az > 0) line(col + (L.nz - 1 - z0) * sz, sz, az);
+      }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CU
     return;
   }
   if (a.ghost) {
-    fill_face_ghosts<R>(tile, SX, SY, szn, x0 - 4, y0 - 3, z0 - 3, a.L, a.ghost);
+    fill_face_ghosts<R, TX, TY>(tile, tzn, x0, y0, z0, a.L, a.ghost, tid);
     __syncthreads();
   }
 

@@ -96,7 +96,7 @@ static __global__ void __launch_bounds__(256, 3)
     return;
   }
   if (a.ghost) {
-    fill_face_ghosts<float>(tile, RSX, RSY, tzn + 6, x0 - 4, y0 - 3, z0 - 3, L, a.ghost);
+    fill_face_ghosts<float, RX, RY>(tile, tzn, x0, y0, z0, L, a.ghost, tid);
     __syncthreads();
   }
 
