@@ -21,9 +21,12 @@
 // pair, where a cell-by-cell tile took 165 and as many again in loads,
 // selection and set-up.  Measured us per periodic stage, the cell-by-cell tile
 // / one kernel per sign triple on 64 x 8 tiles / this kernel: 37 x 33 x 41 4.5
-// / 5.3 / 4.0, 128^3 21.2 / 18.3 / 17.2, 256^3 140 / 98.6 / 97.9, 32 x 256 x
-// 256 21.6 / 21.6 / 17.6.  (Signed strides for the two axes that need no
-// mirrored lanes: 128^3 18.7, 256^3 109.)
+// / 5.3 / 3.8, 128^3 21.2 / 18.3 / 15.7, 256^3 140 / 98.6 / 95.1, 32 x 256 x
+// 256 21.6 / 21.6 / 17.3.  (Signed strides for the two axes that need no
+// mirrored lanes: 128^3 18.7, 256^3 109.  Planes unrolled by 1 / 2 / 4 / 8: 37 x
+// 33 x 41 3.9 / 3.8 / 3.95 / 4.0, 100^3 12.3 / 11.3 / 11.7 / 11.8, 256^3 - / 95.1
+// / 92.8 / 95: a run of planes longer than the instruction cache holds costs
+// the short tiles more than the moves it saves.)
 #pragma once
 
 #include "reinit_x2.cuh"
@@ -344,7 +347,7 @@ static __global__ void __launch_bounds__(kAdvThreads, FIELD ? 4 : 3)
     __syncthreads();
   }
   if constexpr (FIELD) adv_field_tile<W, kAdvThreads, 2>(tile, a, x0, y0, z0, tzn, tid);
-  else adv_tile<W, kAdvThreads, RZ_MAX, 8>(tile, xedge, a, x0, y0, z0, tzn, tid);
+  else adv_tile<W, kAdvThreads, RZ_MAX, 2>(tile, xedge, a, x0, y0, z0, tzn, tid);
 }
 
 // the instance for a row length

@@ -236,17 +236,19 @@ struct TileX2 {
 
 // k_reinit_x2 (64 x 8 cells).  A grid of fewer 8-plane tiles than SMs is a
 // matter of one tile's latency, about 4 us and 0.8 us per plane: 4 planes, or
-// 2 where 4-plane tiles are fewer than SMs too (37 x 33 x 41: 11.7 us per
-// stage with 8, 7.1 with 2; 64^3: 11.7 and 8.0).  Larger grids take 8 or 10
-// planes, whichever makes the busiest SM's tiles shorter in all, a tile
-// costing one plane beside its own (128^3: 25.0 us with 8, 23.5 with 10; 160 x
-// 150 x 140: 37.7 and 40.8; 192^3: 63.0 and 61.0).
+// 2 where 4-plane tiles are fewer than SMs too (37 x 33 x 41: 10.4 us per
+// stage with 8, 5.7 with 2; 64^3: 10.2 and 6.7).  Larger grids take 6, 8 or 10
+// planes, whichever makes the busiest SM's tiles shorter in all, a tile costing
+// one plane beside its own (100^3: 15.2 us with 6, 17.7 with 8, 16.7 with 10;
+// 128^3: 23.9, 23.3, 21.3; 192^3: 65.9, 59.6, 58.4; 256^3: 142, 130, 129).
 inline TileX2 reinit_tile(const Layout &L) {
   const long long cols = (long long)((L.nx + RX - 1) / RX) * ((L.ny + RY - 1) / RY);
   const int sms = sm_count();
   auto tiles = [&](int tz) { return cols * ((L.nz + tz - 1) / tz); };
   auto planes = [&](int tz) { return (tiles(tz) + sms - 1) / sms * (tz + 1); };
-  int tz = planes(10) < planes(8) ? 10 : 8;
+  int tz = 8;
+  for (int t : {6, 10})
+    if (planes(t) < planes(tz)) tz = t;
   if (tiles(8) < sms) tz = tiles(4) < sms ? 2 : 4;
   return TileX2{RX, RY, tz};
 }
