@@ -901,12 +901,12 @@ MEASURED_STAGE_TRAFFIC = 284.6e6
 # FMA-pipe thread-instructions (a packed FFMA2 / FMUL2 / FADD2 counts once)
 # per cell of one headline stage launch (k_reinit_x2, ncu
 # sm__inst_executed_pipe_fma.sum x 32 / 256^3 cells), and FP64 pipe
-# operations (DFMA + DMUL + DADD thread-instructions, the IEEE division and
-# square-root sequences included) per cell-update of the FP64 parity form
+# thread-instructions (the rest of the FP64 arithmetic runs as integer work)
+# per cell-update of the FP64 parity form
 # (3 x one stage launch of k_stage<double, REINIT> at 128^3); both from the
 # captures summarised in profiles/k_reinit_x2_reinit_f32_256.md
-MEASURED_FMA_PIPE_INSTR_PER_CELL_STAGE = 119.9
-MEASURED_FP64_OPS_PER_CELL_UPDATE = 3 * 633.5
+MEASURED_FMA_PIPE_INSTR_PER_CELL_STAGE = 90.8
+MEASURED_FP64_OPS_PER_CELL_UPDATE = 3 * 186.8
 
 
 # ---------------------------------------------------------------------------
