@@ -205,7 +205,8 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
       // (the launch loop runs the single-grid kernel's 32 x 16 tiles)
       G.wide = want_loop || cover(32, Wide::ROWS) <= cover(16, Narrow::ROWS) ? 1 : 0;
       const int tw = G.wide ? 32 : 16, th = want_loop ? kLoopRows : (G.wide ? Wide::ROWS : Narrow::ROWS);
-      G.ntz = (G.L.nz + depth - 1) / depth;
+      const int deep = G.L.nz > 65535 * depth ? kDepth : depth;  // tile positions are 16-bit
+      G.ntz = (G.L.nz + deep - 1) / deep;
       G.tz = ((G.L.nz + G.ntz - 1) / G.ntz + 1) / 2 * 2;
       G.ntz = (G.L.nz + G.tz - 1) / G.tz;
       G.ntx = (G.L.nx + tw - 1) / tw;
