@@ -19,7 +19,9 @@
 // Bound by the issue of FP32 and data-movement instructions (62% and 38% of
 // their pipes at 64% of the issue slots): about 130 packed operations per cell
 // pair, where a cell-by-cell tile took 165 and as many again in loads,
-// selection and set-up.  Measured us per periodic stage, the cell-by-cell tile
+// selection and set-up.  The differences are not divided by the spacing; phi
+// comes in units in which that keeps their squares in range (spacing_scale).
+// Measured us per periodic stage, the cell-by-cell tile
 // / one kernel per sign triple on 64 x 8 tiles / this kernel: 37 x 33 x 41 4.5
 // / 5.3 / 3.8, 128^3 21.2 / 18.3 / 15.7, 256^3 140 / 98.6 / 95.1, 32 x 256 x
 // 256 21.6 / 21.6 / 17.3.  (Signed strides for the two axes that need no

@@ -44,6 +44,7 @@ struct GridDesc {
   Layout L;
   long long off;  // element offset of this grid's region in each work buffer
   float vconst[3], inv[3], floor4[3], dt;  // |velocity|
+  float scale;    // of phi in the work layout (spacing_scale)
   int flip;       // axes of negative velocity: mirrored in the work layout
   int wide;       // 1: 32 x 8 tiles, 0: 16 x 16 tiles
   int tz;         // tile depth, even
@@ -112,14 +113,16 @@ __global__ void __launch_bounds__(kThreads, 6) k_batch_stage(const GridDesc *__r
 }
 
 // copies between the caller's packed LSMLIB arrays (3 ghost cells per side)
-// and the padded work regions; blockIdx.y is the grid, a warp takes x rows
-// (an index division per row, not per cell)
+// and the padded work regions, phi scaled and divided out again (a power of
+// two); blockIdx.y is the grid, a warp takes x rows (an index division per row,
+// not per cell)
 __global__ void __launch_bounds__(256) k_batch_pack(float *work, float *user, const GridDesc *gd,
                                                     const long long *uoff, int unpack) {
   const GridDesc &G = gd[blockIdx.y];
   const Layout L = G.L;
   const int ux = L.nx + 6, uy = L.ny + 6;
   const long long rows = (long long)uy * (L.nz + 6);
+  const float scale = unpack ? 1.f / G.scale : G.scale;
   float *const w0 = work + G.off;
   float *const u0 = user + uoff[blockIdx.y];
   for (long long r = blockIdx.x * 8 + threadIdx.x / 32; r < rows; r += gridDim.x * 8) {
@@ -129,9 +132,9 @@ __global__ void __launch_bounds__(256) k_batch_pack(float *work, float *user, co
     const int step = G.flip & 1 ? -1 : 1;
     float *const u = u0 + r * ux;
     if (unpack) {
-      for (int i = threadIdx.x % 32; i < ux; i += 32) u[i] = w[step * i];
+      for (int i = threadIdx.x % 32; i < ux; i += 32) u[i] = w[step * i] * scale;
     } else {
-      for (int i = threadIdx.x % 32; i < ux; i += 32) w[step * i] = u[i];
+      for (int i = threadIdx.x % 32; i < ux; i += 32) w[step * i] = u[i] * scale;
     }
   }
 }
@@ -194,10 +197,11 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
       G.L = fused::make_layout(dims[3 * g], dims[3 * g + 1], dims[3 * g + 2]);
       G.off = total;
       total += (G.L.elems() + 31) / 32 * 32;
+      G.scale = fused::spacing_scale(spacing + 3 * g);
       for (int d = 0; d < 3; d++) {
         G.vconst[d] = vel[3 * g + d] < 0.f ? -vel[3 * g + d] : vel[3 * g + d];
         G.inv[d] = 1.0f / spacing[3 * g + d];
-        G.floor4[d] = fused::eps_floor4(spacing[3 * g + d]);
+        G.floor4[d] = fused::eps_floor4((double)spacing[3 * g + d] * G.scale);
       }
       G.dt = dt[g];
       G.flip = fused::mirrored_axes(vel + 3 * g);

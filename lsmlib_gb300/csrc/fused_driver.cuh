@@ -29,11 +29,17 @@ constexpr int kPackZ = 8;
 
 // dst2 (optional) receives the same values (the phi0 copy of the
 // reinitialization's sign form); bit d of `flip`: the layout is mirrored
-// along axis d
+// along axis d; FP32 values are multiplied by `scale`, a power of two
+// (spacing_scale), on the way in and by its inverse on the way out
+template <class R>
+__device__ __forceinline__ R scaled(R v, float scale) {
+  if constexpr (sizeof(R) == 4) return v * scale;
+  else return v;
+}
 __device__ __forceinline__ int maybe_mirrored(int i, int n, bool flip) { return flip ? n - 1 - i : i; }
 template <class R>
 __global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int jlo, int klo, R *dst2 = nullptr,
-                       int flip = 0) {
+                       int flip = 0, float scale = 1.f) {
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) - GX;
   const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y) - GY;
   const int k0 = (int)(blockIdx.z * kPackZ) - GZ;
@@ -44,7 +50,7 @@ __global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
     const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
-    v[q] = (in_xy && gk >= gb.lo[2] && gk <= gb.hi[2]) ? src(gi, gj, gk) : R(0);
+    v[q] = (in_xy && gk >= gb.lo[2] && gk <= gb.hi[2]) ? scaled(src(gi, gj, gk), scale) : R(0);
   }
 #pragma unroll
   for (int q = 0; q < kPackZ; q++)
@@ -56,7 +62,8 @@ __global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int
 }
 
 template <class R>
-__global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, int jlo, int klo, int flip = 0) {
+__global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, int jlo, int klo, int flip = 0,
+                         float scale = 1.f) {
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) - 3;
   const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y) - 3;
   const int k0 = (int)(blockIdx.z * kPackZ) - 3;
@@ -66,7 +73,7 @@ __global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, i
   R v[kPackZ];
 #pragma unroll
   for (int q = 0; q < kPackZ; q++)
-    if (k0 + q <= L.nz + 2) v[q] = src[L.idx(i, j, k0 + q)];
+    if (k0 + q <= L.nz + 2) v[q] = scaled(src[L.idx(i, j, k0 + q)], scale);
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
     const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
@@ -404,14 +411,18 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   // by the stage (periodic images) or computed by the next stage's loader
   cudaStream_t s = stream();
   cudaMemsetAsync(err, 0, sizeof(int), s);
-  // k_adv_x2 takes velocities that are not negative
-  const int flip = (!EXACT && sizeof(R) == 4 && rs.mode == ADV_CONST) ? mirrored_axes(rs.vconst) : 0;
+  // k_adv_x2 takes velocities that are not negative, and phi in units that
+  // suit the spacing
+  constexpr bool x2 = !EXACT && sizeof(R) == 4;
+  const double d3[3] = {rs.dx, rs.dy, rs.dz};
+  const int flip = x2 && rs.mode == ADV_CONST ? mirrored_axes(rs.vconst) : 0;
+  const float scale = x2 && rs.mode == ADV_CONST ? spacing_scale(d3) : 1.f;
   {
     const dim3 blk = pack_block(), grd = pack_grid(nx, ny, nz, GX);
     // the phi0 copy of the sign form (read at interior cells only) is
     // written by the same pass
     LSMGPU_LAUNCH(k_pack<R>, grd, blk, 0, A, L, view((const R *)phi_d, gb), gb, fb.lo[0], fb.lo[1], fb.lo[2], P0,
-                  flip);
+                  flip, scale);
     if (rs.mode == ADV_FIELD)
       for (int d = 0; d < 3; d++)
         LSMGPU_LAUNCH(k_pack<R>, grd, blk, 0, V[d], L, view(vel_d[d], vb), vb, fb.lo[0], fb.lo[1], fb.lo[2]);
@@ -434,8 +445,7 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   for (int d = 0; d < 3; d++) a.vel[d] = V[d];
   for (int d = 0; d < 3; d++) a.vconst[d] = (R)(flip >> d & 1 ? -rs.vconst[d] : rs.vconst[d]);
   a.inv[0] = R(1.0) / (R)rs.dx; a.inv[1] = R(1.0) / (R)rs.dy; a.inv[2] = R(1.0) / (R)rs.dz;
-  const double d3[3] = {rs.dx, rs.dy, rs.dz};
-  for (int d = 0; d < 3; d++) a.floor4[d] = (R)eps_floor4((float)d3[d]);
+  for (int d = 0; d < 3; d++) a.floor4[d] = (R)eps_floor4(d3[d] * scale);
   a.dt = (R)rs.dt;
   {
     R m = rmax(rmax((R)rs.dx, (R)rs.dy), (R)rs.dz);
@@ -489,7 +499,8 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, const R *vx
   if (!graph_replay(key, steps)) steps();
   {
     const dim3 blk = pack_block(), grd = pack_grid(nx, ny, nz, 3);
-    LSMGPU_LAUNCH(k_unpack<R>, grd, blk, 0, view(phi_d, gb), gb, A, L, fb.lo[0], fb.lo[1], fb.lo[2], flip);
+    LSMGPU_LAUNCH(k_unpack<R>, grd, blk, 0, view(phi_d, gb), gb, A, L, fb.lo[0], fb.lo[1], fb.lo[2], flip,
+                  1.f / scale);
   }
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);

@@ -18,6 +18,7 @@
 // under- or overflow in single precision (see weno5_fast).
 #pragma once
 
+#include <cmath>
 #include <type_traits>
 
 #include "lsmgpu_common.cuh"
@@ -71,12 +72,37 @@ struct StageArgs {
   int *err;
 };
 
-// 4 (1e-36 dx^2): LSMLIB's floor is in units of the divided differences.  Kept
-// a normal number (for dx below 0.06 the floor is larger than LSMLIB's then,
-// which only data below about 1e-19 dx can tell).
-inline float eps_floor4(float dx) {
-  const float f = 4e-36f * dx * dx;
-  return f > 1.5e-38f ? f : 1.5e-38f;
+// The FP32 constant-velocity stages square undivided differences, so the grid
+// spacing enters the range of the squares.  The copies into the work layout
+// therefore multiply phi by this power of two (exact; divided out by the copies
+// back), which keeps the spacings as the stages see them between 2^-9, where the
+// floor of epsilon (eps_floor4) is still a normal number, and 2^24, where the
+// squares and weight products of slopes up to 7e10 stay finite.  1 for every
+// spacing already there.  (Axes more than 2^33 apart cannot both be: the widest
+// decides.)
+template <class R>
+inline float spacing_scale(const R dx[3]) {
+  int lo = 0, hi = 0;
+  for (int d = 0; d < 3; d++) {
+    const double h = std::fabs((double)dx[d]);
+    if (!(h > 0.0) || !std::isfinite(h)) return 1.f;
+    const int e = std::ilogb(h);  // 2^e <= h < 2^(e+1)
+    lo = d == 0 || e < lo ? e : lo;
+    hi = d == 0 || e > hi ? e : hi;
+  }
+  int p = lo < -9 ? -9 - lo : 0;
+  if (hi + p > 23) p = 23 - hi;
+  p = p > 126 ? 126 : (p < -126 ? -126 : p);  // 1 / scale is a normal number too
+  return std::ldexp(1.f, p);
+}
+// The weights' common scale (window_q) and 4 (1e-36 dx^2) times it, dx scaled:
+// LSMLIB's floor is in units of the divided differences.  (Kept a normal number
+// where one axis' spacing is out of the range above.)
+constexpr float kWeightScale = 1024.f;
+constexpr float kFloor4 = 4e-36f * kWeightScale;  // dx = 1
+inline float eps_floor4(double dx) {
+  const double f = (double)kFloor4 * dx * dx;
+  return f < 1.5e-38 ? 1.5e-38f : (f < 3e38 ? (float)f : 3e38f);
 }
 
 // One-axis extrapolation of LSMLIB's ghost-cell routines
@@ -405,17 +431,22 @@ __device__ __forceinline__ Tri tri_forms(float2 d0, float2 d1, float2 d2) {
 }
 
 // Weight products of a window from its three indicator forms (x4) and the
-// maximum squared difference m: q_k = 4 S_k / (4 eps) + 1 = (S_k + eps) / eps,
-// eps = 1e-6 m + 1e-36 (LSMLIB's, spatial_derivatives3d.f.in:1296, in units
-// of the unscaled differences, or with the floor scaled to them, floor4 / 4);
-// only ratios of the q_k enter the weights.
-// 1 <= q_k < 4e7, so the squared products stay below 3e30.
+// maximum squared difference m: q_k = (4 S_k / (4 eps) + 1) / kWeightScale =
+// (S_k + eps) / eps / kWeightScale, eps = 1e-6 m + 1e-36 (LSMLIB's,
+// spatial_derivatives3d.f.in:1296, in units of the unscaled differences, or
+// with the floor scaled to them; floor4 is 4 kWeightScale times it); only
+// ratios of the q_k enter the weights.  2^-10 <= q_k < 4e4, so the squared
+// products lie between 2^-40 and 3e18: their products with differences up to
+// 1e18, whose squares are the next to overflow, are finite, and those with
+// differences down to 1e-26 normal.
 struct WQ {
   float2 q23, q13, q12;  // (q2 q3)^2, (q1 q3)^2, (q1 q2)^2
 };
-__device__ __forceinline__ WQ window_q(float2 s1, float2 s2, float2 s3, float2 m, float floor4 = 4e-36f) {
-  const float2 s = rcp2(fma2(sp(4e-6f), m, sp(floor4)));  // 1 / (4 eps), finite: floor4 is a normal number
-  const float2 q1 = fma2(s1, s, sp(1.f)), q2 = fma2(s2, s, sp(1.f)), q3 = fma2(s3, s, sp(1.f));
+__device__ __forceinline__ WQ window_q(float2 s1, float2 s2, float2 s3, float2 m, float floor4 = kFloor4) {
+  // 1 / (4 eps kWeightScale), finite: floor4 is a normal number
+  const float2 s = rcp2(fma2(sp(4e-6f * kWeightScale), m, sp(floor4)));
+  const float2 one = sp(1.f / kWeightScale);
+  const float2 q1 = fma2(s1, s, one), q2 = fma2(s2, s, one), q3 = fma2(s3, s, one);
   const float2 a = mul2(q2, q3), b = mul2(q1, q3), c = mul2(q1, q2);
   return {mul2(a, a), mul2(b, b), mul2(c, c)};
 }
@@ -442,7 +473,7 @@ __device__ __forceinline__ void sides_both(const WQ &w, float2 a, float2 nb, flo
 }
 
 // 2 minus(c) of the window W(c) = D[0..4] = D(c-2 .. c+2), per lane
-__device__ __forceinline__ float2 minus_of_window(const float2 D[5], float floor4 = 4e-36f, Tri *mid = nullptr,
+__device__ __forceinline__ float2 minus_of_window(const float2 D[5], float floor4 = kFloor4, Tri *mid = nullptr,
                                                   Tri *last = nullptr) {
   const Tri a0 = tri_forms(D[0], D[1], D[2]), a1 = tri_forms(D[1], D[2], D[3]), a2 = tri_forms(D[2], D[3], D[4]);
   float2 sq[5];

@@ -112,7 +112,7 @@ static __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int q = 0; q < 5; q++) D[q] = sub2(p[q + 1], p[q]);
     Tri a1, a2;
-    const float2 mv = minus_of_window(D, 4e-36f, &a1, &a2);  // a1 = tri(x0-1), a2 = tri(x0)
+    const float2 mv = minus_of_window(D, kFloor4, &a1, &a2);  // a1 = tri(x0-1), a2 = tri(x0)
     const float2 v[6] = {mv, a1.s1, a2.s1, a2.s2, a1.t, a2.t};
 #pragma unroll
     for (int q = 0; q < 6; q++) {
@@ -166,7 +166,7 @@ static __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int q = 0; q < 5; q++) D[q] = sub2(p[q + 1], p[q]);
     Tri a1, a2;
-    gmz = minus_of_window(D, 4e-36f, &a1, &a2);  // minus(z0); a1 = tri(z0-1), a2 = tri(z0)
+    gmz = minus_of_window(D, kFloor4, &a1, &a2);  // minus(z0); a1 = tri(z0-1), a2 = tri(z0)
     float2 sq[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) sq[q] = mul2(D[q], D[q]);
