@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(256) k_rk(View<R> out, View<const R> a, View<c
       R v;
       if (KIND == 0) v = U[q] + w;
       if (KIND == 1) v = R(0.5) * (U[q] + A[q] + w);
-      if (KIND == 2) v = fma(R(0.25), A[q] + w, mul_(R(0.75), U[q]));  // the product by 1/4 is exact
+      if (KIND == 2) v = fpi::plus_quarter(mul_(R(0.75), U[q]), A[q] + w);
       if (KIND == 3) v = mul_(R(1.0 / 3.0), U[q]) + mul_(R(2.0 / 3.0), A[q] + w);
       out(i, j, k0 + q) = v;
     }

@@ -280,6 +280,13 @@ LSMGPU_FPI_DEV double sqrt_any(double a) {
   if (is_zero(w)) return a;
   return unit_sqrt(a);
 }
+// y + x / 4 as two roundings give it: x / 4 is exact, so one fma does, unless it
+// is below the normal numbers
+LSMGPU_FPI_DEV double plus_quarter(double y, double x) {
+  const W2 w = words(x);
+  if ((w.hi & 0x7fffffffu) >= (3u << 20) || is_zero(w)) return fma(0.25, x, y);
+  return y + unit_mul(0.25, x);
+}
 // 2 a, exact: the exponent field raised by one
 LSMGPU_FPI_DEV double twice_any(double a) {
   const W2 w = words(a);

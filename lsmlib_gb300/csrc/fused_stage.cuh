@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CU
 
     const long long cell = L.idx(i, j, k);
     R u = c[0] + mul_(a.dt, rhs);  // tvd_runge_kutta3d.f:78
-    if (a.stage == 2) u = fma(R(0.25), u, mul_(R(0.75), a.phi_n[cell]));  // :403-404 (u / 4 is exact)
+    if (a.stage == 2) u = fpi::plus_quarter(mul_(R(0.75), a.phi_n[cell]), u);  // :403-404
     if (a.stage == 3) u = mul_(R(1.0 / 3.0), a.phi_n[cell]) + mul_(R(2.0 / 3.0), u);  // :490-492
     a.out[cell] = u;
 
