@@ -87,7 +87,7 @@ __device__ __forceinline__ void weno_local_pm(const R D[6], R inv, R &gp, R &gm)
 template <class R>
 __device__ __forceinline__ R cell_vn(const BandArgs<R> &a, const R *c, const long long s[3]) {
   const R f = a.f_half;
-  const R g0 = mul_(c[s[0]] - c[-s[0]], f), g1 = mul_(c[s[1]] - c[-s[1]], f), g2 = mul_(c[s[2]] - c[-s[2]], f);
+  const R g0 = mul_z_(c[s[0]] - c[-s[0]], f), g1 = mul_z_(c[s[1]] - c[-s[1]], f), g2 = mul_z_(c[s[2]] - c[-s[2]], f);
   const R mag = grad_magnitude(g0, g1, g2, R(Consts<double>::zero_tol));
   const R kappa = mean_curvature2(c, s[0], s[1], s[2], g0, g1, g2, mag, a.f_xx, a.f_xx, a.f_xx, a.f_xy, a.f_xy, a.f_xy);
   return a.a_n - mul_(a.b_n, kappa);
@@ -107,7 +107,7 @@ __device__ __forceinline__ R godunov_rhs(const BandArgs<R> &a, R vn, const R gp[
   const R cx = max_nonneg_(abs_(gp[0]), abs_(gm[0])), cy = max_nonneg_(abs_(gp[1]), abs_(gm[1]));
   const R cz = max_nonneg_(abs_(gp[2]), abs_(gm[2]));
   const R ng = sqrt_(sqr_(cx) + sqr_(cy) + sqr_(cz) + mx2);
-  h_over_dx = (ng > tol) ? mul_(div_(abs_(vn), ng), mul_(cx, inv) + mul_(cy, inv) + mul_(cz, inv)) : R(-1.0);
+  h_over_dx = (ng > tol) ? mul_z_(div_(abs_(vn), ng), mul_z_(cx, inv) + mul_z_(cy, inv) + mul_z_(cz, inv)) : R(-1.0);
   return rhs;
 }
 

@@ -31,9 +31,9 @@ __global__ void __launch_bounds__(256) k_mean_curvature(CurvArgs<R> a) {
   const R *c = a.phi.p + a.phi.off(i, j, k);
   const long long sx = 1, sy = a.phi.s1, sz = a.phi.s2;
   // central gradient, its magnitude with the reference's 1e-8 clamps, curvature
-  const R px = mul_(c[sx] - c[-sx], a.gx);
-  const R py = mul_(c[sy] - c[-sy], a.gy);
-  const R pz = mul_(c[sz] - c[-sz], a.gz);
+  const R px = mul_z_(c[sx] - c[-sx], a.gx);
+  const R py = mul_z_(c[sy] - c[-sy], a.gy);
+  const R pz = mul_z_(c[sz] - c[-sz], a.gz);
   const R g = grad_magnitude(px, py, pz, R(1.e-8));
   if (a.mag.p) a.mag(i, j, k) = g;
   a.kappa(i, j, k) = mean_curvature2(c, sx, sy, sz, px, py, pz, g, a.fxx, a.fyy, a.fzz, a.fxy, a.fxz, a.fyz);

@@ -102,9 +102,9 @@ __global__ void __launch_bounds__(256, 6) k_hj_pm_weno5(Out3 plus, Out3 minus, V
 }
 
 // Upwind HJ WENO5 (spatial_derivatives3d.f.in:2628-2996).  The plus side is
-// the minus side of the mirrored line, negated (every rounding is symmetric),
-// so a lane walks its line with the stride's sign and lanes of both sides run
-// the same reconstruction.
+// the minus side of the mirrored line's negated differences (every rounding is
+// symmetric), so a lane walks its line with the stride's sign and lanes of both
+// sides run the same reconstruction.
 __global__ void __launch_bounds__(256, 7) k_hj_upwind_weno5(Out3 g, View<const R> phi, View<const R> vx,
                                                             View<const R> vy, View<const R> vz, Box fb, unsigned axes,
                                                             R ix, R iy, R iz) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256, 7) k_hj_upwind_weno5(Out3 g, View<const R
     for (int q = 0; q < 6; q++) x[q] = __ldg(c + (q - 3) * s);
 #pragma unroll
     for (int q = 0; q < 5; q++) D[q] = x[q + 1] - x[q];
-    out = flip_if_(weno5_side64(D, wide64(a.d == 0 ? ix : (a.d == 1 ? iy : iz)), Consts<R>::tiny), !pos);
+    out = weno5_side64(D, wide64(a.d == 0 ? ix : (a.d == 1 ? iy : iz)), Consts<R>::tiny, !pos);
   }
   g.at(a.d, a.i, a.j, a.k) = out;
 }
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned 
         const R cy = max_nonneg_(abs_(A.pyp(i, j, k)), abs_(A.pym(i, j, k)));
         const R cz = max_nonneg_(abs_(A.pzp(i, j, k)), abs_(A.pzm(i, j, k)));
         const R ng = sqrt_(sqr_(cx) + sqr_(cy) + sqr_(cz) + A.max_dx_sq);
-        v = mul_(div_(avn, ng), mul_(cx, A.ix) + mul_(cy, A.iy) + mul_(cz, A.iz));
+        v = mul_z_(div_(avn, ng), mul_z_(cx, A.ix) + mul_z_(cy, A.iy) + mul_z_(cz, A.iz));
       }
       // a NaN exceeds nothing (the reference's comparison is false)
       if (fpi::mag(v) <= fpi::kInfBits) best = max(best, okey(v));

@@ -258,6 +258,15 @@ LSMGPU_FPI_DEV bool plain(const W2 &w) {
   return ((w.hi & 0x7fffffffu) - ((1023u - LO) << 20)) < ((2u * LO) << 20) || is_zero(w);
 }
 LSMGPU_FPI_DEV double mul_any(double a, double b) {
+  const W2 aw = words(a), bw = words(b);
+  if (plain<511>(aw) && plain<511>(bw)) {
+    const W2 r = words(mul(unpack(a, 1), unpack(b, 1)));
+    return from_words(r.hi | ((aw.hi ^ bw.hi) & 0x80000000u), r.lo);  // a zero gets its sign
+  }
+  return unit_mul(a, b);
+}
+// the same, but a zero product of numbers in range is +0
+LSMGPU_FPI_DEV double mul_any_z(double a, double b) {
   if (plain<511>(words(a)) && plain<511>(words(b))) return mul(unpack(a, 1), unpack(b, 1));
   return unit_mul(a, b);
 }

@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CU
           for (int f = -2; f <= 2; f++) D[f + 2] = c[f * s] - c[(f - 1) * s];
           g = weno5_side64(D, wide64(a.inv[d]), Consts<R>::tiny);
         }
-        const R t = mul_(abs_(u), g);
+        const R t = mul_z_(abs_(u), g);
         dot = d == 0 ? t : dot + t;
       }
       // lsm3dZeroOutLevelSetEqnRHS then lsm3dAddAdvectionTermToLSERHS

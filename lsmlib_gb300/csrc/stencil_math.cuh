@@ -121,6 +121,15 @@ __device__ __forceinline__ R mul_(R a, R b) {
   if constexpr (std::is_same<R, double>::value) return fpi::mul_any(a, b);
   else return a * b;
 }
+// with zero products as +0, for where a zero's sign reaches no result (of a
+// curvature: only the sign of a zero one, on a field of zeros of both signs);
+// 384^3 curvature, gradient magnitude and dt: 4.43 ms with mul_ throughout, 4.34
+// with this where it may
+template <class R>
+__device__ __forceinline__ R mul_z_(R a, R b) {
+  if constexpr (std::is_same<R, double>::value) return fpi::mul_any_z(a, b);
+  else return a * b;
+}
 template <class R>
 __device__ __forceinline__ R sqr_(R a) {
   if constexpr (std::is_same<R, double>::value) return fpi::sqr_any(a);
@@ -215,7 +224,7 @@ __device__ __forceinline__ R reinit_axis(R pc, R gp, R gm) {
 template <class R>
 __device__ __forceinline__ R reinit_from_sq(R pc, R n2, R dx_sq, bool use0) {
   if (!at_least_(pc, R(Consts<R>::zero_tol))) return R(0);
-  const R q = sqr_(pc) + (use0 ? dx_sq : mul_(n2, dx_sq));
+  const R q = sqr_(pc) + (use0 ? dx_sq : mul_z_(n2, dx_sq));
   return mul_(div_(pc, sqrt_(q)), R(1.0) - sqrt_(n2));
 }
 template <class R>
@@ -285,15 +294,15 @@ __device__ __forceinline__ R grad_magnitude(R x, R y, R z, R tol) {
 template <class R, class I>
 __device__ __forceinline__ R mean_curvature2(const R *c, I sx, I sy, I sz, R px, R py, R pz, R g, R fxx, R fyy, R fzz,
                                              R fxy, R fxz, R fyz) {
-  const R den = mul_(mul_(g, g), g);
+  const R den = mul_z_(mul_z_(g, g), g);
   if (less_(den, R(Consts<double>::zero_tol))) return R(0);
-  // c+ - 2 c0 is one fma: 2 c0 is exact
-  const R xx = mul_(fma(R(-2.0), c[0], c[sx]) + c[-sx], fxx);
-  const R yy = mul_(fma(R(-2.0), c[0], c[sy]) + c[-sy], fyy);
-  const R zz = mul_(fma(R(-2.0), c[0], c[sz]) + c[-sz], fzz);
-  const R xy = mul_(c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy], fxy);
-  const R xz = mul_(c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz], fxz);
-  const R yz = mul_(c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz], fyz);
+  // c+ - 2 c0 is one fma: 2 c0 is exact (below 2^1023; beyond, LSMLIB overflows here)
+  const R xx = mul_z_(fma(R(-2.0), c[0], c[sx]) + c[-sx], fxx);
+  const R yy = mul_z_(fma(R(-2.0), c[0], c[sy]) + c[-sy], fyy);
+  const R zz = mul_z_(fma(R(-2.0), c[0], c[sz]) + c[-sz], fzz);
+  const R xy = mul_z_(c[sx + sy] - c[sx - sy] - c[-sx + sy] + c[-sx - sy], fxy);
+  const R xz = mul_z_(c[sx + sz] - c[sx - sz] - c[-sx + sz] + c[-sx - sz], fxz);
+  const R yz = mul_z_(c[sy + sz] - c[sy - sz] - c[-sy + sz] + c[-sy - sz], fyz);
   return div_(curv_numerator(xx, yy, zz, xy, xz, yz, px, py, pz), den);
 }
 

@@ -140,12 +140,17 @@ __device__ __forceinline__ double combine64(double S1, double S2, double S3, dou
   return term(a1, p1) + term(a2, p2) + term(a3, p3);
 }
 
-// One side on the undivided differences d[0..4] (v1 .. v5 once divided).
-__device__ __forceinline__ double weno5_side64(const double d[5], const Wide64 &w, double tiny) {
+// One side on the undivided differences d[0..4] (v1 .. v5 once divided); with
+// `flip` the negated value of the negated differences, which is the same number
+// but for the sign of a zero: the reconstruction of zeros is +0 either way.
+__device__ __forceinline__ double weno5_side64(const double d[5], const Wide64 &w, double tiny, bool flip = false) {
   Range64 rg;
 #pragma unroll
   for (int q = 0; q < 5; q++) rg.add(d[q]);
-  if (!rg.ok(w)) return weno5_unit64(d[0] * w.inv, d[1] * w.inv, d[2] * w.inv, d[3] * w.inv, d[4] * w.inv, tiny);
+  if (!rg.ok(w)) {
+    const double inv = flip ? -w.inv : w.inv;
+    return weno5_unit64(d[0] * inv, d[1] * inv, d[2] * inv, d[3] * inv, d[4] * inv, tiny);
+  }
   Diff64 v[5];
 #pragma unroll
   for (int q = 0; q < 5; q++) v[q] = divided(d[q], w);
@@ -161,7 +166,8 @@ __device__ __forceinline__ double weno5_side64(const double d[5], const Wide64 &
   const double S1 = indicator64(fma(-2.0, v[1].v, v[0].v) + v[2].v, fma(-4.0, v[1].v, v[0].v) + v3x3);
   const double S2 = indicator64(fma(-2.0, v[2].v, v[1].v) + v[3].v, v[1].v - v[3].v);
   const double S3 = indicator64(fma(-2.0, v[3].v, v[2].v) + v[4].v, fma(-4.0, v[3].v, v3x3) + v[4].v);
-  return combine64(S1, S2, S3, eps, p1, p2, p3);
+  const double r = combine64(S1, S2, S3, eps, p1, p2, p3);  // a zero is +0
+  return fpi::flip_if(r, flip && !fpi::is_zero(fpi::words(r)));
 }
 
 // Both sides of an axis at a cell on the undivided differences

@@ -1,11 +1,13 @@
-"""FP64 at the ends of the exponent range: the drop-ins and the fused steppers
-return the oracle's numbers where products become subnormal."""
+"""FP64 at the ends of the exponent range and at zero: the drop-ins and the
+fused steppers return the oracle's numbers where products become subnormal, and
+its signs of zeros."""
 import numpy as np
 import pytest
 
 import lsmlib_gb300 as L
 from tests import harness as H
 from tests import oracle_runs as O
+from tests.test_local import local_case
 
 GB, FB = (-3, 20, -3, 18, -3, 16), (0, 17, 0, 15, 0, 13)
 # integer multiples of the smallest subnormal, and values around the smallest
@@ -43,3 +45,46 @@ def test_fused_advection(kind, bc, gpu_lib):
         got = phi.copy(order="F")
         L.advect_weno5_tvdrk3(got, GB, FB, dx, dt, 2, bc=bc, **kw)
         assert H.same(want, got)
+
+
+def same_bits(a, b):
+    """As H.same, but +0 and -0 differ."""
+    return H.same(a, b) and bool(np.all(np.isnan(a) | (np.signbit(a) == np.signbit(b))))
+
+
+SIGN_KINDS = {"flat": lambda rng, n: np.full(n, 0.75),
+              "plane": lambda rng, n: 0.25 * np.indices(n)[0] - 1.0,
+              "kink": lambda rng, n: np.abs(0.25 * np.indices(n)[-1] - 1.0),
+              "zeros": lambda rng, n: np.where(rng.random(n) < 0.5, 0.0, -0.0),
+              "minus zero": lambda rng, n: np.full(n, -0.0),
+              "zeros and ones": lambda rng, n: rng.choice([0.0, -0.0, 1.0, -1.0], size=n),
+              "1e200": lambda rng, n: rng.standard_normal(n) * 1e200}
+SIGN_SYMS = ["lsm3dhjweno5_", "lsm3dupwindhjweno5_", "lsm3dtvdrk3stage2_", "lsm3dtvdrk3stage3_",
+             "lsm3dcomputereinitializationeqnrhs_", "lsm3dcomputemeancurvatureorder2_", "lsm3dgradientmagnitude_",
+             "lsm3daddnormalveltermtolserhs_", "lsm3daddconstcurvtermtolserhs_", "lsm3daddadvectiontermtolserhs_",
+             "lsm3dcomputereinitializationeqnrhslocal_", "lsm3dcomputemeancurvatureorder2local_",
+             "lsm3dhjweno5local_"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", sorted(SIGN_KINDS))
+@pytest.mark.parametrize("sym", SIGN_SYMS)
+def test_signs_of_zeros(sym, kind, gpu_lib):
+    """Zeros come out with LSMLIB's sign, with one input array of each kind at
+    a time and with all of them.  (A zero mean curvature is +0; LSMLIB's is
+    now and then -0 on a field of zeros of both signs.)"""
+    if "meancurvature" in sym and kind.startswith("zeros"):
+        pytest.skip("the sign of a zero curvature")
+    base = local_case(sym, 4) if sym.endswith("local_") else H.dense_case(sym, seed=4)
+    names = [k for k, v in base.items() if isinstance(v, np.ndarray) and v.dtype == np.float64]
+    for which in [[name] for name in names] + [names]:
+        vals = dict(base)
+        for name in which:
+            vals[name] = np.asfortranarray(SIGN_KINDS[kind](np.random.default_rng(8), vals[name].shape))
+        with np.errstate(all="ignore"):
+            want, _ = H.run(H.oracle(), sym, vals)
+            got, _ = H.run(gpu_lib, sym, vals)
+        L.check()
+        for name in H.written_names(sym):
+            if name in want and want[name].dtype == np.float64:
+                assert same_bits(want[name], got[name]), (which, name)
