@@ -166,10 +166,15 @@ def invoke(handle, sym, values, abi=None):
     """
     spec = (abi or ABI)[sym]
     # per thread, and out of the table during the call, so that no two calls
-    # share a plan's buffer; a call that raises drops it
-    plan = _plans.__dict__.pop(sym, None)
-    if plan is None or plan.handle is not handle or plan.spec is not spec:
+    # share a plan's buffer; a call that raises drops it.  One per library, for
+    # programs that call the same entry point of several (four at most).
+    kept = _plans.__dict__.pop(sym, ())
+    for plan in kept:
+        if plan.handle is handle and plan.spec is spec:
+            break
+    else:
         plan = _Plan(handle, sym, spec)
+        kept = (plan,) + kept[:3]
     try:
         for pointer, name in plan.arrays:
             v = values[name]
@@ -187,7 +192,7 @@ def invoke(handle, sym, values, abi=None):
         plan.pack_into(plan.buf, 0, *[_SCALAR_CT[k](v).value for k, v in zip(plan.kinds, scalars)])
     plan.fn(*plan.args)
     out = dict(zip(plan.names, plan.unpack_from(plan.buf, 0)))
-    _plans.__dict__[sym] = plan
+    _plans.__dict__[sym] = kept
     return out
 
 

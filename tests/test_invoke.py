@@ -66,3 +66,28 @@ def test_threads_do_not_share_a_call():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def test_two_libraries_called_in_turn_keep_their_plans(monkeypatch):
+    """A program that compares two libraries prepares each entry point once per
+    library, not once per call."""
+    import ctypes
+    libs = [ctypes.CDLL(H.oracle()._name) for _ in range(2)]
+    made = []
+
+    class Counted(L._Plan):
+        def __init__(self, *args):
+            made.append(args)
+            super().__init__(*args)
+
+    monkeypatch.setattr(L, "_Plan", Counted)
+    for seed in range(1, 7):
+        vals, out, u, rhs = _axpy_call(seed)
+        L.invoke(libs[seed % 2], "lsm3drk1step_", vals)
+        inner = (slice(1, 5), slice(1, 4), slice(1, 3))
+        assert np.array_equal(out[inner], (u + 0.1 * seed * rhs)[inner])
+    assert len(made) == 2
+    for _ in range(6):  # any number of libraries
+        vals, out, u, rhs = _axpy_call(3)
+        L.invoke(ctypes.CDLL(H.oracle()._name), "lsm3drk1step_", vals)
+        assert np.array_equal(out[inner], (u + 0.1 * 3 * rhs)[inner])
