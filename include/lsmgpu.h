@@ -83,6 +83,12 @@ int lsmgpu_bounds_check_read(long long *count, int *first);
  * parameters were seen before, and captures a new one otherwise. */
 long long lsmgpu_graph_capture_count(void);
 
+/* The tile (cells along x, y and z) that the FP32 stage kernels of a stepper
+ * run on a grid of nx x ny x nz cells: mode 0 advection by a constant velocity,
+ * 1 by a velocity field, 2 reinitialization.  A query, for tests and profiles;
+ * no GPU is needed (152 SMs are assumed then). */
+int lsmgpu_stage_tile_f32(int mode, int nx, int ny, int nz, int *tile);
+
 /* Device memory (bytes, all devices) the library's grow-only staging and
  * temporary arena holds.  It grows with cudaMalloc and is never freed. */
 long long lsmgpu_arena_bytes(void);

@@ -81,6 +81,16 @@ def graph_capture_count(handle=None):
     return int((handle or lib()).lsmgpu_graph_capture_count())
 
 
+def stage_tile(mode, n, handle=None):
+    """(x, y, z) cells of the tiles the FP32 stepper `mode` ("advect_const",
+    "advect" or "reinit") runs on a grid of n = (nx, ny, nz) cells."""
+    tile = (ctypes.c_int * 3)()
+    kind = ("advect_const", "advect", "reinit").index(mode)
+    if (handle or lib()).lsmgpu_stage_tile_f32(kind, *map(int, n), tile) != 0:
+        raise ValueError("stage_tile: invalid grid %r" % (n,))
+    return tuple(tile)
+
+
 def measure_fma_rates(handle=None):
     """(FP32 lane operations/s through packed FFMA2, FP64 FMAs/s) measured by
     the library's fixed-length probe kernels on the current device."""

@@ -270,11 +270,20 @@ inline TileX2 reinit_tile(const Layout &L) {
 // 32 x 2 8.6 (8.7), x 10 10.0 (10.4); field: 100^3 64 x 8 x 2 14.4 (15.5), x 8
 // 18.6 (19.2); 128^3 64 x 8 x 4 20.5 (21.4), x 8 23.2 (24.1); 192^3 62.6 (62.9)
 // and 63.2 (63.6).
+// Of tiles of equal cost (as many of them, as deep) those with at most 2/3 of
+// the warps on rows of the grid: a grid narrower than a row fills few lanes of
+// each (constant velocity, periodic, 64 / 32 / 16 cells: 6 x 6 x 20000 63 / 46 /
+// 43; 16 x 16 x 3000 21.9 / 12.7 / 9.4; 8 x 8 x 5000 21.9 / 15.2 / 13.9).  With
+// 5/6 of them the fuller rows are no faster: 137 x 34 x 233 33.0 on 64 cells,
+// 34.2 on 32.
 inline TileX2 adv_tile_of(const Layout &L, bool field) {
   const float lone = field ? 0.85f : 0.69f, tile = field ? 0.24f : 0.41f, plane = field ? 0.59f : 0.39f;
   const int sms = sm_count();
   TileX2 t{RX, RY, 8};
   float best = INFINITY;
+  long long count = 0;
+  // warps of a plane that hold cells: 64 / w rows of w cells each
+  auto warps = [&](int w) { return (long long)((L.nx + w - 1) / w) * ((L.ny + 64 / w - 1) / (64 / w)); };
   for (int w = RX; w >= 16; w /= 2) {
     const int h = 512 / w;
     const long long cols = (long long)((L.nx + w - 1) / w) * ((L.ny + h - 1) / h);
@@ -282,7 +291,8 @@ inline TileX2 adv_tile_of(const Layout &L, bool field) {
       const long long zt = (L.nz + tz - 1) / tz;
       if (zt > 65535) continue;
       const float cost = 2.5f + lone * tz + (float)((cols * zt + sms - 1) / sms - 1) * (tile + plane * tz);
-      if (cost < best) t = TileX2{w, h, tz}, best = cost;
+      const bool fuller = cols * zt == count && tz == t.tz && 3 * warps(w) <= 2 * warps(t.w);
+      if (cost < best || fuller) t = TileX2{w, h, tz}, best = cost, count = cols * zt;
     }
   }
   return t;
