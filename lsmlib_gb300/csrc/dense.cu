@@ -322,26 +322,16 @@ __global__ void __launch_bounds__(256) k_zero(R *p, long long n) {
 }
 
 // Bound by memory: two products on the FP64 unit beside the three sums, the
-// third on the integer pipes.
+// third on the integer pipes.  One cell per thread: many warps with seven loads
+// each hide more than a quarter of them with 28 (us, every product on the FP64
+// unit / this / four planes per thread: 100^3 18.6 / 16.5 / 18.5, 128^3 28.8 /
+// 25.0 / 31.0, 256^3 198 / 167 / 189).
 __global__ void __launch_bounds__(256) k_add_advection(View<R> rhs, View<const R> px, View<const R> py,
                                                        View<const R> pz, View<const R> vx, View<const R> vy,
-                                                       View<const R> vz, Box fb, int planes) {
-  const int i = fb.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = fb.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k0 = first_plane(fb, planes), n = min(planes, fb.hi[2] - k0 + 1);
-  if (i > fb.hi[0] || j > fb.hi[1]) return;
-  R r[kPlanes], g[kPlanes][3], v[kPlanes][3];
-#pragma unroll
-  for (int q = 0; q < kPlanes; q++)
-    if (q < n) {
-      const int k = k0 + q;
-      r[q] = rhs(i, j, k);
-      g[q][0] = px(i, j, k); g[q][1] = py(i, j, k); g[q][2] = pz(i, j, k);
-      v[q][0] = vx(i, j, k); v[q][1] = vy(i, j, k); v[q][2] = vz(i, j, k);
-    }
-#pragma unroll
-  for (int q = 0; q < kPlanes; q++)
-    if (q < n) rhs(i, j, k0 + q) = r[q] - (v[q][0] * g[q][0] + v[q][1] * g[q][1] + mul_(v[q][2], g[q][2]));
+                                                       View<const R> vz, Box fb) {
+  LSMGPU_CELL_INDEX(fb, i, j, k);
+  rhs(i, j, k) = rhs(i, j, k) - (vx(i, j, k) * px(i, j, k) + vy(i, j, k) * py(i, j, k) +
+                                 mul_(vz(i, j, k), pz(i, j, k)));
 }
 
 // vn field (const_vn == false) or constant (const_vn == true)
@@ -837,9 +827,8 @@ void lsm3daddadvectiontermtolserhs_(R *lse_rhs, BOXARG(r), const R *phi_x, const
   View<const R> VX = view((const R *)call.in(vel_x, nv), vb), VY = view((const R *)call.in(vel_y, nv), vb),
                 VZ = view((const R *)call.in(vel_z, nv), vb);
   if (!call.ok()) return;
-  int planes;
-  const Grid3 g3 = cover_planes(fb, planes);
-  LSMGPU_LAUNCH(k_add_advection, g3.grid, g3.block, 0, O, X, Y, Z, VX, VY, VZ, fb, planes);
+  const Grid3 g3 = cover(fb);
+  LSMGPU_LAUNCH(k_add_advection, g3.grid, g3.block, 0, O, X, Y, Z, VX, VY, VZ, fb);
   call.finish();
 }
 
