@@ -443,7 +443,18 @@ struct RedArgs {
   R vn_const, ix, iy, iz, max_dx_sq;
 };
 
-constexpr int kRedZ = 8;  // planes a thread walks: fewer blocks to fold, more loads in flight
+// Planes a thread of the reductions walks: up to 8, which leaves fewer blocks to
+// fold and more loads in flight, fewer where that would leave less than 8 blocks
+// per SM.  us, advection dt with 8 / 4 / 2 / 1 planes: 8^3 34.2 / 34.3 / 32.7 /
+// 30.8, 100^3 45.7 / 36.4 / 36.7 / 46.2, 128^3 46.7 / 44.6 / 46.0 / 51.1, 256^3
+// 108 / 112 / 158 / 249; |a - b| at 8^3 32.5 / 28.6 / 26.9 / 26.4.
+constexpr int kRedZ = 8;
+inline int reduction_planes(const Box &ib) {
+  const long long cols = ((ib.n(0) + 31) / 32) * ((ib.n(1) + 7) / 8);
+  int zn = kRedZ;
+  while (zn > 1 && cols * ((ib.n(2) + zn - 1) / zn) < 8 * 152) zn /= 2;
+  return zn;
+}
 
 // an FP32 bound from above on |x| (infinity where FP32 does not reach, and
 // for NaN), and one from below on x (for x < 2^-100: less than any bound)
@@ -465,15 +476,15 @@ __device__ __forceinline__ float below32(R x) {
 // settles nearly every cell without FP64 arithmetic (the running maximum of
 // the earlier blocks is the start); the others evaluate the reference's sum.
 // Bound by memory then (384^3: 1.18 ms with every cell in FP64).
-__global__ void __launch_bounds__(256) k_advection_max(RedArgs A, Box ib, unsigned long long *key) {
+__global__ void __launch_bounds__(256) k_advection_max(RedArgs A, Box ib, unsigned long long *key, int zn) {
   const int i = ib.lo[0] + blockIdx.x * 32 + threadIdx.x;
   const int j = ib.lo[1] + blockIdx.y * 8 + threadIdx.y;
-  const int k0 = ib.lo[2] + blockIdx.z * kRedZ, n = min(kRedZ, ib.hi[2] - k0 + 1);
+  const int k0 = ib.lo[2] + blockIdx.z * zn, n = min(zn, ib.hi[2] - k0 + 1);
   unsigned long long best = __ldcg(key);
   float low = below32(okey_inv(best));
   const float ix = above32(A.ix), iy = above32(A.iy), iz = above32(A.iz);
   if (i <= ib.hi[0] && j <= ib.hi[1]) {
-    for (int h = 0; h < kRedZ; h += kPlanes) {
+    for (int h = 0; h < n; h += kPlanes) {
       R u[kPlanes], v[kPlanes], w[kPlanes];
       bool take[kPlanes];
 #pragma unroll
@@ -506,14 +517,14 @@ __global__ void __launch_bounds__(256) k_advection_max(RedArgs A, Box ib, unsign
 
 // mode 3: |a - b|; modes 1, 2: the normal velocity's H / dx
 template <int MODE>
-__global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned long long *key) {
+__global__ void __launch_bounds__(256) k_reduce_max(RedArgs A, Box ib, unsigned long long *key, int zn) {
   const int i = ib.lo[0] + blockIdx.x * 32 + threadIdx.x;
   const int j = ib.lo[1] + blockIdx.y * 8 + threadIdx.y;
-  const int k0 = ib.lo[2] + blockIdx.z * kRedZ;
+  const int k0 = ib.lo[2] + blockIdx.z * zn;
   unsigned long long best = okey(R(-1.0e308));
   if (i <= ib.hi[0] && j <= ib.hi[1]) {
 #pragma unroll 4
-    for (int k = k0; k < k0 + kRedZ && k <= ib.hi[2]; k++) {
+    for (int k = k0; k < k0 + zn && k <= ib.hi[2]; k++) {
       if (A.cv_sgn != 0 && !(MODE == 3 && i == ib.lo[0] && j == ib.lo[1] && k == ib.lo[2])) {
         const R c = A.cv(i, j, k);
         if (!is_pos_(flip_if_(c, A.cv_sgn < 0))) continue;
@@ -556,10 +567,11 @@ void reduce_max(Call &call, RedArgs &A, const Box &ib, R *out, R cfl, R init) {
   if (!call.ok()) return;
   LSMGPU_LAUNCH(k_set_key, 1, 1, 0, key, init);
   if (!ib.empty()) {
+    const int zn = reduction_planes(ib);
     const dim3 grd((unsigned)((ib.n(0) + 31) / 32), (unsigned)((ib.n(1) + 7) / 8),
-                   (unsigned)((ib.n(2) + kRedZ - 1) / kRedZ));
-    if constexpr (MODE == 0) LSMGPU_LAUNCH(k_advection_max, grd, dim3(32, 8), 0, A, ib, key);
-    else LSMGPU_LAUNCH(k_reduce_max<MODE>, grd, dim3(32, 8), 0, A, ib, key);
+                   (unsigned)((ib.n(2) + zn - 1) / zn));
+    if constexpr (MODE == 0) LSMGPU_LAUNCH(k_advection_max, grd, dim3(32, 8), 0, A, ib, key, zn);
+    else LSMGPU_LAUNCH(k_reduce_max<MODE>, grd, dim3(32, 8), 0, A, ib, key, zn);
   }
   LSMGPU_LAUNCH(k_finish_scalar, 1, 1, 0, key, dout, MODE, cfl, init);
   call.finish();
