@@ -172,6 +172,7 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
       set_error(LSMGPU_ERR_BOUNDS, "%s: grid %d has more than 65535 tiles along an axis", name, g);
       return LSMGPU_ERR_BOUNDS;
     }
+    desc[g].scale = fused::spacing_scale(spacing + 3 * g);
     uoff[g] = offsets[g];
     user_total = std::max(user_total, offsets[g] + (long long)(nx + 6) * (ny + 6) * (nz + 6));
   }
@@ -188,7 +189,7 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
 
-  // layouts and tiles of `depth` planes at most
+  // layouts and tiles of `depth` planes at most (the scales are there)
   long long total = 0, ntiles = 0;
   auto build_desc = [&](int depth) {
     total = ntiles = 0;
@@ -197,7 +198,6 @@ extern "C" int lsmgpu_advect_batch_weno5_tvdrk3_f32(float *phi, const long long 
       G.L = fused::make_layout(dims[3 * g], dims[3 * g + 1], dims[3 * g + 2]);
       G.off = total;
       total += (G.L.elems() + 31) / 32 * 32;
-      G.scale = fused::spacing_scale(spacing + 3 * g);
       for (int d = 0; d < 3; d++) {
         G.vconst[d] = vel[3 * g + d] < 0.f ? -vel[3 * g + d] : vel[3 * g + d];
         G.inv[d] = 1.0f / spacing[3 * g + d];

@@ -30,7 +30,8 @@ constexpr int kPackZ = 8;
 // dst2 (optional) receives the same values (the phi0 copy of the
 // reinitialization's sign form); bit d of `flip`: the layout is mirrored
 // along axis d; FP32 values are multiplied by `scale`, a power of two
-// (spacing_scale), on the way in and by its inverse on the way out
+// (spacing_scale), on the way in and by its inverse on the way out, after all
+// loads (a product beside each load made them wait for one another, 2 us)
 template <class R>
 __device__ __forceinline__ R scaled(R v, float scale) {
   if constexpr (sizeof(R) == 4) return v * scale;
@@ -50,14 +51,15 @@ __global__ void k_pack(R *dst, Layout L, View<const R> src, Box gb, int ilo, int
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
     const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
-    v[q] = (in_xy && gk >= gb.lo[2] && gk <= gb.hi[2]) ? scaled(src(gi, gj, gk), scale) : R(0);
+    v[q] = (in_xy && gk >= gb.lo[2] && gk <= gb.hi[2]) ? src(gi, gj, gk) : R(0);
   }
 #pragma unroll
   for (int q = 0; q < kPackZ; q++)
     if (k0 + q <= L.nz + 2) {
       const long long c = L.idx(i, j, k0 + q);
-      dst[c] = v[q];
-      if (dst2) dst2[c] = v[q];
+      const R u = scaled(v[q], scale);
+      dst[c] = u;
+      if (dst2) dst2[c] = u;
     }
 }
 
@@ -73,11 +75,11 @@ __global__ void k_unpack(View<R> dst, Box gb, const R *src, Layout L, int ilo, i
   R v[kPackZ];
 #pragma unroll
   for (int q = 0; q < kPackZ; q++)
-    if (k0 + q <= L.nz + 2) v[q] = scaled(src[L.idx(i, j, k0 + q)], scale);
+    if (k0 + q <= L.nz + 2) v[q] = src[L.idx(i, j, k0 + q)];
 #pragma unroll
   for (int q = 0; q < kPackZ; q++) {
     const int gk = maybe_mirrored(k0 + q, L.nz, flip & 4) + klo;
-    if (k0 + q <= L.nz + 2 && gk >= gb.lo[2] && gk <= gb.hi[2]) dst(gi, gj, gk) = v[q];
+    if (k0 + q <= L.nz + 2 && gk >= gb.lo[2] && gk <= gb.hi[2]) dst(gi, gj, gk) = scaled(v[q], scale);
   }
 }
 
