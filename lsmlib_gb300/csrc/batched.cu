@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) k_batch_pack(float *work, float *user, co
   const Layout L = G.L;
   const int ux = L.nx + 6, uy = L.ny + 6;
   const long long rows = (long long)uy * (L.nz + 6);
-  const float scale = unpack ? 1.f / G.scale : G.scale;
+  const float scale = unpack ? fused::pow2_recip(G.scale) : G.scale;
   float *const w0 = work + G.off;
   float *const u0 = user + uoff[blockIdx.y];
   for (long long r = blockIdx.x * 8 + threadIdx.x / 32; r < rows; r += gridDim.x * 8) {
