@@ -65,22 +65,6 @@ __device__ __forceinline__ void raise_key(unsigned long long *key, unsigned long
   if (k > __ldcg(key)) atomicMax(key, k);
 }
 
-// Both WENO5 sides of one axis at a cell, with the local routines' epsilon
-// floor (spatial_derivatives2d_local.f.in:892), on its six undivided
-// differences
-template <class R, bool EXACT>
-__device__ __forceinline__ void weno_local_pm(const R D[6], R inv, R &gp, R &gm) {
-  if constexpr (EXACT) {
-    weno5_pm64(D, wide64(inv), 1.e-35, gp, gm);
-  } else {
-    float v[6];
-#pragma unroll
-    for (int q = 0; q < 6; q++) v[q] = (float)(D[q] * inv);
-    gp = (R)fused::weno5_fast(v[5], v[4], v[3], v[2], v[1]);
-    gm = (R)fused::weno5_fast(v[0], v[1], v[2], v[3], v[4]);
-  }
-}
-
 // normal speed Vn = a_n - b_n kappa at a level-0 cell: central gradient,
 // |grad phi| with zero_tol clamps, mean curvature
 // (spatial_derivatives3d_local.f.in:825-839, :1251-1272; curvature3d_local.f.in)
@@ -112,20 +96,20 @@ __device__ __forceinline__ R godunov_rhs(const BandArgs<R> &a, R vn, const R gp[
 }
 
 // the RHS of one level-0 cell, before the cut-off; also the cell's H/dx for dt
-template <class R, bool EXACT>
+template <class R>
 __device__ __forceinline__ R cell_rhs(const BandArgs<R> &a, long long o, R &h_over_dx) {
   const R *c = a.src.p + o;
   const long long s[3] = {1, a.src.s1, a.src.s2};
   const R vn = cell_vn<R>(a, c, s);
-  // HJ WENO5 plus/minus from the band values of src
-  const R inv = a.inv_dx;
+  // HJ WENO5 plus/minus from the band values of src, with the local routines'
+  // epsilon floor (spatial_derivatives2d_local.f.in:892)
   R gp[3], gm[3];
 #pragma unroll 1
   for (int d = 0; d < 3; d++) {
     R D[6];
 #pragma unroll
     for (int q = -2; q <= 3; q++) D[q + 2] = c[q * s[d]] - c[(q - 1) * s[d]];
-    weno_local_pm<R, EXACT>(D, inv, gp[d], gm[d]);
+    weno5_pm64(D, wide64(a.inv_dx), 1.e-35, gp[d], gm[d]);
   }
   return godunov_rhs<R>(a, vn, gp, gm, h_over_dx);
 }
@@ -242,14 +226,14 @@ __device__ __forceinline__ R rk_update(int stage, R un, R us, R dt, R rhs) {
 }
 
 // stage 1, pass 1: RHS (cut off) per entry and the dt maximum
-template <class R, bool EXACT>
+template <class R>
 __global__ void k_band_rhs(BandArgs<R> a) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   double h = -1.0e308;
   if (l < a.n0) {
     const long long o = a.off0[l];
     R hd;
-    const R r = cell_rhs<R, EXACT>(a, o, hd);
+    const R r = cell_rhs<R>(a, o, hd);
     h = (double)hd;
     a.rhs[l] = cutoff<R>(r, a.src.p[o], a.beta, a.gamma);
   }
@@ -276,14 +260,14 @@ __global__ void k_band_update1(BandArgs<R> a) {
 }
 
 // stages 2 and 3: RHS, cut-off and update in one pass
-template <class R, bool EXACT>
+template <class R>
 __global__ void k_band_stage(BandArgs<R> a) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= a.n0) return;
   const long long o = a.off0[l];
   R hd;
   const R us = a.src.p[o];
-  const R r = cutoff<R>(cell_rhs<R, EXACT>(a, o, hd), us, a.beta, a.gamma);
+  const R r = cutoff<R>(cell_rhs<R>(a, o, hd), us, a.beta, a.gamma);
   a.out.p[o] = rk_update<R>(a.stage, a.phin.p[o], us, *a.dt, r);
 }
 
@@ -506,7 +490,7 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, R dx, R a_n
     a.stage = 1;
     cudaMemsetAsync(key, 0, sizeof(unsigned long long), s);
     if constexpr (packed) LSMGPU_LAUNCH((small ? k_band_rhs_x2<unsigned> : k_band_rhs_x2<unsigned long long>), blocks2, 128, 0, a);
-    else LSMGPU_LAUNCH((k_band_rhs<R, EXACT>), blocks, 128, 0, a);
+    else LSMGPU_LAUNCH(k_band_rhs<R>, blocks, 128, 0, a);
     LSMGPU_LAUNCH(k_band_dt<R>, 1, 1, 0, key, dt, cfl, dtl ? dtl + step : nullptr);
     if constexpr (packed) LSMGPU_LAUNCH((small ? k_band_update1_x2<unsigned> : k_band_update1_x2<unsigned long long>), blocks2, 128, 0, a);
     else LSMGPU_LAUNCH(k_band_update1<R>, blocks, 128, 0, a);
@@ -516,13 +500,13 @@ int run(const char *name, R *phi_user, const Box &gb, const Box &fb, R dx, R a_n
     a.phin = view((const R *)phi, gb);
     a.stage = 2;
     if constexpr (packed) LSMGPU_LAUNCH((small ? k_band_stage_x2<unsigned> : k_band_stage_x2<unsigned long long>), blocks2, 128, 0, a);
-    else LSMGPU_LAUNCH((k_band_stage<R, EXACT>), blocks, 128, 0, a);
+    else LSMGPU_LAUNCH(k_band_stage<R>, blocks, 128, 0, a);
     // stage 3 (in place on phi: each cell reads only its own phi^n)
     a.src = view((const R *)u2, gb);
     a.out = view(phi, gb);
     a.stage = 3;
     if constexpr (packed) LSMGPU_LAUNCH((small ? k_band_stage_x2<unsigned> : k_band_stage_x2<unsigned long long>), blocks2, 128, 0, a);
-    else LSMGPU_LAUNCH((k_band_stage<R, EXACT>), blocks, 128, 0, a);
+    else LSMGPU_LAUNCH(k_band_stage<R>, blocks, 128, 0, a);
   }
   if (dt_log) cudaMemcpyAsync(dt_log, dtl, sizeof(double) * n_steps, cudaMemcpyDeviceToHost, s);
   call.finish();

@@ -296,12 +296,6 @@ LSMGPU_FPI_DEV double plus_quarter(double y, double x) {
   if ((w.hi & 0x7fffffffu) >= (3u << 20) || is_zero(w)) return fma(0.25, x, y);
   return y + unit_mul(0.25, x);
 }
-// 2 a, exact: the exponent field raised by one
-LSMGPU_FPI_DEV double twice_any(double a) {
-  const W2 w = words(a);
-  if (plain<511>(w)) return from_words(w.hi + (is_zero(w) ? 0u : 0x00100000u), w.lo);
-  return unit_mul(2.0, a);
-}
 // |a| and a with its sign flipped where `flip`, on the high word (a standalone
 // FP64 absolute value or negation is an instruction of the FP64 pipe)
 LSMGPU_FPI_DEV double abs_bits(double a) {

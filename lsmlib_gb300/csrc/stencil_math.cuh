@@ -163,7 +163,10 @@ __device__ __forceinline__ R flip_if_(R a, bool flip) {
   else return flip ? -a : a;
 }
 template <class R>
-__device__ __forceinline__ R pos_part_(R a) { return is_pos_(a) ? a : R(0); }
+__device__ __forceinline__ R pos_part_(R a) {
+  if constexpr (std::is_same<R, double>::value) return fpi::positive_part(a);
+  else return a > R(0) ? a : R(0);
+}
 template <class R>
 __device__ __forceinline__ R max_nonneg_(R a, R b) {
   if constexpr (std::is_same<R, double>::value) return fpi::max_nonneg(a, b);
