@@ -102,3 +102,74 @@ def test_dropin_weno5_around_the_floor_of_epsilon(sym, scale, gpu_lib):
     for name in H.written_names(sym):
         if name in got and not name.startswith("d"):
             assert H.same(want[name], got[name]), name
+
+
+def operands(rng, n):
+    """Significands as random, with few bits, nearly full and next to powers of
+    two; exponents over 2^-40 .. 2^40."""
+    m = rng.integers(0, 1 << 52, size=n, dtype=np.uint64)
+    kind = rng.integers(0, 6, size=n)
+    m = np.where(kind == 1, m & np.uint64(0xfffff80000000), m)
+    m = np.where(kind == 2, m | np.uint64(0xfffffff000000), m)
+    m = np.where(kind == 3, m % np.uint64(5), m)
+    m = np.where(kind == 4, np.uint64((1 << 52) - 1) - m % np.uint64(5), m)
+    e = rng.integers(1023 - 40, 1023 + 41, size=n).astype(np.uint64)
+    return np.asfortranarray(((e << np.uint64(52)) | m).view(np.float64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_device_square_roots(seed, gpu_lib):
+    """The root's device form starts from the approximate instruction: a million
+    roots per seed, through |grad phi|, against numpy's."""
+    import torch
+    n = (128, 96, 90)
+    rng = np.random.default_rng(seed)
+    g = [operands(rng, n) * 2.0 ** 30 for _ in range(3)]  # their squares are above the routine's zero tolerance
+    want = np.sqrt((g[0] * g[0] + g[1] * g[1]) + g[2] * g[2])
+    if seed == 2:  # roots of squares
+        g[1][...] = g[2][...] = 0.0
+        want = np.sqrt(g[0] * g[0])
+    box = (0, n[0] - 1, 0, n[1] - 1, 0, n[2] - 1)
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+    out = torch.zeros(n[::-1], dtype=torch.float64, device="cuda")
+    vals, _ = H.make_call("lsm3dgradientmagnitude_", box, box,
+                          arrays=dict(zip(("phi_x", "phi_y", "phi_z"), g), grad_phi_mag=np.zeros(n, order="F")))
+    vals.update(phi_x=to(g[0]), phi_y=to(g[1]), phi_z=to(g[2]), grad_phi_mag=out)
+    L.invoke(gpu_lib, "lsm3dgradientmagnitude_", vals)
+    L.check()
+    assert np.array_equal(out.cpu().numpy().T, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_device_quotients(seed, gpu_lib):
+    """The quotient likewise: the mean curvature of phi with grad phi = (1, 0, 0)
+    is (phi_yy + phi_zz) / |grad phi|^3, |grad phi| being an argument."""
+    import torch
+    n = (128, 96, 90)
+    rng = np.random.default_rng(seed)
+    phi, mag = operands(rng, n), operands(rng, n)
+    phi *= rng.choice([1.0, -1.0], size=n)
+    one, zero = np.ones(n, order="F"), np.zeros(n, order="F")
+    gb = (0, n[0] - 1, 0, n[1] - 1, 0, n[2] - 1)
+    fb = (1, n[0] - 2, 1, n[1] - 2, 1, n[2] - 2)
+    h = 0.5
+    to = lambda a: torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+    vals, _ = H.make_call("lsm3dcomputemeancurvatureorder2_", gb, fb,
+                          arrays=dict(phi=phi, phi_x=one, phi_y=zero, phi_z=zero, grad_phi_mag=mag,
+                                      kappa=np.zeros(n, order="F")), scalars={"dx": h, "dy": h, "dz": h})
+    out = torch.zeros(n[::-1], dtype=torch.float64, device="cuda")
+    vals.update(phi=to(phi), phi_x=to(one), phi_y=to(zero), phi_z=to(zero), grad_phi_mag=to(mag), kappa=out)
+    L.invoke(gpu_lib, "lsm3dcomputemeancurvatureorder2_", vals)
+    L.check()
+    c = phi[1:-1, 1:-1, 1:-1]
+    f = 1.0 / h / h
+    yy = ((phi[1:-1, 2:, 1:-1] - 2.0 * c) + phi[1:-1, :-2, 1:-1]) * f
+    zz = ((phi[1:-1, 1:-1, 2:] - 2.0 * c) + phi[1:-1, 1:-1, :-2]) * f
+    m = mag[1:-1, 1:-1, 1:-1]
+    den = (m * m) * m
+    want = np.where(den < 1e-11, 0.0, (yy + zz) / den)
+    got = out.cpu().numpy().T[1:-1, 1:-1, 1:-1]
+    assert np.count_nonzero(den >= 1e-11) > 500000
+    assert np.array_equal(got, want)
