@@ -719,7 +719,7 @@ def batched_case(dev, n_grids=4096, seed=11, lo=16, hi=96):
 
 def sub_batched(stream, dev, n_grids=4096, steps=30):
     """Batched uneven grids (batched_case), periodic, WENO5 / TVD-RK3 at CFL
-    0.5, 30 steps, FP32: one persistent launch per stage in a CUDA graph
+    0.5, 30 steps, FP32: one launch per stage in a CUDA graph (persistent_graph)
     against one single-grid launch per grid per stage."""
     import lsmlib_gb300 as L
     buf, offsets, dims, vel, spacing, dt = batched_case(dev, n_grids)
@@ -729,7 +729,7 @@ def sub_batched(stream, dev, n_grids=4096, steps=30):
                        "30 steps, FP32", "grids": n_grids, "cells": cells}
     for name, flags in (("persistent_graph", 0), ("launch_loop", L.BATCH_LOOP)):
         buf.copy_(pristine)
-        L.advect_batch_weno5_tvdrk3(buf, offsets, dims, vel, spacing, dt, 1, flags=flags)  # tune / warm up
+        L.advect_batch_weno5_tvdrk3(buf, offsets, dims, vel, spacing, dt, 1, flags=flags)  # warm up
         buf.copy_(pristine)
         ms = _timed(lambda: L.advect_batch_weno5_tvdrk3(buf, offsets, dims, vel, spacing, dt, steps, flags=flags),
                     stream)
@@ -894,9 +894,9 @@ def sub_geometry(stream, dev, n=512, reps=10):
 
 # DRAM bytes (read + write) of one fused FP32 reinitialization stage launch
 # at 256^3, from one ncu capture of a stage-2 launch of k_reinit_x2
-# (profiles/k_reinit_x2_reinit_f32_256.md: 233.1 + 51.5 MB; the stage's
+# (profiles/k_reinit_x2_reinit_f32_256.md: 233.2 + 50.2 MB; the stage's
 # algorithmic bytes are 16 B/cell = 268.4 MB)
-MEASURED_STAGE_TRAFFIC = 284.6e6
+MEASURED_STAGE_TRAFFIC = 283.3e6
 
 # FMA-pipe thread-instructions (a packed FFMA2 / FMUL2 / FADD2 counts once)
 # per cell of one headline stage launch (k_reinit_x2, ncu

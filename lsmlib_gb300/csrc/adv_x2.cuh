@@ -225,7 +225,8 @@ __device__ __forceinline__ void adv_tile(const float *tile, float *xedge, const 
 // selection 60 moves.  us per stage, two z-neighbouring cells per thread of a
 // 32 x 8 tile / this: 64^3 5.96 / 5.4, 100^3 19.3 / 14.4, 192^3 76 / 62, 256^3
 // 167 / 133.  (Four CTAs per SM at 64 registers; three at 80: 192^3 65, 256^3
-// 138.  Planes unrolled by 1 / 4: 192^3 gradient 1% slower.)
+// 138; ten planes of 64 or 16 cells, 64.5 and 58.4 KB staged, leave room for
+// three.  Planes unrolled by 1 / 4: 192^3 gradient 1% slower.)
 template <int W, int T, int UNROLL>
 __device__ __forceinline__ void adv_field_tile(const float *tile, const StageArgs<float> &a, int x0, int y0, int z0,
                                                int tzn, int tid) {

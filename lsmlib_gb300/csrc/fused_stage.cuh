@@ -6,16 +6,17 @@
 // Work layout in HBM (one buffer per stage field): interior cells (0..nx-1,
 // 0..ny-1, 0..nz-1) with GX = 4 ghost cells below x and 3 above, 3 ghost
 // layers in y and z; rows padded to a multiple of 32 elements so each row
-// starts on a 128-byte boundary.  A CTA of 32 x 8 threads owns a 32 x 8 x 8
-// tile and stages the tile plus its 3-cell halo (40 x 14 x 14 elements) into
-// shared memory with one 3D TMA load (the FP64 stage: 1 to 4 planes per tile); the x origin of the box is the tile's
-// 32-aligned row offset, which satisfies TMA's 16-byte rule for both element
-// sizes.  Each thread then walks the 8 cells of its z column.
+// starts on a 128-byte boundary.  A CTA stages its tile plus a 3-cell halo into
+// shared memory with one 3D TMA load; the x origin of the box is the tile's
+// row offset, a multiple of 16 cells, which satisfies TMA's 16-byte rule for
+// both element sizes.
 //
-// EXACT selects the FP64 parity arithmetic (LSMLIB's operation order; the
-// including unit is compiled with -fmad=false).  Otherwise the FP32 form runs
-// with FMA contraction and an epsilon-scaled WENO weight formula that cannot
-// under- or overflow in single precision (see weno5_fast).
+// Here: the FP64 stage (k_stage: LSMLIB's operation order, the including unit
+// compiled with -fmad=false; 32 x 8 threads, each walking its z column of a
+// 32 x 8 tile of 1 to 4 planes, 8 on grids of more than 262140), and the FP32
+// arithmetic of the stages in adv_x2.cuh and reinit_x2.cuh, with FMA contraction
+// and epsilon-scaled WENO weights that cannot under- or overflow in single
+// precision (see weno5_fast).
 #pragma once
 
 #include <cmath>
@@ -216,10 +217,11 @@ __device__ __forceinline__ float weno5_fast(float v1, float v2, float v3, float 
 // The FP64 stage.  Bound by its arithmetic (weno64.cuh: the FP64 pipe with the
 // integer pipes close behind), so the tile only has to be there in time: tiles
 // of `tz` planes (1 to 4, chosen by the launcher so that the last wave of
-// tiles is a small part of the run), six CTAs per SM at 40 registers
+// tiles is a small part of the run), at 40 registers for six CTAs per SM
 // (reinitialization 121 x 118 x 109, 5 steps: four 10.27 ms, five 10.04, six
 // 9.95, seven 10.14; field advection 111 x 104 x 92: five 3.95, six 3.87,
-// seven 3.93).
+// seven 3.93; both on tiles of one plane).  Tiles of one and two planes leave
+// room for six, four planes (44.8 KB staged) for five.
 template <class R, int MODE, bool EXACT>
 __global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CUtensorMap tm, StageArgs<R> a, int tzn) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -327,11 +329,10 @@ __global__ void __launch_bounds__(TX * TY, 6) k_stage(const __grid_constant__ CU
 }  // namespace lsmgpu
 
 // ---------------------------------------------------------------------------
-// FP32 stage kernel on cell pairs: each thread advances cells (z, z+1) of its
-// column together, one cell per lane of Blackwell's packed FP32x2
-// instructions (FADD2 / FMUL2 / FFMA2), which halves the issued instructions
-// of the WENO5 arithmetic.  Comparisons, selections and the reciprocals stay
-// per lane.
+// FP32 arithmetic on cell pairs: two cells at a time, one per lane of
+// Blackwell's packed FP32x2 instructions (FADD2 / FMUL2 / FFMA2), which halves
+// the issued instructions of the WENO5 arithmetic.  Comparisons, selections and
+// the reciprocals stay per lane.
 // ---------------------------------------------------------------------------
 namespace lsmgpu {
 namespace fused {
