@@ -80,7 +80,7 @@ struct StageArgs {
 // floor of epsilon (eps_floor4) is still a normal number, and 2^24, where the
 // squares and weight products of slopes up to 7e10 stay finite.  1 for every
 // spacing already there.  (Axes more than 2^33 apart cannot both be: the widest
-// decides.)
+// decides; and with dx below 2^-9 a phi beyond 3.4e38 / scale becomes infinite.)
 template <class R>
 inline float spacing_scale(const R dx[3]) {
   int lo = 0, hi = 0;
